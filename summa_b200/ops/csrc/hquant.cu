@@ -16,6 +16,7 @@
 
 #include "host_util.h"
 #include "sm100.cuh"
+#include "w4_stream.h"
 
 namespace sb {
 
@@ -420,27 +421,14 @@ extern "C" int sb_w4_gemv_small(const void* x, const void* wk8, const void* scal
 // (up to 8), so that a 4096-column projection puts ~30 warps on every SM instead of 8. Each CTA
 // streams its K slice (4 warps, scale groups round robin, the next group's 16 loads are issued
 // before the current group is consumed), the slices meet through distributed shared memory in the
-// cluster's first CTA, which adds the residual and writes bf16. Optional fused RMSNorm of x: the
-// CTAs exchange their partial sums of squares over the cluster and scale their slice by
-// rstd * gamma (rounded to bf16, as the separate norm kernel would) before the product.
+// cluster's first CTA. Used by the fused tensor-parallel all-reduce form below; the single-GPU projections of a
+// decode step run on w4_stream.cu.
 #include <cooperative_groups.h>
 
 namespace sb {
 namespace cg = cooperative_groups;
 
 constexpr int WC_WARPS = 4;
-
-// Epilogue of the qkv projection of a decode step: rotary embedding at the device-side position and
-// the append of k / v to the cache, as the separate kernel of `attention_decode.cu` does them.
-struct RopeAppend {
-  const float* cos_t;      // [max_pos, D/2]; null = plain epilogue
-  const float* sin_t;
-  __nv_bfloat16* kc;       // caches `[B, cap, Hkv, D]` addressed through the strides below
-  __nv_bfloat16* vc;
-  const int* pos_ptr;
-  int Hq, Hkv, D, cap;
-  long c_sb, c_ss, c_sh;
-};
 
 // Row-parallel projection of a tensor-parallel decode step: the all-reduce of the partial outputs happens
 // in this kernel's epilogue over NVLink peer memory. The CTA that owns a block of output columns stores its
@@ -459,14 +447,12 @@ struct ArFuse {
   long n_pad;
 };
 
-// GATED (CPL = 2 only): W is `[K, 2I]` = [gate | value]; a lane's two columns are n and I + n and the
-// output is silu(gate) * value, `[M, I]` (the SwiGLU of a decode step without its own launch).
-template <int MR, int CPL, bool GATED>
+template <int MR, int CPL>
 __global__ void __launch_bounds__(WC_WARPS * 32)
 w4_gemv_cluster_kernel(const __nv_bfloat16* __restrict__ x, const uint32_t* __restrict__ wk8,
                        const __nv_bfloat16* __restrict__ scales, const __nv_bfloat16* __restrict__ residual,
                        __nv_bfloat16* __restrict__ y, int M, int N, int K, long ldx, int gpc,
-                       const float* __restrict__ gamma, float eps, const RopeAppend rope, const ArFuse ar) {
+                       const ArFuse ar) {
   extern __shared__ __align__(16) unsigned char wc_smem[];
   cg::cluster_group cluster = cg::this_cluster();
   const int S = (int)cluster.num_blocks();
@@ -477,20 +463,17 @@ w4_gemv_cluster_kernel(const __nv_bfloat16* __restrict__ x, const uint32_t* __re
   __nv_bfloat16* xs = reinterpret_cast<__nv_bfloat16*>(wc_smem);                          // [MR][kslice]
   float* red = reinterpret_cast<float*>(wc_smem + (size_t)MR * kslice * 2);               // [WC_WARPS][MR][32*CPL]
   float* part = red + WC_WARPS * MR * 32 * CPL;                                           // [MR][32*CPL]
-  float* ssq = part + MR * 32 * CPL;                                                      // [MR] (+pad)
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int n0 = GATED ? blockIdx.x * 32 + lane : blockIdx.x * 32 * CPL + lane * CPL;
-  const int cstride = GATED ? (N >> 1) : 1;                                               // distance of a lane's columns
+  const int n0 = blockIdx.x * 32 * CPL + lane * CPL;
   const int kbase = g_lo * 128;
   const int k8n = max(0, (g_hi - g_lo) * 16);                                             // 8-element chunks in my slice
-  const bool live = n0 < (GATED ? (N >> 1) : N);
+  const bool live = n0 < N;
   uint32_t wcur[16][CPL], wnxt[16][CPL];
   auto load_group = [&](uint32_t (&w)[16][CPL], int g) {
 #pragma unroll
     for (int r = 0; r < 16; ++r) {
       const uint32_t* p = wk8 + (long)(16 * g + r) * N + n0;
-      if (GATED) { w[r][0] = __ldcs(p); w[r][1 % CPL] = __ldcs(p + cstride); }
-      else if (CPL == 4) { const uint4 t = __ldcs(reinterpret_cast<const uint4*>(p)); w[r][0] = t.x; w[r][1 % CPL] = t.y; w[r][2 % CPL] = t.z; w[r][3 % CPL] = t.w; }
+      if (CPL == 4) { const uint4 t = __ldcs(reinterpret_cast<const uint4*>(p)); w[r][0] = t.x; w[r][1 % CPL] = t.y; w[r][2 % CPL] = t.z; w[r][3 % CPL] = t.w; }
       else if (CPL == 2) { const uint2 t = __ldcs(reinterpret_cast<const uint2*>(p)); w[r][0] = t.x; w[r][1 % CPL] = t.y; }
       else w[r][0] = __ldcs(p);
     }
@@ -503,49 +486,12 @@ w4_gemv_cluster_kernel(const __nv_bfloat16* __restrict__ x, const uint32_t* __re
   asm volatile("griddepcontrol.wait;" ::: "memory");
   // the previous call of this kernel has completed (and bumped the call number) once the wait returns
   const uint32_t ar_epoch = ar.world > 1 ? *reinterpret_cast<volatile unsigned int*>(ar.epoch_word) + 1u : 0u;
-  // ---- stage my slice of x; with a fused norm also its sum of squares
-  float sq[MR];
-#pragma unroll
-  for (int m = 0; m < MR; ++m) sq[m] = 0.f;
+  // ---- stage my slice of x
   for (int i = threadIdx.x; i < MR * k8n; i += WC_WARPS * 32) {
     const int m = i / k8n, c = i - m * k8n;
     uint4 v = make_uint4(0u, 0u, 0u, 0u);
     if (m < M) v = *reinterpret_cast<const uint4*>(x + (long)m * ldx + kbase + 8 * c);
     reinterpret_cast<uint4*>(xs + (size_t)m * kslice)[c] = v;
-    if (gamma != nullptr) {
-      const float a0 = bf16_lo(v.x), a1 = bf16_hi(v.x), a2 = bf16_lo(v.y), a3 = bf16_hi(v.y);
-      const float a4 = bf16_lo(v.z), a5 = bf16_hi(v.z), a6 = bf16_lo(v.w), a7 = bf16_hi(v.w);
-      const float s = a0 * a0 + a1 * a1 + a2 * a2 + a3 * a3 + a4 * a4 + a5 * a5 + a6 * a6 + a7 * a7;
-#pragma unroll
-      for (int mm = 0; mm < MR; ++mm) if (mm == m) sq[mm] += s;
-    }
-  }
-  if (gamma != nullptr) {
-    if (threadIdx.x < MR) ssq[threadIdx.x] = 0.f;
-    __syncthreads();
-#pragma unroll
-    for (int m = 0; m < MR; ++m) {
-      const float s = warp_sum(sq[m]);
-      if (lane == 0) atomicAdd(&ssq[m], s);
-    }
-    cluster.sync();                                   // every CTA's partial sum of squares is in its `ssq`
-    float rstd[MR];
-#pragma unroll
-    for (int m = 0; m < MR; ++m) {
-      float t = 0.f;
-      for (int r = 0; r < S; ++r) t += cluster.map_shared_rank(ssq, r)[m];
-      rstd[m] = rsqrtf(t / static_cast<float>(K) + eps);
-    }
-    for (int i = threadIdx.x; i < MR * k8n * 4; i += WC_WARPS * 32) {       // pairs of elements
-      const int m = i / (k8n * 4), c = i - m * (k8n * 4);
-      uint32_t* p = reinterpret_cast<uint32_t*>(xs + (size_t)m * kslice) + c;
-      const uint32_t v = *p;
-      const float2 gm = *reinterpret_cast<const float2*>(gamma + kbase + 2 * c);
-      float r = 0.f;
-#pragma unroll
-      for (int mm = 0; mm < MR; ++mm) if (mm == m) r = rstd[mm];
-      *p = pack_bf16(bf16_lo(v) * r * gm.x, bf16_hi(v) * r * gm.y);
-    }
   }
   __syncthreads();
   // ---- stream my groups
@@ -567,7 +513,7 @@ w4_gemv_cluster_kernel(const __nv_bfloat16* __restrict__ x, const uint32_t* __re
     if (live) {
       float sc[CPL];
 #pragma unroll
-      for (int c = 0; c < CPL; ++c) sc[c] = __bfloat162float(scales[(long)g * N + n0 + c * cstride]);
+      for (int c = 0; c < CPL; ++c) sc[c] = __bfloat162float(scales[(long)g * N + n0 + c]);
       float pt[MR][CPL];
 #pragma unroll
       for (int m = 0; m < MR; ++m)
@@ -617,56 +563,7 @@ w4_gemv_cluster_kernel(const __nv_bfloat16* __restrict__ x, const uint32_t* __re
   }
   cluster.sync();                                       // all partial tiles are in shared memory
   bool released = false;
-  if (crank == 0 && GATED) {
-    const int I = N >> 1;
-    for (int i = threadIdx.x; i < MR * 32; i += WC_WARPS * 32) {
-      const int m = i >> 5, l = i & 31;
-      const int n = blockIdx.x * 32 + l;
-      float gt = 0.f, vl = 0.f;
-      for (int r = 0; r < S; ++r) {
-        const float* rp = cluster.map_shared_rank(part, r) + m * 64 + 2 * l;
-        gt += rp[0];
-        vl += rp[1 % CPL];
-      }
-      // the unfused path stores gate and value as bf16 before the activation
-      gt = __bfloat162float(__float2bfloat16(gt));
-      vl = __bfloat162float(__float2bfloat16(vl));
-      if (m < M && n < I) y[(long)m * I + n] = __float2bfloat16(gt / (1.f + __expf(-gt)) * vl);
-    }
-  } else if (crank == 0 && rope.cos_t != nullptr) {
-    // pairs of adjacent columns (interleaved rotary convention); columns of a CTA start on an even n
-    const int pos = min(*rope.pos_ptr, rope.cap - 1);
-    const int D = rope.D, half = D >> 1;
-    for (int i = threadIdx.x; i < MR * 16 * CPL; i += WC_WARPS * 32) {
-      const int m = i / (16 * CPL), c = 2 * (i - m * 16 * CPL);
-      const int n = blockIdx.x * 32 * CPL + c;
-      if (m >= M || n >= N) continue;
-      float a = 0.f, b = 0.f;
-      for (int r = 0; r < S; ++r) {
-        const float* rp = cluster.map_shared_rank(part, r) + m * 32 * CPL + c;
-        a += rp[0];
-        b += rp[1];
-      }
-      a = __bfloat162float(__float2bfloat16(a));        // the projection's output is bf16 before the rotation
-      b = __bfloat162float(__float2bfloat16(b));
-      const int h = n / D, d = n - h * D;
-      if (h < rope.Hq + rope.Hkv) {
-        const float cs = rope.cos_t[(long)pos * half + (d >> 1)], sn = rope.sin_t[(long)pos * half + (d >> 1)];
-        const float ra = a * cs - b * sn, rb = a * sn + b * cs;
-        a = ra;
-        b = rb;
-      }
-      const uint32_t packed = pack_bf16(a, b);
-      if (h < rope.Hq) {
-        *reinterpret_cast<uint32_t*>(y + (long)m * N + n) = packed;
-      } else {
-        const bool is_k = h < rope.Hq + rope.Hkv;
-        const int hk = is_k ? h - rope.Hq : h - rope.Hq - rope.Hkv;
-        __nv_bfloat16* dst = (is_k ? rope.kc : rope.vc) + (long)m * rope.c_sb + (long)pos * rope.c_ss + (long)hk * rope.c_sh + d;
-        *reinterpret_cast<uint32_t*>(dst) = packed;
-      }
-    }
-  } else if (crank == 0 && ar.world > 1) {
+  if (crank == 0 && ar.world > 1) {
     const long slot = 4 * ar.n_pad;
     const long poff = (long)(ar_epoch & 1u) * ar.world * slot;
     // (a) my partial of this column block into slot [rank] of every rank's inbox
@@ -728,22 +625,17 @@ w4_gemv_cluster_kernel(const __nv_bfloat16* __restrict__ x, const uint32_t* __re
   }
 }
 
-template <int MR, int CPL, bool GATED = false>
+template <int MR, int CPL>
 static int launch_w4_cluster(const void* x, const void* wk8, const void* scales, const void* residual, void* y, int M,
-                             int N, int K, long ldx, const float* gamma, float eps, cudaStream_t st,
-                             const RopeAppend* rope_args = nullptr, const ArFuse* ar_args = nullptr) {
-  RopeAppend rope = {};
-  if (rope_args) rope = *rope_args;
-  ArFuse ar = {};
-  if (ar_args) ar = *ar_args;
+                             int N, int K, long ldx, cudaStream_t st, const ArFuse& ar) {
   const int groups = K / 128;
-  const int blocks = GATED ? (N / 2 + 31) / 32 : (N + 32 * CPL - 1) / (32 * CPL);
+  const int blocks = (N + 32 * CPL - 1) / (32 * CPL);
   // split K until every warp still has a group and the grid holds about 6 CTAs (24 warps) per SM
   int S = 1;
   while (S < 8 && groups / (2 * S) >= WC_WARPS && (long)blocks * 2 * S <= 8L * num_sms()) S *= 2;
   const int gpc = (groups + S - 1) / S;
   const size_t smem = (size_t)MR * gpc * 128 * 2 + (size_t)(WC_WARPS + 1) * MR * 32 * CPL * 4 + 64;
-  auto kern = w4_gemv_cluster_kernel<MR, CPL, GATED>;
+  auto kern = w4_gemv_cluster_kernel<MR, CPL>;
   static size_t allowed = 48 * 1024;
   if (smem > allowed) {
     SB_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
@@ -767,27 +659,20 @@ static int launch_w4_cluster(const void* x, const void* wk8, const void* scales,
   cfg.numAttrs = 2;
   SB_CHECK_CUDA(cudaLaunchKernelEx(&cfg, kern, (const __nv_bfloat16*)x, (const uint32_t*)wk8,
                                    (const __nv_bfloat16*)scales, (const __nv_bfloat16*)residual, (__nv_bfloat16*)y, M,
-                                   N, K, ldx, gpc, gamma, eps, rope, ar));
+                                   N, K, ldx, gpc, ar));
   return SB_OK;
 }
 
 }  // namespace sb
 
-// As sb_w4_gemv_small, with the K range split over a thread-block cluster. gamma (fp32 [K]) != null
-// fuses y = rmsnorm(x; gamma, eps) @ W.
+// y[M,N] bf16 = x[M,K] @ dequant(k8-repacked int4 g128 weights) (+ residual), M <= 4, on the streaming kernel
+// (w4_stream.cu). gamma (fp32 [K]) != null fuses y = rmsnorm(x; gamma, eps) @ W. x and wk8 16-byte, scales 8-byte aligned.
 extern "C" int sb_w4_gemv_cluster(const void* x, const void* wk8, const void* scales, const void* residual, void* y,
                                   int M, int N, int K, long ldx, const float* gamma, float eps, cudaStream_t st) {
   SB_CHECK_ARG(M >= 1 && M <= 4 && K > 0 && K % 128 == 0 && N > 0 && N % 4 == 0 && ldx % 8 == 0);
-  const int sms = sb::num_sms();
-  const int cpl = (N / 128 >= 4 * sms) ? 4 : ((N / 64 >= 2 * sms && N % 64 == 0) ? 2 : 1);
-  const int mr = M <= 1 ? 1 : (M <= 2 ? 2 : 4);
-#define SB_W4C(MR, CPL) return sb::launch_w4_cluster<MR, CPL>(x, wk8, scales, residual, y, M, N, K, ldx, gamma, eps, st)
-  if (cpl == 4) { if (mr == 1) SB_W4C(1, 4); if (mr == 2) SB_W4C(2, 4); SB_W4C(4, 4); }
-  if (cpl == 2) { if (mr == 1) SB_W4C(1, 2); if (mr == 2) SB_W4C(2, 2); SB_W4C(4, 2); }
-  if (mr == 1) SB_W4C(1, 1);
-  if (mr == 2) SB_W4C(2, 1);
-  SB_W4C(4, 1);
-#undef SB_W4C
+  const sb::W4StreamArgs a = {(const __nv_bfloat16*)x, (const uint32_t*)wk8, (const __nv_bfloat16*)scales,
+                              (const __nv_bfloat16*)residual, (__nv_bfloat16*)y, M, N, K, ldx, gamma, eps, {}};
+  return sb::launch_w4_stream(a, sb::W4S_PLAIN, st);
 }
 
 // y[M, I] = silu(g) * v with [g | v] = (rmsnorm(x) or x) @ dequant(W[K, 2I]): the gated in-projection of a
@@ -795,9 +680,9 @@ extern "C" int sb_w4_gemv_cluster(const void* x, const void* wk8, const void* sc
 extern "C" int sb_w4_gemv_cluster_swiglu(const void* x, const void* wk8, const void* scales, void* y, int M, int N,
                                          int K, long ldx, const float* gamma, float eps, cudaStream_t st) {
   SB_CHECK_ARG(M >= 1 && M <= 4 && K > 0 && K % 128 == 0 && N > 0 && N % 8 == 0 && ldx % 8 == 0);
-  if (M <= 1) return sb::launch_w4_cluster<1, 2, true>(x, wk8, scales, nullptr, y, M, N, K, ldx, gamma, eps, st);
-  if (M <= 2) return sb::launch_w4_cluster<2, 2, true>(x, wk8, scales, nullptr, y, M, N, K, ldx, gamma, eps, st);
-  return sb::launch_w4_cluster<4, 2, true>(x, wk8, scales, nullptr, y, M, N, K, ldx, gamma, eps, st);
+  const sb::W4StreamArgs a = {(const __nv_bfloat16*)x, (const uint32_t*)wk8, (const __nv_bfloat16*)scales, nullptr,
+                              (__nv_bfloat16*)y, M, N, K, ldx, gamma, eps, {}};
+  return sb::launch_w4_stream(a, sb::W4S_GATED, st);
 }
 
 // The qkv projection of a decode step with its RoPE and KV-cache append in the epilogue: q heads are
@@ -813,9 +698,9 @@ extern "C" int sb_w4_gemv_cluster_rope(const void* x, const void* wk8, const voi
   r.cos_t = cos_t; r.sin_t = sin_t; r.kc = (__nv_bfloat16*)k_cache; r.vc = (__nv_bfloat16*)v_cache; r.pos_ptr = pos_ptr;
   r.Hq = Hq; r.Hkv = Hkv; r.D = D; r.cap = cap;
   r.c_sb = cache_strides[0]; r.c_ss = cache_strides[1]; r.c_sh = cache_strides[2];
-  if (M <= 1) return sb::launch_w4_cluster<1, 1>(x, wk8, scales, nullptr, y, M, N, K, ldx, gamma, eps, st, &r);
-  if (M <= 2) return sb::launch_w4_cluster<2, 1>(x, wk8, scales, nullptr, y, M, N, K, ldx, gamma, eps, st, &r);
-  return sb::launch_w4_cluster<4, 1>(x, wk8, scales, nullptr, y, M, N, K, ldx, gamma, eps, st, &r);
+  const sb::W4StreamArgs a = {(const __nv_bfloat16*)x, (const uint32_t*)wk8, (const __nv_bfloat16*)scales, nullptr,
+                              (__nv_bfloat16*)y, M, N, K, ldx, gamma, eps, r};
+  return sb::launch_w4_stream(a, sb::W4S_ROPE, st);
 }
 
 // ---------------------------------------------------------------------------- W4 GEMV, dequantisation into mma fragments
@@ -1361,7 +1246,7 @@ extern "C" int sb_w4_gemv_cluster_allreduce(const void* x, const void* wk8, cons
   ar.rank = rank; ar.world = world; ar.n_pad = n_pad;
   if (!ar.err) return sb::SB_ERR_CUDA;
   // one column-block width for all ranks and calls (the flags are per 32-column block): CPL = 1
-  if (M <= 1) return sb::launch_w4_cluster<1, 1>(x, wk8, scales, residual, y, M, N, K, ldx, nullptr, 0.f, st, nullptr, &ar);
-  if (M <= 2) return sb::launch_w4_cluster<2, 1>(x, wk8, scales, residual, y, M, N, K, ldx, nullptr, 0.f, st, nullptr, &ar);
-  return sb::launch_w4_cluster<4, 1>(x, wk8, scales, residual, y, M, N, K, ldx, nullptr, 0.f, st, nullptr, &ar);
+  if (M <= 1) return sb::launch_w4_cluster<1, 1>(x, wk8, scales, residual, y, M, N, K, ldx, st, ar);
+  if (M <= 2) return sb::launch_w4_cluster<2, 1>(x, wk8, scales, residual, y, M, N, K, ldx, st, ar);
+  return sb::launch_w4_cluster<4, 1>(x, wk8, scales, residual, y, M, N, K, ldx, st, ar);
 }

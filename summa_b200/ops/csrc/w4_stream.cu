@@ -1,0 +1,473 @@
+// 4-bit projection of a decode step, y[M,N] = x[M,K] @ dequant(W) for few rows (weights in the k8-repacked form of
+// quant.cu), as a register-prefetched weight stream feeding warp-level integer mma.
+//
+// What bounds it: the weight bytes, if the code words can be consumed in few instructions and enough of them are in
+// flight. Measured on a B200: a kernel that only loads the words of a 4096 x 28672 weight takes 14.0 us (6.3 TB/s plus
+// 4.6 us of launch and ramp) with 16 warps x 4 KB in flight per SM, and 20 us with 8 warps.
+//   * x is quantised EXACTLY ENOUGH instead of the weights being widened: per scale group of 128 k, x becomes a 22-bit
+//     fixed-point number (power-of-two step below 2^-21 of the group's largest magnitude, so every bf16 within a factor
+//     2^13 of it is exact) in three signed base-256 digits. A code word then needs one shift and two LOP3 to be the s8
+//     operands 16 (q - 8) of 8 k, against seven instructions for bf16 pairs, and ONE mma.m16n8k32 (s8, s32 accumulation,
+//     exact) takes 16 columns x 32 k of weights against 8 columns of digits. The products of a group are whole numbers;
+//     only the combination over groups rounds (fp32).
+//   * one CTA per SM walks a contiguous run of 16-column tiles over the whole K range; its 16 warps take the scale groups
+//     round robin, each through a ring of its own in shared memory that asynchronous copies fill D groups (D KB) ahead,
+//     across tiles; no barrier, no producer. (A ring in registers is held up by whatever touches a loaded register
+//     early: a scale that was combined on arrival cost 27 us instead of 21.6, spilled ring registers 28 us, N 28672.)
+//   * per tile every warp leaves its partial sums in one of four shared-memory buffers and streams on; the warp whose
+//     turn it is adds them and runs the epilogue two tiles later (mbarriers both ways). With one block barrier and an
+//     immediate epilogue per tile its latency was paid per tile. No cluster, no atomics.
+//   * the weights depend on nothing, so the first groups are requested before `griddepcontrol.wait`.
+// Measured against the CUDA-core cluster kernel it replaces (weights from HBM, graph of launches, one row): K 4096 N 6144
+// 12.0 -> 7.5 us, N 4096 7.4 -> 6.1, N 28672 28.9 -> 21.1 (gated with norm 33.2 -> 23.5), N 32000 30.2 -> 22.6, K 14336
+// N 4096 19.9 -> 13.0; four rows: 20.0 -> 10.4, 14.6 -> 8.6, 60.7 -> 27.2, 66.0 -> 28.7, 41.6 -> 23.5. Relative error
+// against 64 bits: the same 0.00165 (the rounding of y to bf16).
+#include "host_util.h"
+#include "sm100.cuh"
+#include "w4_stream.h"
+
+namespace sb {
+
+constexpr int W4S_WARPS = 16, W4S_THREADS = 512, W4S_TILE = 16, W4S_NB = 4;
+constexpr int W4S_SMEM = 220 * 1024;
+
+__device__ __forceinline__ void w4s_mma(int (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
+                                        uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, "
+               "{%0, %1, %2, %3};"
+               : "+r"(d[0]), "+r"(d[1]), "+r"(d[2]), "+r"(d[3])
+               : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ void w4s_copy8(uint32_t dst_smem, const void* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst_smem), "l"(reinterpret_cast<uint64_t>(src)) : "memory");
+}
+// codes of k 0,4,1,5 / 2,6,3,7 of a word as s8 bytes 16 (q - 8)
+__device__ __forceinline__ uint32_t w4s_lo(uint32_t w) { return ((w << 4) & 0xF0F0F0F0u) ^ 0x80808080u; }
+__device__ __forceinline__ uint32_t w4s_hi(uint32_t w) { return (w & 0xF0F0F0F0u) ^ 0x80808080u; }
+
+template <int MT> constexpr int W4S_X_BYTES = MT == 0 ? 84 * 1024 : 104 * 1024;     // digits of x of one K pass
+template <int MT> constexpr int W4S_DEPTH = MT == 0 ? 6 : 4;
+constexpr int W4S_MAGIC = 0x4B400000;        // float bits of 1.5 * 2^23: adding a small integer to the bits adds it to the value
+
+// MT = 0: up to two rows, their 3 M digits are the columns of one mma. MT = 1: up to eight rows, one mma per digit.
+constexpr int W4S_SLOT = 1024 + 32;           // a group of a tile: 16 k8 rows x 64 bytes (chunks swizzled), 16 scales
+struct W4SLayout {                           // shared memory, in bytes
+  int ring, pitch, sx, red, psum, gsq, total;   // pitch: digit row of x (32 mod 128: conflict-free B loads)
+};
+__host__ __device__ inline W4SLayout w4s_layout(int rows, int depth, int M, int pass_groups, int groups, bool norm, int psum_tiles) {
+  W4SLayout l;
+  l.ring = 3 * M * (pass_groups * 128 + 32);                       // [warps][depth] slots
+  l.pitch = pass_groups * 128 + 32;
+  l.sx = l.ring + W4S_WARPS * depth * W4S_SLOT;                                           // [pass_groups][rows] fp32
+  l.red = l.sx + pass_groups * rows * 4;                            // [buffers][warps][rows][16] fp32
+  l.psum = l.red + W4S_NB * W4S_WARPS * rows * W4S_TILE * 4;             // [psum_tiles][M][16] fp32 (more than one K pass)
+  l.gsq = l.psum + psum_tiles * M * W4S_TILE * 4;                   // [M] rstd, [M][groups] sums of squares
+  l.total = l.gsq + (norm ? (M + M * groups) * 4 : 0);
+  return l;
+}
+
+template <int MT, int MODE>
+__global__ void __launch_bounds__(W4S_THREADS, 1)
+w4_stream_kernel(const W4StreamArgs p, const int tile_base, const int tiles, const int pass_groups, const int psum_tiles,
+                 unsigned int* err) {
+  constexpr bool COMPACT = MT == 0;
+  constexpr int SETS = COMPACT ? 1 : MT;      // accumulator sets (8 columns of digits or 8 rows each)
+  constexpr int DIG = COMPACT ? 1 : 3;
+  constexpr int ROWS = 8 * SETS;
+  constexpr int D = W4S_DEPTH<MT>;            // units (scale groups) in flight per warp
+  extern __shared__ __align__(128) unsigned char w4s_smem[];
+  __shared__ uint64_t full[W4S_NB], empty[W4S_NB];
+  __shared__ int abort_flag;
+  asm volatile("griddepcontrol.launch_dependents;");
+  const int M = p.M, N = p.N, K = p.K;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gq = lane >> 2, tq = lane & 3;
+  const int groups = K >> 7;
+  const W4SLayout L = w4s_layout(ROWS, D, M, pass_groups, groups, p.gamma != nullptr, psum_tiles);
+  unsigned char* xq = w4s_smem;
+  float* sx = reinterpret_cast<float*>(w4s_smem + L.sx);
+  float* red = reinterpret_cast<float*>(w4s_smem + L.red);
+  float* psum = reinterpret_cast<float*>(w4s_smem + L.psum);
+  float* rstd = reinterpret_cast<float*>(w4s_smem + L.gsq);
+  float* gsq = rstd + M;
+  const int t_lo = tile_base + (int)((long)blockIdx.x * tiles / gridDim.x);
+  const int t_hi = tile_base + (int)((long)(blockIdx.x + 1) * tiles / gridDim.x);
+  const int I = N >> 1;                       // gated: columns of the gate half
+  const int passes = (groups + pass_groups - 1) / pass_groups;
+  constexpr int TILE_COLS = MODE == W4S_GATED ? 8 : W4S_TILE;       // columns (gated: gate columns) of a tile
+  const int cols = MODE == W4S_GATED ? I : N;
+
+  if (threadIdx.x == 0) {
+    for (int b = 0; b < W4S_NB; ++b) { mbar_init(&full[b], W4S_WARPS); mbar_init(&empty[b], (W4S_TILE * M + 31) / 32); }
+    abort_flag = 0;
+    fence_barrier_init();
+  }
+  __syncthreads();
+
+  // Epilogue of this CTA's q-th tile (counted over the passes): 32 outputs o = m * 16 + c at a time; chunk k of tile ct
+  // belongs to warp (ct + k) % 16, which runs it two tiles later, when the other warps have long handed theirs over.
+  const int chunks = (W4S_TILE * M + 31) / 32, ntiles = t_hi - t_lo;
+  auto epilogue = [&](int q) {
+    const int pass = q / ntiles, ct = t_lo + q - pass * ntiles;
+    const int chunk = (warp - ct) & (W4S_WARPS - 1);
+    if (chunk >= chunks) return;
+    const bool last = pass + 1 == passes;
+    const float* rb = red + (q & (W4S_NB - 1)) * W4S_WARPS * ROWS * W4S_TILE;
+    const int o = chunk * 32 + lane, m = o >> 4, c = o & 15;
+    const bool row = m < M;
+    const int mm = row ? m : 0;
+    const int n = MODE == W4S_GATED ? ct * 8 + (c >> 1) : ct * W4S_TILE + c;
+    float rv = 0.f;
+    if (MODE == W4S_PLAIN && last && p.residual != nullptr && row && n < N)
+      rv = bf16_lo(__ldcg(reinterpret_cast<const unsigned short*>(p.residual) + (long)m * N + n));
+    if (!mbar_wait(&full[q & (W4S_NB - 1)], (q / W4S_NB) & 1, &abort_flag, err)) return;
+    float v = 0.f;
+#pragma unroll
+    for (int w = 0; w < W4S_WARPS; ++w) {
+      if (COMPACT) {
+        const float* r = rb + (w * ROWS + 3 * mm) * W4S_TILE + c;
+        v += r[0] + r[W4S_TILE] + r[2 * W4S_TILE];
+      } else {
+        v += rb[(w * ROWS + mm) * W4S_TILE + c];
+      }
+    }
+    if (passes > 1) {
+      float* ps = psum + ((ct - t_lo) * M + mm) * W4S_TILE + c;
+      if (pass > 0 && row) v += *ps;
+      if (!last && row) *ps = v;
+    }
+    if (!last) {
+    } else if (MODE == W4S_GATED) {
+      // the unfused path stores gate and value as bf16 before the activation
+      v = __bfloat162float(__float2bfloat16(v));
+      const float val = __shfl_xor_sync(0xffffffffu, v, 1);
+      if (row && !(c & 1) && n < I) p.y[(long)m * I + n] = __float2bfloat16(v / (1.f + __expf(-v)) * val);
+    } else if (MODE == W4S_ROPE) {
+      // pairs of adjacent columns (interleaved rotary convention); the projection's output is bf16 before the rotation
+      const RopeAppend& rp = p.rope;
+      v = __bfloat162float(__float2bfloat16(v));
+      const float u = __shfl_xor_sync(0xffffffffu, v, 1);
+      if (row && !(c & 1) && n < N) {
+        const int pos = min(*reinterpret_cast<const volatile int*>(rp.pos_ptr), rp.cap - 1);
+        const int h = n / rp.D, dcol = n - h * rp.D;
+        float a = v, b = u;
+        if (h < rp.Hq + rp.Hkv) {
+          const long at = (long)pos * (rp.D >> 1) + (dcol >> 1);
+          const float cs = rp.cos_t[at], sn = rp.sin_t[at];
+          a = v * cs - u * sn;
+          b = v * sn + u * cs;
+        }
+        __nv_bfloat16* dst;
+        if (h < rp.Hq) {
+          dst = p.y + (long)m * N + n;
+        } else {
+          const bool is_k = h < rp.Hq + rp.Hkv;
+          const int hk = is_k ? h - rp.Hq : h - rp.Hq - rp.Hkv;
+          dst = (is_k ? rp.kc : rp.vc) + (long)m * rp.c_sb + (long)pos * rp.c_ss + (long)hk * rp.c_sh + dcol;
+        }
+        *reinterpret_cast<uint32_t*>(dst) = pack_bf16(a, b);
+      }
+    } else if (row && n < N) {
+      p.y[(long)m * N + n] = __float2bfloat16(v + rv);
+    }
+    __syncwarp();
+    if (lane == 0) mbar_arrive(&empty[q & (W4S_NB - 1)]);
+  };
+  int handed = 0;                             // tiles handed over so far
+
+  // ---- the warp's ring. Copy: lane moves chunks (row lane / 4, chunk lane % 4) and (row + 8, same chunk); read: lane
+  // (g, t) takes its two columns of k8 rows 4 j + t. Chunk c of row r lies at c ^ (r & 2), which makes both conflict-free.
+  const uint32_t ring = smem_u32(w4s_smem + L.ring) + warp * (D * W4S_SLOT);
+  const int cr = lane >> 2, cc = lane & 3;
+  const int ccol = MODE == W4S_GATED ? (cc < 2 ? 4 * cc : I + 4 * (cc - 2)) : 4 * cc;        // first column of the chunk
+  const uint32_t cdst = cr * 64 + ((cc ^ (cr & 2)) << 4);
+  const uint32_t rsrc = MODE == W4S_GATED ? tq * 64 + (((gq >> 2) ^ (tq & 2)) << 4) + (gq & 3) * 4
+                                          : tq * 64 + (((gq >> 1) ^ (tq & 2)) << 4) + (gq & 1) * 8;
+  int lt, li, lmine, lgpw;                    // load cursor: tile, unit of this warp; valid units, units per tile
+  uint32_t lslot = 0;
+  const uint32_t* lw;
+  const __nv_bfloat16* ls;
+  auto rewind = [&](int g0) {                 // cursor to the first unit of tile lt
+    lw = p.wk8 + (long)(16 * (g0 + warp) + cr) * N + (long)lt * TILE_COLS + ccol;
+    ls = p.scales + (long)(g0 + warp) * N + (long)lt * TILE_COLS + ccol;
+  };
+  auto load = [&](int g0) {
+    if (lt < t_hi && li < lmine) {
+      const bool live = lt * TILE_COLS + (MODE == W4S_GATED ? 4 * (cc & 1) : 4 * cc) < cols;   // (columns come in fours)
+      const uint32_t dst = ring + lslot * W4S_SLOT;
+      cp_async16_zfill(dst + cdst, live ? lw : p.wk8, live ? 16 : 0);
+      cp_async16_zfill(dst + cdst + 512, live ? lw + 8L * N : p.wk8, live ? 16 : 0);
+      if (cr == 0 && live) w4s_copy8(dst + 1024 + 8 * cc, ls);
+    }
+    cp_async_commit();
+    lslot = lslot + 1 == D ? 0 : lslot + 1;
+    lw += (long)(16 * W4S_WARPS) * N;
+    ls += (long)W4S_WARPS * N;
+    if (++li == lgpw) {
+      li = 0;
+      ++lt;
+      rewind(g0);
+    }
+  };
+
+  for (int pass = 0; pass < passes; ++pass) {
+    const int g0 = pass * pass_groups, g1 = min(groups, g0 + pass_groups), ng = g1 - g0;
+    const int gpw = (ng + W4S_WARPS - 1) / W4S_WARPS;
+    const int mine = (ng - warp + W4S_WARPS - 1) / W4S_WARPS;
+    const int total = (t_hi - t_lo) * gpw;
+    lt = t_lo; li = 0; lmine = mine; lgpw = gpw;
+    rewind(g0);
+    lslot = 0;
+    for (int d = 0; d < D; ++d) load(g0);
+    // ---- x: (fused norm) -> digits and steps of this pass; half a warp takes one (row, group)
+    const int l16 = threadIdx.x & 15;
+    uint4 v[4];
+    bool kept = false;                        // v holds this half-warp's items already
+    if (pass == 0) {
+      if (p.gamma != nullptr)                 // the gains come from HBM in a decode step; ask for them early as well
+        for (int i = threadIdx.x; i < K / 32; i += 32 * W4S_WARPS)
+          asm volatile("prefetch.global.L2 [%0];" ::"l"(p.gamma + 32 * i));
+      asm volatile("griddepcontrol.wait;" ::: "memory");
+      if (p.gamma != nullptr) {
+        for (int i1 = 2 * warp; i1 < M * groups; i1 += 4 * 32) {               // (the warp's two halves stay together)
+          const int i0 = i1 + (lane >> 4);
+          kept = passes == 1 && M * groups <= 128;
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            const int i = i0 + 32 * q, m = i / groups, g = i - m * groups;
+            v[q] = i < M * groups ? __ldcg(reinterpret_cast<const uint4*>(p.x + (long)m * p.ldx + g * 128) + l16) : make_uint4(0u, 0u, 0u, 0u);
+          }
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            const float a0 = bf16_lo(v[q].x), a1 = bf16_hi(v[q].x), a2 = bf16_lo(v[q].y), a3 = bf16_hi(v[q].y);
+            const float a4 = bf16_lo(v[q].z), a5 = bf16_hi(v[q].z), a6 = bf16_lo(v[q].w), a7 = bf16_hi(v[q].w);
+            float s = a0 * a0 + a1 * a1 + a2 * a2 + a3 * a3 + a4 * a4 + a5 * a5 + a6 * a6 + a7 * a7;
+#pragma unroll
+            for (int o = 8; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+            if (l16 == 0 && i0 + 32 * q < M * groups) gsq[i0 + 32 * q] = s;
+          }
+        }
+        __syncthreads();
+        for (int m = warp; m < M; m += W4S_WARPS) {
+          float s = 0.f;
+          for (int g = lane; g < groups; g += 32) s += gsq[m * groups + g];
+          s = warp_sum(s);
+          if (lane == 0) rstd[m] = rsqrtf(s / static_cast<float>(K) + p.eps);
+        }
+      }
+    }
+    for (int i = threadIdx.x; i < ng * ROWS; i += 32 * W4S_WARPS) sx[i] = 0.f;    // rows beyond M
+    __syncthreads();                                                             // (pass > 0: nobody reads the old digits any more)
+    for (int i1 = 2 * warp; i1 < M * ng; i1 += 4 * 32) {
+      const int i0 = i1 + (lane >> 4);
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const int i = i0 + 32 * q, m = i / ng, gl = i - m * ng;
+        if (!kept) v[q] = i < M * ng ? __ldcg(reinterpret_cast<const uint4*>(p.x + (long)m * p.ldx + (g0 + gl) * 128) + l16) : make_uint4(0u, 0u, 0u, 0u);
+      }
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        if (i1 + 32 * q >= M * ng) break;
+        const int i = min(i0 + 32 * q, M * ng - 1), m = i / ng, gl = i - m * ng;
+        uint32_t u[4] = {v[q].x, v[q].y, v[q].z, v[q].w};
+        if (p.gamma != nullptr) {
+          const float r = rstd[m];
+          const float2* gp = reinterpret_cast<const float2*>(p.gamma + (g0 + gl) * 128 + 8 * l16);
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const float2 gm = __ldg(gp + e);
+            u[e] = pack_bf16(bf16_lo(u[e]) * r * gm.x, bf16_hi(u[e]) * r * gm.y);
+          }
+        }
+        // largest magnitude of the group, as bf16 bits (NaN > Inf > finite as unsigned numbers)
+        uint32_t mx = __vmaxu2(__vmaxu2(u[0] & 0x7FFF7FFFu, u[1] & 0x7FFF7FFFu), __vmaxu2(u[2] & 0x7FFF7FFFu, u[3] & 0x7FFF7FFFu));
+        mx = max(mx & 0xFFFFu, mx >> 16);
+#pragma unroll
+        for (int o = 8; o > 0; o >>= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+        const bool finite = mx < 0x7F80u;
+        const uint32_t E = max(mx >> 7, 27u);                       // biased exponent; |x| < 2^(E - 126)
+        const float inv = __uint_as_float((274u - min(E, 254u)) << 23);          // 2^(20 - (E - 127)): |x inv| < 2^21
+        uint32_t y[8];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const float a = finite ? bf16_lo(u[e]) : 0.f, b = finite ? bf16_hi(u[e]) : 0.f;
+          y[2 * e] = (__float_as_uint(fmaf(a, inv, 12582912.f)) - (uint32_t)W4S_MAGIC + 0x808080u) ^ 0x808080u;
+          y[2 * e + 1] = (__float_as_uint(fmaf(b, inv, 12582912.f)) - (uint32_t)W4S_MAGIC + 0x808080u) ^ 0x808080u;
+        }
+        if (i0 + 32 * q < M * ng) {
+#pragma unroll
+          for (int d = 0; d < 3; ++d) {
+            const uint32_t sel = d | ((4 + d) << 4);
+            const uint32_t b0 = __byte_perm(__byte_perm(y[0], y[4], sel), __byte_perm(y[1], y[5], sel), 0x5410);
+            const uint32_t b1 = __byte_perm(__byte_perm(y[2], y[6], sel), __byte_perm(y[3], y[7], sel), 0x5410);
+            *reinterpret_cast<uint2*>(xq + (3 * m + d) * L.pitch + gl * 128 + 8 * l16) = make_uint2(b0, b1);
+          }
+          const float step = finite ? __uint_as_float((E - 24u) << 23) : __uint_as_float(0x7FC00000u);   // 2^(E - 127 - 20) / 16
+          if (l16 < (COMPACT ? 3 : 1))
+            sx[gl * ROWS + (COMPACT ? 3 * m + l16 : m)] = step * (l16 == 0 ? 1.f : (l16 == 1 ? 256.f : 65536.f));
+        }
+      }
+    }
+    __syncthreads();
+
+    // ---- the stream
+    float acc[SETS][4];
+#pragma unroll
+    for (int n = 0; n < SETS; ++n)
+#pragma unroll
+      for (int c = 0; c < 4; ++c) acc[n][c] = 0.f;
+    int ci = 0;                               // consume cursor: unit of the tile
+    uint32_t slot = 0;
+    for (int it = 0; it < total; ++it) {
+      cp_async_wait_group<D - 1>();
+      __syncwarp();
+      if (ci < mine) {
+        const unsigned char* sl = w4s_smem + L.ring + (warp * D + slot) * W4S_SLOT;
+        const int gl = warp + W4S_WARPS * ci;
+        int dd[SETS][DIG][4];
+#pragma unroll
+        for (int n = 0; n < SETS; ++n)
+#pragma unroll
+          for (int q = 0; q < DIG; ++q)
+#pragma unroll
+            for (int c = 0; c < 4; ++c) dd[n][q][c] = W4S_MAGIC;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          uint32_t w0, w1;
+          if (MODE == W4S_GATED) {
+            w0 = *reinterpret_cast<const uint32_t*>(sl + rsrc + 256 * j);
+            w1 = *reinterpret_cast<const uint32_t*>(sl + (rsrc ^ 32u) + 256 * j);
+          } else {
+            const uint2 w = *reinterpret_cast<const uint2*>(sl + rsrc + 256 * j);
+            w0 = w.x;
+            w1 = w.y;
+          }
+          const uint32_t a0 = w4s_lo(w0), a1 = w4s_lo(w1), a2 = w4s_hi(w0), a3 = w4s_hi(w1);
+#pragma unroll
+          for (int n = 0; n < SETS; ++n) {
+#pragma unroll
+            for (int q = 0; q < DIG; ++q) {
+              const int row = COMPACT ? gq : 3 * (8 * n + gq) + q;
+              const uint2 xb = row < 3 * M ? *reinterpret_cast<const uint2*>(xq + row * L.pitch + gl * 128 + 8 * (4 * j + tq))
+                                           : make_uint2(0u, 0u);
+              w4s_mma(dd[n][q], a0, a1, a2, a3, xb.x, xb.y);
+            }
+          }
+        }
+        float s0, s1;
+        if (MODE == W4S_GATED) {
+          s0 = bf16_lo(*reinterpret_cast<const unsigned short*>(sl + 1024 + 2 * gq));
+          s1 = bf16_lo(*reinterpret_cast<const unsigned short*>(sl + 1040 + 2 * gq));
+        } else {
+          const uint32_t w = *reinterpret_cast<const uint32_t*>(sl + 1024 + 4 * gq);
+          s0 = bf16_lo(w);
+          s1 = bf16_hi(w);
+        }
+#pragma unroll
+        for (int n = 0; n < SETS; ++n) {
+          const float2 st = *reinterpret_cast<const float2*>(sx + gl * ROWS + 8 * n + 2 * tq);
+          float f[4];
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {
+            f[c] = __int_as_float(dd[n][DIG - 1][c]) - 12582912.f;
+#pragma unroll
+            for (int q = DIG - 2; q >= 0; --q) f[c] = fmaf(f[c], 256.f, __int_as_float(dd[n][q][c]) - 12582912.f);
+          }
+          acc[n][0] = fmaf(f[0], s0 * st.x, acc[n][0]);            // first column, x columns 2 t, 2 t + 1
+          acc[n][1] = fmaf(f[1], s0 * st.y, acc[n][1]);
+          acc[n][2] = fmaf(f[2], s1 * st.x, acc[n][2]);            // second column
+          acc[n][3] = fmaf(f[3], s1 * st.y, acc[n][3]);
+        }
+      }
+      __syncwarp();                         // everyone has read the slot
+      load(g0);
+      slot = slot + 1 == D ? 0 : slot + 1;
+      if (++ci < gpw) continue;
+      // ---- tile done: hand this warp's sums over
+      ci = 0;
+      const int hb = handed & (W4S_NB - 1);
+      if (handed >= W4S_NB && !mbar_wait(&empty[hb], ((handed / W4S_NB) - 1) & 1, &abort_flag, err)) return;
+#pragma unroll
+      for (int n = 0; n < SETS; ++n) {
+        float* r = red + ((hb * W4S_WARPS + warp) * ROWS + 8 * n + 2 * tq) * W4S_TILE + 2 * gq;
+        *reinterpret_cast<float2*>(r) = make_float2(acc[n][0], acc[n][2]);
+        *reinterpret_cast<float2*>(r + W4S_TILE) = make_float2(acc[n][1], acc[n][3]);
+        acc[n][0] = acc[n][1] = acc[n][2] = acc[n][3] = 0.f;
+      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&full[hb]);
+      if (++handed > 2) epilogue(handed - 3);
+    }
+    cp_async_wait_all();
+    if (pass + 1 < passes) __syncthreads();   // every warp is done with the digits
+  }
+  for (int q = max(handed - 2, 0); q < handed; ++q) epilogue(q);
+}
+
+template <int MT, int MODE>
+static int w4s_launch(const W4StreamArgs& a, cudaStream_t st) {
+  constexpr int ROWS = MT == 0 ? 8 : 8 * MT;
+  const int groups = a.K / 128;
+  const bool norm = a.gamma != nullptr;
+  const int tiles = MODE == W4S_GATED ? (a.N / 2 + 7) / 8 : (a.N + W4S_TILE - 1) / W4S_TILE;
+  // K passes: the digits of a pass stay in shared memory while the CTA walks its tiles
+  const int fit = W4S_X_BYTES<MT> / (a.M * 3 * 128);
+  const int passes = (groups + fit - 1) / fit;
+  int pass_groups = (groups + passes - 1) / passes;
+  if (passes > 1) {             // whole rounds of the warps
+    pass_groups = (pass_groups + W4S_WARPS - 1) / W4S_WARPS * W4S_WARPS;
+    if (pass_groups > fit) pass_groups = fit < W4S_WARPS ? fit : fit / W4S_WARPS * W4S_WARPS;
+  }
+  const int base_smem = w4s_layout(ROWS, W4S_DEPTH<MT>, a.M, pass_groups, groups, norm, 0).total;
+  int most = tiles;
+  if (pass_groups < groups)     // partial sums wait in shared memory: as many tiles per CTA as fit, the rest in further launches
+    most = (W4S_SMEM - base_smem) / (a.M * W4S_TILE * 4) * num_sms();
+  SB_CHECK_ARG(base_smem <= W4S_SMEM && most > 0);
+  unsigned int* err = error_word();
+  if (!err) return SB_ERR_CUDA;
+  auto kern = w4_stream_kernel<MT, MODE>;
+  static bool attr_set[64] = {false};
+  int dev = 0;
+  SB_CHECK_CUDA(cudaGetDevice(&dev));
+  if (!attr_set[dev & 63]) {
+    SB_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, W4S_SMEM));
+    attr_set[dev & 63] = true;
+  }
+  for (int t0 = 0; t0 < tiles; t0 += most) {
+    const int nt = tiles - t0 < most ? tiles - t0 : most;
+    const int grid = nt < num_sms() ? nt : num_sms();
+    const int psum_tiles = pass_groups < groups ? (nt + grid - 1) / grid : 0;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid, 1, 1);
+    cfg.blockDim = dim3(W4S_THREADS, 1, 1);
+    cfg.dynamicSmemBytes = w4s_layout(ROWS, W4S_DEPTH<MT>, a.M, pass_groups, groups, norm, psum_tiles).total;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    // programmatic dependent launch: this grid may start while its predecessor in the stream still runs; before
+    // `griddepcontrol.wait` it only reads weights, and it writes nothing
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    SB_CHECK_CUDA(cudaLaunchKernelEx(&cfg, kern, a, t0, nt, pass_groups, psum_tiles, err));
+  }
+  return SB_OK;
+}
+
+bool w4_stream_one_pass(int M, int K) { return (long)M * 3 * K <= (M <= 2 ? W4S_X_BYTES<0> : W4S_X_BYTES<1>); }
+
+int launch_w4_stream(const W4StreamArgs& a, W4StreamMode mode, cudaStream_t st) {
+  SB_CHECK_ARG(a.M >= 1 && a.M <= W4S_MAX_ROWS && a.K > 0 && a.K % 128 == 0 && a.N > 0 && a.N % 4 == 0 && a.ldx % 8 == 0);
+  SB_CHECK_ARG(((reinterpret_cast<uintptr_t>(a.wk8) | reinterpret_cast<uintptr_t>(a.x)) & 15) == 0 && (reinterpret_cast<uintptr_t>(a.scales) & 7) == 0);
+  if (mode == W4S_GATED) {
+    SB_CHECK_ARG(a.M <= 8 && a.N % 8 == 0);
+    return a.M <= 2 ? w4s_launch<0, W4S_GATED>(a, st) : w4s_launch<1, W4S_GATED>(a, st);
+  }
+  if (mode == W4S_ROPE) {
+    SB_CHECK_ARG(a.M <= 8);
+    return a.M <= 2 ? w4s_launch<0, W4S_ROPE>(a, st) : w4s_launch<1, W4S_ROPE>(a, st);
+  }
+  if (a.M <= 2) return w4s_launch<0, W4S_PLAIN>(a, st);
+  return w4s_launch<1, W4S_PLAIN>(a, st);
+}
+
+}  // namespace sb

@@ -1059,13 +1059,19 @@ N.register("sb_w4_gemv_small", [N.P] * 5 + [N.I, N.I, N.I, N.L, N.P])
 N.register("sb_w4_gemv_cluster", [N.P] * 5 + [N.I, N.I, N.I, N.L, N.P, N.F, N.P])
 N.register("sb_w4_gemv_mma", [N.P] * 5 + [N.I, N.I, N.I, N.L, N.P, N.F, N.P])
 N.register("sb_w4_gemv_stream", [N.P] * 5 + [N.I, N.I, N.I, N.L, N.P, N.F, N.I, N.P])
-# "cluster" (default): the CUDA-core GEMV with cluster split-K; "mma": nibble pairs go straight into warp-level
-# mma fragments (1..8 rows). Measured on the 7B decode step: 348 tokens/s with "cluster", 124 with "mma".
+# "cluster" (default): the streaming integer-mma kernel (w4_stream.cu); "mma" / "stream": the older bf16-mma forms, which
+# expand every code to bf16 (slower at every decode shape; kept as independent implementations for the tests).
 W4_GEMV_KERNEL = os.environ.get("SUMMA_W4_GEMV", "cluster")
 N.register("sb_w4_gemv_cluster_swiglu", [N.P] * 4 + [N.I, N.I, N.I, N.L, N.P, N.F, N.P])
 
 
 N.register("sb_w4_gemv_cluster_rope", [N.P] * 4 + [N.I, N.I, N.I, N.L, N.P, N.F] + [N.P] * 5 + [N.I, N.I, N.I, N.P, N.I, N.P])
+
+
+def _w4_operands(packed_k8: torch.Tensor, scales: torch.Tensor):
+    """The streaming kernel copies codes in 16-byte and scales in 8-byte pieces; a view that starts elsewhere is copied."""
+    return (packed_k8 if packed_k8.data_ptr() % 16 == 0 else packed_k8.clone(),
+            scales if scales.data_ptr() % 8 == 0 else scales.clone())
 
 
 def int4_gemv_rope_append(x, packed_k8, scales, norm, cos, sin, k_cache, v_cache, pos, Hq, Hkv, D, cap):
@@ -1080,6 +1086,7 @@ def int4_gemv_rope_append(x, packed_k8, scales, norm, cos, sin, k_cache, v_cache
         x2 = rmsnorm(x2, norm[0], norm[1])
         ldx = x2.stride(0)
     y = torch.empty(M, Nn, device=x.device, dtype=BF16)
+    packed_k8, scales = _w4_operands(packed_k8, scales)
     cs = (ctypes.c_long * 3)(k_cache.stride(0), k_cache.stride(1), k_cache.stride(2))
     N.call("sb_w4_gemv_cluster_rope", x2.data_ptr(), packed_k8.data_ptr(), scales.data_ptr(), y.data_ptr(), M, Nn, K,
            ldx, norm[0].data_ptr() if fuse else None, float(norm[1]) if fuse else 0.0, cos.data_ptr(), sin.data_ptr(),
@@ -1097,6 +1104,7 @@ def int4_gemv_swiglu(x, packed_k8, scales, norm=None):
     if norm is not None and not fuse:
         x2 = rmsnorm(x2, norm[0], norm[1])
         ldx = x2.stride(0)
+    packed_k8, scales = _w4_operands(packed_k8, scales)
     y = torch.empty(M, Nn // 2, device=x.device, dtype=BF16)
     N.call("sb_w4_gemv_cluster_swiglu", x2.data_ptr(), packed_k8.data_ptr(), scales.data_ptr(), y.data_ptr(), M, Nn, K,
            ldx, norm[0].data_ptr() if fuse else None, float(norm[1]) if fuse else 0.0, N.stream())
@@ -1113,6 +1121,8 @@ def int4_gemv(x, packed, scales, residual=None, packed_k8=None, norm=None):
     x2, ldx = _rows(x)
     y = torch.empty(M, Nn, device=x.device, dtype=BF16)
     res = residual.contiguous() if residual is not None else None
+    if packed_k8 is not None and M <= 8:
+        packed_k8, scales = _w4_operands(packed_k8, scales)
     use_mma = W4_GEMV_KERNEL == "mma"
     if (W4_GEMV_KERNEL == "stream" and packed_k8 is not None and M <= 4 and ldx % 8 == 0 and x2.data_ptr() % 16 == 0
             and K % 128 == 0 and Nn % 4 == 0 and K <= 16384):

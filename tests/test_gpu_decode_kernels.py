@@ -1,0 +1,71 @@
+"""Kernels of a decode step at the sizes where their dispatch, tiles and remainders change."""
+import pytest
+import torch
+
+gpu = pytest.mark.gpu
+
+
+def _w4(K, N, seed):
+    from summa_b200.ops import reference
+    torch.manual_seed(seed)
+    packed, scales = reference.quantize_int4_g128(torch.randn(K, N) * 0.05)
+    packed, scales = packed.cuda(), scales.cuda()
+    return packed, scales, reference.repack_int4_k8(packed), reference.dequantize_int4_g128(packed.cpu(), scales.cpu()).double().cuda()
+
+
+@gpu
+@pytest.mark.parametrize("M,K,N", [
+    (1, 128, 4), (2, 256, 20), (3, 2048, 16), (1, 2176, 132), (8, 1920, 68),        # one group; fewer and more than 16 groups; ragged tiles
+    (2, 14464, 36), (1, 20480, 28), (4, 9088, 44), (8, 4352, 2400),                 # K in passes / the last that fits one pass
+    (8, 4736, 52), (5, 14336, 40)])                                                 # rows 5..8 beyond one pass: the other kernel
+@pytest.mark.parametrize("spread", [0, 24])
+def test_w4_projection_against_fp64(M, K, N, spread):
+    """x spreads over 2^-spread .. 1: a group's fixed-point step is 2^-21 of its largest magnitude, so a product is off by at
+    most 2^-21 max|x| |w| per term, next to fp32 sums (2^-20 of the terms' sum is above both) and one rounding to bf16."""
+    from summa_b200 import ops
+    packed, scales, k8, wq = _w4(K, N, M + K + N)
+    x = (torch.randn(M, K, device="cuda") * torch.exp2(-spread * torch.rand(M, K, device="cuda"))).to(torch.bfloat16)
+    res = torch.randn(M, N, device="cuda").to(torch.bfloat16)
+    ref = x.double() @ wq
+    big = x.double().view(M, K // 128, 128).abs().amax(-1, keepdim=True).expand(M, K // 128, 128).reshape(M, K)
+    slack = 2.0 ** -20 * (big @ wq.abs())
+    if M > 4 and 3 * M * K > 104 * 1024:                                            # that kernel rounds the weights to bf16
+        slack += 2.0 ** -9 * (x.double().abs() @ wq.abs())
+    for got, want in ((ops.int4_gemv(x, packed, scales, None, k8), ref), (ops.int4_gemv(x, packed, scales, res, k8), ref + res.double())):
+        assert bool(((got.double() - want).abs() <= 2.0 ** -8 * want.abs() + slack + 1e-30).all())
+
+
+@gpu
+def test_w4_projection_keeps_nan_and_inf_in_their_row():
+    from summa_b200 import ops
+    packed, scales, k8, wq = _w4(512, 40, 3)
+    x = torch.randn(4, 512, device="cuda").to(torch.bfloat16)
+    clean = ops.int4_gemv(x, packed, scales, None, k8)
+    x[1, 7], x[2, 300] = float("inf"), float("nan")
+    got = ops.int4_gemv(x, packed, scales, None, k8)
+    assert bool(got[1].isnan().all()) and bool(got[2].isnan().all())
+    assert torch.equal(got[0], clean[0]) and torch.equal(got[3], clean[3])
+
+
+@gpu
+def test_w4_projection_takes_unaligned_operand_views():
+    from summa_b200 import ops
+    packed, scales, k8, wq = _w4(256, 24, 5)
+    s1 = torch.empty(scales.numel() + 1, device="cuda", dtype=scales.dtype)[1:].view_as(scales).copy_(scales)
+    k1 = torch.empty(k8.numel() + 1, device="cuda", dtype=k8.dtype)[1:].view_as(k8).copy_(k8)
+    assert s1.data_ptr() % 8 and k1.data_ptr() % 16
+    x = torch.randn(2, 256, device="cuda").to(torch.bfloat16)
+    assert torch.equal(ops.int4_gemv(x, packed, s1, None, k1), ops.int4_gemv(x, packed, scales, None, k8))
+
+
+@gpu
+@pytest.mark.parametrize("M,K,I", [(1, 128, 4), (3, 9088, 20), (2, 14464, 12)])
+def test_w4_gated_projection_edges(M, K, I):
+    from summa_b200.ops import cuda_ops
+    packed, scales, k8, wq = _w4(K, 2 * I, M + K + I)
+    x = torch.randn(M, K, device="cuda").to(torch.bfloat16)
+    got = cuda_ops.int4_gemv_swiglu(x, k8, scales).double()
+    u = (x.double() @ wq).to(torch.bfloat16).double()
+    ref = torch.nn.functional.silu(u[:, :I]) * u[:, I:]
+    # gate and value are rounded to bf16 first and may fall to the other side of a rounding boundary (2^-8 each)
+    assert bool(((got - ref).abs() <= 2.0 ** -6 * ref.abs() + 2.0 ** -7 * u.abs().amax()).all())
