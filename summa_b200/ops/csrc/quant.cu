@@ -90,21 +90,21 @@ int4_gemv_kernel(const __nv_bfloat16* __restrict__ x, const uint8_t* __restrict_
 // no global accumulator, no atomics. Launched with programmatic stream serialization: barrier set-up,
 // tensor-memory allocation and descriptor prefetch overlap the tail of the preceding kernel.
 //
-// Two instances. Decode (M <= 64): 8 ring stages, x tile of up to 64 rows, 128 tensor-memory columns, two CTAs
+// Two instances. Decode (M <= 64): 8 ring stages, x tile of up to 64 rows, 256 tensor-memory columns, two CTAs
 // per SM, K split over the cluster. Prefill (M > 64): grid.z walks the rows in tiles of MP = 128 or 256, 6 ring
 // stages with a 256-row x tile, 512 tensor-memory columns (128 for four weight buffers + up to 256 for D),
 // one CTA per SM, no K split: the weight tile is expanded once per 128 x MP output tile, in registers, on its
 // way into tensor memory, and never exists in global memory.
 constexpr int WQ_WBYTES = 8 * 128 * 4;           // repacked weight tile
-// decode rows with three groups (SUMMA_W4A16_DECODE_GROUPS=3): 12 % faster on the 28672-wide projection, 20 % slower at
-// 64 rows x 4096 columns, level elsewhere (all 20-60 us launches): one group stays the default
-constexpr int W4A16_DECODE_GROUPS_DEFAULT = 1;
+// Decode rows run three expanding groups too: 64 rows, N 28672 52.8 -> 44.4 us against one group, N 6144 18.8 -> 16.9,
+// K 14336 N 4096 27.2 -> 25.6, N 4096 level (12.6 / 12.7).
+constexpr int W4A16_GROUPS = 3;
 template <int MPMAX, int G> struct WqCfg {
   static constexpr int NS = MPMAX <= 64 ? 8 : 6;                 // ring stages
   static constexpr int XBYTES = MPMAX * 128;                     // x tile at MP = MPMAX
   static constexpr int STAGE = WQ_WBYTES + XBYTES;
   static constexpr int SMEM = NS * STAGE + 256 + 1024;
-  static constexpr int TMEM_COLS = MPMAX <= 64 ? (G == 1 ? 128 : 256) : 512;
+  static constexpr int TMEM_COLS = MPMAX <= 64 ? 256 : 512;
   static constexpr int MIN_CTAS = MPMAX <= 64 ? 2 : 1;
   // dequant warps = 4 * DQ, in DQ groups of 128 threads (thread = output column; every group reaches every
   // tensor-memory lane). With one CTA per SM one group cannot expand a weight tile within the 512 cycles its four
@@ -115,7 +115,7 @@ template <int MPMAX, int G> struct WqCfg {
   // groups in turn: each group has three block times to expand one block.
   static constexpr int DQ = G;
   static constexpr int THREADS = 128 * DQ + 64;
-  static constexpr int NA = G == 1 ? 2 : 4;                 // expanded weight buffers in tensor memory (32 columns each)
+  static constexpr int NA = 4;                              // expanded weight buffers in tensor memory (32 columns each)
   // a group skips blocks, so it does not see every phase of a buffer's `free` barrier; a parity wait stays
   // unambiguous because the ring bounds how far the MMA can lag: block i is only loaded once block i - NS has been
   // consumed, and i - NS >= i - 2 NA
@@ -168,10 +168,9 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
   constexpr uint32_t COL_A = 0, COL_D = 32 * NA;  // A: NA buffers x 32 columns, D: MP columns
   const int m0 = blockIdx.z * p.MP;               // first row of this CTA's row tile (decode: one tile)
   asm volatile("griddepcontrol.wait;" ::: "memory");   // x and the residual come from the preceding kernel
-  float* tile = reinterpret_cast<float*>(smem);   // [128][MP + 1], reuses the ring once the products are done
-  const int tpitch = p.MP + 1;
+  float* tile = reinterpret_cast<float*>(smem);   // [MP][128 n], reuses the ring once the products are done
   // one K split, whole 128-column tile, 16-byte aligned rows of y: the tile is parked as bf16 `[m][128 n]` and
-  // leaves in 16-byte row segments; otherwise as fp32 `[n][m]` for the cluster's reduction and scalar stores
+  // leaves in 16-byte row segments; otherwise as fp32 `[m][128 n]` for the cluster's reduction
   __nv_bfloat16* tileb = reinterpret_cast<__nv_bfloat16*>(smem);
   const bool fast_out = gridDim.y == 1 && (p.N & 7) == 0 && n0 + 128 <= p.N;
 
@@ -261,13 +260,13 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
           for (int j = 0; j < 16; ++j) tileb[(c + j) * 128 + t] = __float2bfloat16(__uint_as_float(v[j]));
         } else {
 #pragma unroll
-          for (int j = 0; j < 16; ++j) tile[t * tpitch + c + j] = __uint_as_float(v[j]);
+          for (int j = 0; j < 16; ++j) tile[(c + j) * 128 + t] = __uint_as_float(v[j]);
         }
       }
     } else if (nkb == 0) {
       for (int c = h; c < p.MP; c += DQ) {
         if (fast_out) tileb[c * 128 + t] = __float2bfloat16(0.f);
-        else tile[t * tpitch + c] = 0.f;
+        else tile[c * 128 + t] = 0.f;
       }
     }
   }
@@ -301,18 +300,34 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
       }
     }
   } else if (threadIdx.x < 128 * DQ) {
-    // every CTA of the cluster reduces its share of the rows (m = rank, rank + S, ...), so the
-    // distributed-shared-memory reads are spread over the cluster instead of serialised in one CTA
-    const int t = threadIdx.x & 127, n = n0 + t, h = threadIdx.x >> 7;
+    // Every CTA of the cluster reduces its share of the rows (m = rank, rank + S, ...): a warp takes a row, a lane four
+    // columns, so a remote read is 512 contiguous bytes and the S ranks' reads are independent. (One column per lane over
+    // an `[n][m]` tile cost 32 remote transactions per read: 64 rows, K = N = 4096: 36.6 -> 12.6 us; K 14336: 52.5 -> 27.2; 256 rows 59.2 -> 18.7.)
     const int S = (int)cluster.num_blocks(), r0 = (int)cluster.block_rank();
     const int rows = min(p.MP, p.M - m0);
-    if (n < p.N) {
-      for (int m = r0 + S * h; m < rows; m += S * DQ) {
-        float v = 0.f;
+    const int n = n0 + 4 * lane;
+    const bool vec_out = ((reinterpret_cast<uintptr_t>(p.residual) | reinterpret_cast<uintptr_t>(p.y)) & 7) == 0;
+    for (int m = r0 + S * warp; m < rows; m += S * 4 * DQ) {
+      float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll 8
-        for (int r = 0; r < S; ++r) v += cluster.map_shared_rank(tile, r)[t * tpitch + m];
-        if (p.residual) v += __bfloat162float(p.residual[(long)(m0 + m) * p.N + n]);
-        p.y[(long)(m0 + m) * p.N + n] = __float2bfloat16(v);
+      for (int r = 0; r < S; ++r) {
+        const float4 u = *reinterpret_cast<const float4*>(cluster.map_shared_rank(tile, r) + m * 128 + 4 * lane);
+        v.x += u.x; v.y += u.y; v.z += u.z; v.w += u.w;
+      }
+      if (n < p.N) {                              // N % 4 == 0
+        const long at = (long)(m0 + m) * p.N + n;
+        if (vec_out) {
+          if (p.residual) {
+            const uint2 rv = *reinterpret_cast<const uint2*>(p.residual + at);
+            v.x += bf16_lo(rv.x); v.y += bf16_hi(rv.x); v.z += bf16_lo(rv.y); v.w += bf16_hi(rv.y);
+          }
+          *reinterpret_cast<uint2*>(p.y + at) = make_uint2(pack_bf16(v.x, v.y), pack_bf16(v.z, v.w));
+        } else {
+          const float o[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+          for (int c = 0; c < 4; ++c)
+            p.y[at + c] = __float2bfloat16(p.residual ? o[c] + __bfloat162float(p.residual[at + c]) : o[c]);
+        }
       }
     }
   }
@@ -607,7 +622,7 @@ static int launch_w4a16(const void* x, const void* packed_k8, const void* scales
   if (MPMAX <= 64) {
     p.MP = M <= 16 ? 16 : (M <= 32 ? 32 : 64);
     // K splits = cluster size (1, 2, 4 or 8): about one round of two-per-SM CTAs, at least 4 k-blocks each
-    // (twice as many splits measured slower: 5,539 against 6,494 decode tokens/s at batch 64)
+    // (twice as many measured slower where it applies: 64 rows, N 28672 52.8 -> 62.4 us, N 6144 18.8 -> 23.4)
     while (splits < 8 && n_tiles * 2 * splits <= 2 * num_sms() && kblocks / (2 * splits) >= 4) splits *= 2;
   } else {
     p.MP = M <= 128 ? 128 : 256;
@@ -664,11 +679,6 @@ extern "C" int sb_w4a16_gemm(const void* x, const void* packed_k8, const void* s
                             (const __nv_bfloat16*)residual, (__nv_bfloat16*)y, M, N, K, ldx, nullptr, 0.f, {}};
     return launch_w4_stream(a, W4S_PLAIN, st);
   }
-  if (M <= 64) {
-    // decode rows: one expanding group per CTA, or three (whole 64-k blocks in turn, like the prefill instance)
-    static const int groups = [] { const char* e = getenv("SUMMA_W4A16_DECODE_GROUPS"); return e ? atoi(e) : W4A16_DECODE_GROUPS_DEFAULT; }();
-    if (groups == 3) return launch_w4a16<64, 3>(x, packed_k8, scales, residual, y, M, N, K, ldx, st);
-    return launch_w4a16<64, 1>(x, packed_k8, scales, residual, y, M, N, K, ldx, st);
-  }
-  return launch_w4a16<256, 3>(x, packed_k8, scales, residual, y, M, N, K, ldx, st);
+  if (M <= 64) return launch_w4a16<64, W4A16_GROUPS>(x, packed_k8, scales, residual, y, M, N, K, ldx, st);
+  return launch_w4a16<256, W4A16_GROUPS>(x, packed_k8, scales, residual, y, M, N, K, ldx, st);
 }

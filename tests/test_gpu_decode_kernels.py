@@ -69,3 +69,22 @@ def test_w4_gated_projection_edges(M, K, I):
     ref = torch.nn.functional.silu(u[:, :I]) * u[:, I:]
     # gate and value are rounded to bf16 first and may fall to the other side of a rounding boundary (2^-8 each)
     assert bool(((got - ref).abs() <= 2.0 ** -6 * ref.abs() + 2.0 ** -7 * u.abs().amax()).all())
+
+
+@gpu
+@pytest.mark.parametrize("M,K,N", [(9, 512, 132), (33, 4096, 260), (64, 14336, 128), (64, 1024, 2052), (128, 4096, 384), (257, 2048, 516)])
+def test_w4a16_split_k_reduction(M, K, N):
+    """K split over a cluster with ragged rows and columns; the residual also as a view that is not 8-byte aligned. The kernel
+    rounds the weights to bf16 (2^-9 of each term), sums in fp32 and rounds once."""
+    from summa_b200.ops import cuda_ops, native
+    packed, scales, k8, wq = _w4(K, N, M + K + N)
+    x = torch.randn(M, K, device="cuda").to(torch.bfloat16)
+    res = torch.randn(M * N + 1, device="cuda").to(torch.bfloat16)
+    slack = 2.0 ** -9 * (x.double().abs() @ wq.abs())
+    for r in (res[:-1].view(M, N), res[1:].view(M, N)):
+        y = torch.empty(M, N, device="cuda", dtype=torch.bfloat16)
+        native.call("sb_w4a16_gemm", x.data_ptr(), k8.data_ptr(), scales.data_ptr(), None, r.data_ptr(), y.data_ptr(), M, N, K, K,
+                    native.stream())
+        want = x.double() @ wq + r.double()
+        assert bool(((y.double() - want).abs() <= 2.0 ** -7 * (want.abs() + r.double().abs()) + slack).all())
+    assert native.read_error_flag() == 0
