@@ -10,7 +10,7 @@
 //     operands 16 (q - 8) of 8 k, against seven instructions for bf16 pairs, and ONE mma.m16n8k32 (s8, s32 accumulation,
 //     exact) takes 16 columns x 32 k of weights against 8 columns of digits. The products of a group are whole numbers;
 //     only the combination over groups rounds (fp32).
-//   * one CTA per SM walks a contiguous run of 16-column tiles over the whole K range; its 16 warps take the scale groups
+//   * one CTA per SM walks 16-column tiles over the whole K range; its 16 warps take the scale groups
 //     round robin, each through a ring of its own in shared memory that asynchronous copies fill D groups (D KB) ahead,
 //     across tiles; no barrier, no producer. (A ring in registers is held up by whatever touches a loaded register
 //     early: a scale that was combined on arrival cost 27 us instead of 21.6, spilled ring registers 28 us, N 28672.)
@@ -19,8 +19,8 @@
 //     immediate epilogue per tile its latency was paid per tile. No cluster, no atomics.
 //   * the weights depend on nothing, so the first groups are requested before `griddepcontrol.wait`.
 // Measured against the CUDA-core cluster kernel it replaces (weights from HBM, graph of launches, one row): K 4096 N 6144
-// 12.0 -> 7.5 us, N 4096 7.4 -> 6.1, N 28672 28.9 -> 21.1 (gated with norm 33.2 -> 23.5), N 32000 30.2 -> 22.6, K 14336
-// N 4096 19.9 -> 13.0; four rows: 20.0 -> 10.4, 14.6 -> 8.6, 60.7 -> 27.2, 66.0 -> 28.7, 41.6 -> 23.5. Relative error
+// 12.0 -> 7.3 us, N 4096 7.4 -> 5.8, N 28672 29.0 -> 20.2 (gated with norm 32.9 -> 22.2), N 32000 30.1 -> 22.4, K 14336
+// N 4096 20.0 -> 12.5; four rows: 20.0 -> 9.5, 14.6 -> 8.0, 60.4 -> 25.7, 66.7 -> 27.6, 41.6 -> 22.8. Relative error
 // against 64 bits: the same 0.00165 (the rounding of y to bf16).
 #include "host_util.h"
 #include "sm100.cuh"
@@ -89,8 +89,10 @@ w4_stream_kernel(const W4StreamArgs p, const int tile_base, const int tiles, con
   float* psum = reinterpret_cast<float*>(w4s_smem + L.psum);
   float* rstd = reinterpret_cast<float*>(w4s_smem + L.gsq);
   float* gsq = rstd + M;
-  const int t_lo = tile_base + (int)((long)blockIdx.x * tiles / gridDim.x);
-  const int t_hi = tile_base + (int)((long)(blockIdx.x + 1) * tiles / gridDim.x);
+  // Tiles are dealt out in turn, so that the CTAs read neighbouring pieces of the same weight rows at the same time (DRAM
+  // pages): N 28672 20.2 us, 21.1 with contiguous runs.
+  const int t_lo = tile_base + blockIdx.x, t_hi = tile_base + tiles, t_step = gridDim.x;
+  const int ntiles = (tiles - (int)blockIdx.x + t_step - 1) / t_step;
   const int I = N >> 1;                       // gated: columns of the gate half
   const int passes = (groups + pass_groups - 1) / pass_groups;
   constexpr int TILE_COLS = MODE == W4S_GATED ? 8 : W4S_TILE;       // columns (gated: gate columns) of a tile
@@ -103,12 +105,12 @@ w4_stream_kernel(const W4StreamArgs p, const int tile_base, const int tiles, con
   }
   __syncthreads();
 
-  // Epilogue of this CTA's q-th tile (counted over the passes): 32 outputs o = m * 16 + c at a time; chunk k of tile ct
-  // belongs to warp (ct + k) % 16, which runs it two tiles later, when the other warps have long handed theirs over.
-  const int chunks = (W4S_TILE * M + 31) / 32, ntiles = t_hi - t_lo;
+  // Epilogue of this CTA's q-th tile (counted over the passes): 32 outputs o = m * 16 + c at a time; chunk k of the i-th
+  // tile belongs to warp (i + k) % 16, which runs it two tiles later, when the other warps have long handed theirs over.
+  const int chunks = (W4S_TILE * M + 31) / 32;
   auto epilogue = [&](int q) {
-    const int pass = q / ntiles, ct = t_lo + q - pass * ntiles;
-    const int chunk = (warp - ct) & (W4S_WARPS - 1);
+    const int pass = q / ntiles, local = q - pass * ntiles, ct = t_lo + local * t_step;
+    const int chunk = (warp - local) & (W4S_WARPS - 1);
     if (chunk >= chunks) return;
     const bool last = pass + 1 == passes;
     const float* rb = red + (q & (W4S_NB - 1)) * W4S_WARPS * ROWS * W4S_TILE;
@@ -131,7 +133,7 @@ w4_stream_kernel(const W4StreamArgs p, const int tile_base, const int tiles, con
       }
     }
     if (passes > 1) {
-      float* ps = psum + ((ct - t_lo) * M + mm) * W4S_TILE + c;
+      float* ps = psum + (local * M + mm) * W4S_TILE + c;
       if (pass > 0 && row) v += *ps;
       if (!last && row) *ps = v;
     }
@@ -204,7 +206,7 @@ w4_stream_kernel(const W4StreamArgs p, const int tile_base, const int tiles, con
     ls += (long)W4S_WARPS * N;
     if (++li == lgpw) {
       li = 0;
-      ++lt;
+      lt += t_step;
       rewind(g0);
     }
   };
@@ -213,7 +215,7 @@ w4_stream_kernel(const W4StreamArgs p, const int tile_base, const int tiles, con
     const int g0 = pass * pass_groups, g1 = min(groups, g0 + pass_groups), ng = g1 - g0;
     const int gpw = (ng + W4S_WARPS - 1) / W4S_WARPS;
     const int mine = (ng - warp + W4S_WARPS - 1) / W4S_WARPS;
-    const int total = (t_hi - t_lo) * gpw;
+    const int total = ntiles * gpw;
     lt = t_lo; li = 0; lmine = mine; lgpw = gpw;
     rewind(g0);
     lslot = 0;
