@@ -202,19 +202,28 @@ class _GraphDecoder:
 
     @staticmethod
     def _norm_proj(norm, proj, h):
-        """proj(norm(h)); an RMSNorm in front of a quantised projection runs inside its GEMV kernel."""
+        """proj(norm(h)); an RMSNorm in front of a projection runs inside its GEMV kernel."""
+        from .layers import Linear
         from .quantized import QuantLinear
-        if isinstance(proj, QuantLinear) and getattr(norm, "kind", None) == "rmsnorm" and h.shape[0] <= 4:
-            return proj(h, norm=(norm.gamma, norm.eps))
+        if getattr(norm, "kind", None) == "rmsnorm":
+            if isinstance(proj, QuantLinear) and h.shape[0] <= 4:
+                return proj(h, norm=(norm.gamma, norm.eps))
+            if type(proj) is Linear and h.is_cuda:
+                from ..ops import cuda_ops
+                return cuda_ops.decode_linear(h, proj.weight, proj.bias, norm=(norm.gamma, norm.eps))
         return proj(norm(h))
 
     @staticmethod
     def _proj_add(proj, x, h):
         """h + proj(x), with the add fused into the projection's epilogue when it can be."""
+        from .layers import Linear
         from .quantized import QuantLinear
         from ..parallel.tp import RowParallelLinear
         if isinstance(proj, (QuantLinear, RowParallelLinear)):
             return proj(x, residual=h)
+        if type(proj) is Linear and x.is_cuda:
+            from ..ops import cuda_ops
+            return cuda_ops.decode_linear(x, proj.weight, proj.bias, residual=h)
         return h + proj(x)
 
     def run(self, first: torch.Tensor, steps: int) -> torch.Tensor:

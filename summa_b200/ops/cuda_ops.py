@@ -143,6 +143,36 @@ def linear(x, weight, bias=None):
     return _Linear.apply(x, weight, bias)
 
 
+N.register("sb_decode_linear", [N.P] * 3 + [N.I] + [N.P] * 2 + [N.I] * 3 + [N.L, N.L, N.P, N.F, N.I, N.P])
+N.register("sb_decode_linear_one_pass", [N.I, N.I])
+
+
+def decode_linear(x, weight, bias=None, residual=None, norm=None):
+    """(rmsnorm(x) or x) @ W (+ bias) (+ residual) for a decode step's x `[M, K]`, no gradients. Up to 8 rows and a
+    row-major bf16 weight run as one weight-streaming launch that may start reading W before the kernel in front of it
+    has finished, so W must not be written by work still in flight (a served model's weights are not); everything else
+    takes the separate ops."""
+    M, K = x.shape
+    fits = (M <= 8 and weight.dtype == BF16 and x.dtype == BF16 and weight.stride(1) == 1 and weight.stride(0) % 8 == 0
+            and K % 8 == 0 and x.stride(1) == 1 and x.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0 and weight.data_ptr() % 16 == 0
+            and (bias is None or bias.dtype in (BF16, torch.float32)))
+    if norm is not None:
+        g = norm[0]
+        if not (fits and g.dtype == torch.float32 and g.is_contiguous() and g.data_ptr() % 16 == 0
+                and N.call_value("sb_decode_linear_one_pass", M, K)):
+            x, norm = rmsnorm(x, norm[0], norm[1]), None
+    if not fits:
+        y = linear(x, weight, bias)
+        return y if residual is None else residual + y
+    Nn = weight.shape[1]
+    y = torch.empty(M, Nn, device=x.device, dtype=BF16)
+    res = residual.contiguous() if residual is not None else None
+    N.call("sb_decode_linear", x.data_ptr(), weight.data_ptr(), N.ptr(bias), 1 if (bias is not None and bias.dtype == BF16) else 0,
+           N.ptr(res), y.data_ptr(), M, Nn, K, x.stride(0), weight.stride(0), norm[0].data_ptr() if norm is not None else None,
+           float(norm[1]) if norm is not None else 0.0, 1, N.stream())
+    return y
+
+
 # ------------------------------------------------------------------ RMSNorm
 
 def _gamma32(g: torch.Tensor) -> torch.Tensor:

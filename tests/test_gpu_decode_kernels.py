@@ -88,3 +88,54 @@ def test_w4a16_split_k_reduction(M, K, N):
         want = x.double() @ wq + r.double()
         assert bool(((y.double() - want).abs() <= 2.0 ** -7 * (want.abs() + r.double().abs()) + slack).all())
     assert native.read_error_flag() == 0
+
+
+@gpu
+@pytest.mark.parametrize("M,K,N", [
+    (1, 8, 2), (2, 96, 3072), (3, 1000, 353), (8, 4104, 2366), (5, 1032, 2369),     # K and N tails; the last N of 16-column tiles
+    (8, 14344, 48), (6, 14336, 4100), (1, 40968, 24)])                              # K in passes, both tile widths
+def test_bf16_projection_against_fp64(M, K, N):
+    """`ops.linear` with up to 8 rows and the decode form (bias, residual, fused norm) on a weight with padded rows. fp32 sums
+    (2^-18 of the terms' sum), one rounding to bf16, one more before a residual."""
+    from summa_b200 import ops
+    from summa_b200.ops import cuda_ops, native
+    torch.manual_seed(M + K + N)
+    w = (torch.randn(K, (N + 15) // 8 * 8, device="cuda") * 0.05).to(torch.bfloat16)[:, :N]
+    x = torch.randn(M, K, device="cuda").to(torch.bfloat16)
+    bias, res = torch.randn(N, device="cuda"), torch.randn(M, N, device="cuda").to(torch.bfloat16)
+    gamma = 1 + 0.1 * torch.randn(K, device="cuda")
+    xn = ops.rmsnorm(x, gamma, 1e-5)
+
+    def check(got, inp, b, r):
+        proj = inp.double() @ w.double() + (0 if b is None else b.double())
+        want = proj if r is None else proj + r.double()
+        tol = 2.0 ** -8 * (want.abs() + (0 if r is None else proj.abs())) + 2.0 ** -18 * (inp.double().abs() @ w.double().abs())
+        assert bool(((got.double() - want).abs() <= tol + 1e-30).all())
+    if N % 8 == 0:                                        # the general entry's own shape rule
+        check(ops.linear(x, w, None), x, None, None)
+        check(ops.linear(x, w, bias), x, bias, None)
+    check(cuda_ops.decode_linear(x, w, bias.to(torch.bfloat16), res), x, bias.to(torch.bfloat16), res)
+    got = cuda_ops.decode_linear(x, w, None, res, norm=(gamma, 1e-5))
+    # the fused norm may round single elements of the normed row the other way (2^-8 of one term each)
+    proj = xn.double() @ w.double()
+    tol = 2.0 ** -7 * (proj.abs() + res.double().abs()) + 2.0 ** -8 * (xn.double().pow(2) @ w.double().pow(2)).sqrt() + 2.0 ** -18 * (xn.double().abs() @ w.double().abs())
+    assert bool(((got.double() - proj - res.double()).abs() <= tol + 1e-30).all())
+    assert native.read_error_flag() == 0
+
+
+@gpu
+@pytest.mark.parametrize("rows,H", [(1, 2048), (64, 4096), (7, 8192), (3, 2056), (1184, 2048), (1185, 2048), (5, 8200)])
+def test_rmsnorm_row_per_cta(rows, H):
+    from summa_b200 import ops
+    torch.manual_seed(rows + H)
+    x, r = torch.randn(rows, H, device="cuda").to(torch.bfloat16), torch.randn(rows, H, device="cuda").to(torch.bfloat16)
+    gamma = 1 + 0.1 * torch.randn(H, device="cuda")
+    for res in (None, r):
+        s = x if res is None else (x.float() + res.float()).to(torch.bfloat16)
+        ref = s.double() * torch.rsqrt(s.double().pow(2).mean(-1, keepdim=True) + 1e-5) * gamma.double()
+        y = ops.rmsnorm(x, gamma, 1e-5) if res is None else ops.add_rmsnorm(x, res, gamma, 1e-5)
+        if res is not None:
+            assert torch.equal(y[1], s)
+            y = y[0]
+        # one rounding to bf16 next to fp32 statistics
+        assert bool(((y.double() - ref).abs() <= (2.0 ** -8 + 2.0 ** -18) * ref.abs() + 1e-30).all())
