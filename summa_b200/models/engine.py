@@ -65,13 +65,16 @@ class InferenceEngine:
         return cls(model, tp)
 
     def reset(self, batch: int, capacity: int):
-        """Start a new set of sequences. A state of the same shape is recycled (the caches are
-        overwritten as the new sequences grow), which also keeps the captured decode graph."""
+        """Start a new set of sequences. A state of the same shape is recycled (the KV caches are
+        overwritten as the new sequences grow, recurrent states start anew), which also keeps the captured decode graph."""
         st = self.state
-        if st is not None and st.capacity == capacity and st.layers and hasattr(st.layers[0], "k") \
-                and st.layers[0].k.shape[0] == batch and all(hasattr(l, "length") for l in st.layers):
-            for l in st.layers:
-                l.length = 0
+        if st is not None and st.capacity == capacity and st.layers \
+                and all((l.k if hasattr(l, "length") else l.conv).shape[0] == batch for l in st.layers):
+            for i, l in enumerate(st.layers):
+                if hasattr(l, "length"):
+                    l.length = 0
+                else:
+                    st.layers[i] = self.model.layers[i].ssm.make_state(batch, l.h.device, l.conv.dtype)
             st.pos = 0
             return
         self.state = self.model.make_state(batch, capacity)
@@ -116,12 +119,17 @@ class _GraphDecoder:
     @classmethod
     def try_build(cls, model, state, max_steps: int):
         from .layers import FeedForward, MultiHeadAttention
+        from ..ops import cuda_ops
         cfgm = model.cfg
         for blk in model.layers:
+            if not blk.pre_norm or not blk.residual or blk.memory is not None or not isinstance(blk.feed_forward, FeedForward):
+                return None
             a = blk.attention
-            if (not isinstance(a, MultiHeadAttention) or not blk.pre_norm or not blk.residual or blk.memory is not None
-                    or not isinstance(blk.feed_forward, FeedForward) or a.head_dim != 128 or a.window is not None
-                    or a.q_norm is not None or not a.use_rope or not a.causal or a.num_heads // a.num_kv_heads > 8):
+            if blk.ssm is not None:
+                if not cuda_ops.mamba_decode_usable(blk.ssm):
+                    return None
+            elif (not isinstance(a, MultiHeadAttention) or a.head_dim != 128 or a.window is not None or a.q_norm is not None
+                    or not a.use_rope or not a.causal or a.num_heads // a.num_kv_heads > 8):
                 return None
         if cfgm.embeddings.scale is not None or model.stream_dtype != torch.bfloat16:
             return None
@@ -130,51 +138,44 @@ class _GraphDecoder:
     def __init__(self, model, state, max_steps: int):
         from ..ops import native
         self.model, self.state, self.max_steps = model, state, max_steps
+        self.attn = [i for i, blk in enumerate(model.layers) if blk.ssm is None]
+        self.ssm = [i for i, blk in enumerate(model.layers) if blk.ssm is not None]
+        dev = model.embedding.weight.device
         st0 = state.layers[0]
-        self.B, self.cap = st0.k.shape[0], st0.k.shape[1]
-        dev = st0.k.device
+        self.B = (st0.conv if self.ssm and self.ssm[0] == 0 else st0.k).shape[0]
+        self.cap = state.layers[self.attn[0]].k.shape[1] if self.attn else state.capacity
+        # The captured step updates recurrent states of its own: a prefill leaves its results in fresh tensors, which `run`
+        # copies in, and callers get copies back.
+        self.rec = {i: (torch.empty_like(state.layers[i].conv, dtype=torch.bfloat16), torch.empty_like(state.layers[i].h))
+                    for i in self.ssm}
         self.tok = torch.zeros(self.B, 1, dtype=torch.long, device=dev)
         self.pos = torch.zeros(1, dtype=torch.int32, device=dev)
         self.col = torch.zeros(1, 1, dtype=torch.long, device=dev)
         self.out = torch.zeros(self.B, max_steps, dtype=torch.long, device=dev)
-        a0 = model.layers[0].attention
-        self.splits = native.call_value("sb_attention_decode_splits", self.B, a0.num_kv_heads, self.cap)
-        need = native.call_value("sb_attention_decode_workspace", self.B, a0.num_kv_heads, self.splits)
-        self.ws = torch.empty(need, dtype=torch.float32, device=dev)
+        if self.attn:                            # (the largest of the blocks: their head counts may differ)
+            heads = {model.layers[i].attention.num_kv_heads for i in self.attn}
+            self.splits = {k: native.call_value("sb_attention_decode_splits", self.B, k, self.cap) for k in heads}
+            need = max(native.call_value("sb_attention_decode_workspace", self.B, k, n) for k, n in self.splits.items())
+            self.ws = torch.empty(need, dtype=torch.float32, device=dev)
         P, I, L, F = native.P, native.I, native.L, native.F
         native.register("sb_decode_rope_append", [P] * 6 + [I, I, I, I, L, P, I, P])
         native.register("sb_attention_decode_dyn", [P] * 5 + [I, I, I, P, I, I, I] + [P] * 4 + [F, I, P])
         self.graph = None
 
     def _step(self):
-        import ctypes
-        from ..ops import native
+        from .quantized import QuantLinear, in_proj_swiglu
         m, B = self.model, self.B
         h = torch.nn.functional.embedding(self.tok.view(-1), m.embedding.weight).to(torch.bfloat16)
-        cos, sin = m.rope(h.device)
-        for blk, st in zip(m.layers, self.state.layers):
-            a = blk.attention
-            cs = (ctypes.c_long * 3)(st.k.stride(0), st.k.stride(1), st.k.stride(2))
-            if self._rope_fusable(blk, h):
+        cos, sin = m.rope(h.device) or (None, None)
+        for i, (blk, st) in enumerate(zip(m.layers, self.state.layers)):
+            if blk.ssm is not None:
                 from ..ops import cuda_ops
-                qkv = cuda_ops.int4_gemv_rope_append(h, a.qkv_proj.packed_k8(), a.qkv_proj.scales,
-                                                     (blk.attn_norm.gamma, blk.attn_norm.eps), cos, sin, st.k, st.v,
-                                                     self.pos, a.num_heads, a.num_kv_heads, a.head_dim, self.cap)
+                xz = self._norm_proj(blk.attn_norm, blk.ssm.in_proj, h)
+                h = self._proj_add(blk.ssm.out_proj, cuda_ops.mamba_decode_step(blk.ssm, xz, *self.rec[i]), h)
             else:
-                qkv = self._norm_proj(blk.attn_norm, a.qkv_proj, h)
-                native.call("sb_decode_rope_append", qkv.data_ptr(), cos.data_ptr(), sin.data_ptr(), st.k.data_ptr(),
-                            st.v.data_ptr(), self.pos.data_ptr(), B, a.num_heads, a.num_kv_heads, a.head_dim,
-                            qkv.stride(0), cs, self.cap, native.stream())
-            o = torch.empty(B, a.q_dim, dtype=torch.bfloat16, device=h.device)
-            qs = (ctypes.c_long * 2)(qkv.stride(0), a.head_dim)
-            os_ = (ctypes.c_long * 2)(o.stride(0), a.head_dim)
-            native.call("sb_attention_decode_dyn", qkv.data_ptr(), st.k.data_ptr(), st.v.data_ptr(), o.data_ptr(),
-                        self.ws.data_ptr(), B, a.num_heads, a.num_kv_heads, self.pos.data_ptr(), 1, self.cap, a.head_dim,
-                        qs, cs, cs, os_, 1.0 / a.head_dim ** 0.5, self.splits, native.stream())
-            h = self._proj_add(a.o_proj, o, h)
+                h = self._attend(blk, st, h, cos, sin)
             ff = blk.feed_forward
-            if _FUSED_EPILOGUES and ff.gated and ff.act in ("swiglu", "silu") and getattr(blk.ffn_norm, "kind", None) == "rmsnorm" and h.shape[0] <= 4:
-                from .quantized import in_proj_swiglu
+            if _FUSED_EPILOGUES and ff.gated and ff.act in ("swiglu", "silu") and getattr(blk.ffn_norm, "kind", None) == "rmsnorm" and h.shape[0] <= 4 and isinstance(ff.in_proj, QuantLinear):
                 u = in_proj_swiglu(ff.in_proj, h, norm=(blk.ffn_norm.gamma, blk.ffn_norm.eps))
             else:
                 u = self._norm_proj(blk.ffn_norm, ff.in_proj, h)
@@ -186,6 +187,30 @@ class _GraphDecoder:
         self.tok.copy_(nxt)
         self.pos += 1
         self.col += 1
+
+    def _attend(self, blk, st, h, cos, sin):
+        """The attention branch of a block with its residual: qkv projection, RoPE, cache append, split-KV attention, o_proj."""
+        import ctypes
+        from ..ops import native
+        B, a = self.B, blk.attention
+        cs = (ctypes.c_long * 3)(st.k.stride(0), st.k.stride(1), st.k.stride(2))
+        if self._rope_fusable(blk, h):
+            from ..ops import cuda_ops
+            qkv = cuda_ops.int4_gemv_rope_append(h, a.qkv_proj.packed_k8(), a.qkv_proj.scales,
+                                                 (blk.attn_norm.gamma, blk.attn_norm.eps), cos, sin, st.k, st.v,
+                                                 self.pos, a.num_heads, a.num_kv_heads, a.head_dim, self.cap)
+        else:
+            qkv = self._norm_proj(blk.attn_norm, a.qkv_proj, h)
+            native.call("sb_decode_rope_append", qkv.data_ptr(), cos.data_ptr(), sin.data_ptr(), st.k.data_ptr(),
+                        st.v.data_ptr(), self.pos.data_ptr(), B, a.num_heads, a.num_kv_heads, a.head_dim,
+                        qkv.stride(0), cs, self.cap, native.stream())
+        o = torch.empty(B, a.q_dim, dtype=torch.bfloat16, device=h.device)
+        qs = (ctypes.c_long * 2)(qkv.stride(0), a.head_dim)
+        os_ = (ctypes.c_long * 2)(o.stride(0), a.head_dim)
+        native.call("sb_attention_decode_dyn", qkv.data_ptr(), st.k.data_ptr(), st.v.data_ptr(), o.data_ptr(),
+                    self.ws.data_ptr(), B, a.num_heads, a.num_kv_heads, self.pos.data_ptr(), 1, self.cap, a.head_dim,
+                    qs, cs, cs, os_, 1.0 / a.head_dim ** 0.5, self.splits[a.num_kv_heads], native.stream())
+        return self._proj_add(a.o_proj, o, h)
 
     @staticmethod
     def _rope_fusable(blk, h) -> bool:
@@ -227,9 +252,12 @@ class _GraphDecoder:
         return h + proj(x)
 
     def run(self, first: torch.Tensor, steps: int) -> torch.Tensor:
-        start = self.state.layers[0].length
-        if start + steps > self.cap:
+        start = self.state.layers[self.attn[0]].length if self.attn else self.state.pos
+        if self.attn and start + steps > self.cap:
             raise RuntimeError(f"KV cache overflow: {start + steps} > capacity {self.cap}")
+        for i, (conv, hid) in self.rec.items():
+            conv.copy_(self.state.layers[i].conv)
+            hid.copy_(self.state.layers[i].h)
         self.tok.copy_(first)
         self.pos.fill_(start)
         self.col.zero_()
@@ -245,7 +273,10 @@ class _GraphDecoder:
                 self.graph = g
         for _ in range(steps - done):
             self.graph.replay()
-        for st in self.state.layers:
-            st.length = start + steps
+        for i in self.attn:
+            self.state.layers[i].length = start + steps
+        for i, (conv, hid) in self.rec.items():
+            self.state.layers[i].conv = conv.to(self.state.layers[i].conv.dtype, copy=True)
+            self.state.layers[i].h = hid.clone()
         self.state.pos += steps
         return self.out[:, :steps].clone()

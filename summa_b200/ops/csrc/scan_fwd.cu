@@ -263,6 +263,122 @@ extern "C" int sb_conv1d_fwd(const void* x, const float* w, const float* bias, c
   return SB_OK;
 }
 
+// ---------------------------------------------------------------------------- single-token decode step
+// One token per sequence. The two kernels between the projections of a Mamba block: what bounds them is the launch (B 1,
+// C 3072, N 128: 3 MB of recurrent state, half a microsecond of HBM time), so everything between two projections is one
+// launch and the states are updated in place (a captured step replays on fixed addresses).
+namespace sb {
+
+// xc = silu(conv(state ++ x) + bias); state shifts by one. Thread = channel.
+template <int K, typename W>
+__global__ void __launch_bounds__(128)
+mamba_conv_step_kernel(const __nv_bfloat16* __restrict__ x, long ldx, __nv_bfloat16* __restrict__ state,
+                       const W* __restrict__ w, const float* __restrict__ bias, __nv_bfloat16* __restrict__ xc, int C) {
+  const int c = blockIdx.x * 128 + threadIdx.x, b = blockIdx.y;
+  if (c >= C) return;
+  __nv_bfloat16* st = state + ((long)b * C + c) * (K - 1);
+  __nv_bfloat16 win[K];
+#pragma unroll
+  for (int k = 0; k < K - 1; ++k) win[k] = st[k];
+  win[K - 1] = x[b * ldx + c];
+  float a = bias ? bias[c] : 0.f;
+#pragma unroll
+  for (int k = 0; k < K; ++k) a = fmaf(static_cast<float>(w[(long)c * K + k]), __bfloat162float(win[k]), a);
+#pragma unroll
+  for (int k = 0; k < K - 1; ++k) st[k] = win[k + 1];
+  xc[(long)b * C + c] = __float2bfloat16(silu_f(a));
+}
+
+// h = exp(dt A) h + dt u B, y = <h, C> + D u, out = y silu(z), with dt = softplus(delta) and A = -exp(a_log). A lane owns
+// SPL states (4, or 8 for N = 256, or 2 for N = 8) of one channel; N / SPL lanes share a channel.
+template <int N, int SPL>
+__global__ void __launch_bounds__(256)
+mamba_scan_step_kernel(const __nv_bfloat16* __restrict__ u, const __nv_bfloat16* __restrict__ delta,
+                       const float* __restrict__ a_log, const __nv_bfloat16* __restrict__ Bm,
+                       const __nv_bfloat16* __restrict__ Cm, long ld_bc, const float* __restrict__ D,
+                       const __nv_bfloat16* __restrict__ z, long ldz, float* __restrict__ h, __nv_bfloat16* __restrict__ out,
+                       int C) {
+  constexpr int LPC = N / SPL;
+  const int c = (blockIdx.x * 256 + threadIdx.x) / LPC, b = blockIdx.y;
+  const int n0 = (threadIdx.x % LPC) * SPL;
+  const bool live = c < C;
+  float acc = 0.f, uv = 0.f;
+  if (live) {
+    const long at = (long)b * C + c;
+    uv = __bfloat162float(u[at]);
+    const float dt = softplusf_(__bfloat162float(delta[at])), du = dt * uv;
+    float* hp = h + at * N + n0;
+    float hv[SPL], al[SPL];
+#pragma unroll
+    for (int i = 0; i < SPL; i += 2) {
+      const float2 t = *reinterpret_cast<const float2*>(hp + i), a = *reinterpret_cast<const float2*>(a_log + (long)c * N + n0 + i);
+      hv[i] = t.x; hv[i + 1] = t.y;
+      al[i] = a.x; al[i + 1] = a.y;
+    }
+#pragma unroll
+    for (int i = 0; i < SPL; ++i) {
+      const float bv = __bfloat162float(Bm[b * ld_bc + n0 + i]), cv = __bfloat162float(Cm[b * ld_bc + n0 + i]);
+      hv[i] = fmaf(__expf(-dt * __expf(al[i])), hv[i], du * bv);
+      acc = fmaf(hv[i], cv, acc);
+    }
+#pragma unroll
+    for (int i = 0; i < SPL; i += 2) *reinterpret_cast<float2*>(hp + i) = make_float2(hv[i], hv[i + 1]);
+  }
+#pragma unroll
+  for (int o = LPC / 2; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+  if (live && n0 == 0) {
+    // the scan's output is bf16 before the gate, as on the general path
+    const float y = __bfloat162float(__float2bfloat16(fmaf(D[c], uv, acc)));
+    const float zv = __bfloat162float(z[b * ldz + c]);
+    out[(long)b * C + c] = __float2bfloat16(y * silu_f(zv));
+  }
+}
+
+}  // namespace sb
+
+// x `[B, C]` (row stride ldx), state `[B, C, K-1]` bf16 (updated), w `[C, K]` fp32 or bf16, bias `[C]` fp32 or null, xc
+// `[B, C]`. K in 2..4.
+extern "C" int sb_mamba_conv_step(const void* x, long ldx, void* state, const void* w, int w_is_bf16, const float* bias, void* xc,
+                                  int B, int C, int K, cudaStream_t st) {
+  using namespace sb;
+  SB_CHECK_ARG(B > 0 && B <= 65535 && C > 0 && K >= 2 && K <= 4);
+  const dim3 grid((C + 127) / 128, B);
+#define SB_CONV_STEP(KK)                                                                                                       \
+  if (w_is_bf16) mamba_conv_step_kernel<KK, __nv_bfloat16><<<grid, 128, 0, st>>>((const __nv_bfloat16*)x, ldx, (__nv_bfloat16*)state, \
+                                                                                 (const __nv_bfloat16*)w, bias, (__nv_bfloat16*)xc, C); \
+  else mamba_conv_step_kernel<KK, float><<<grid, 128, 0, st>>>((const __nv_bfloat16*)x, ldx, (__nv_bfloat16*)state, (const float*)w,   \
+                                                               bias, (__nv_bfloat16*)xc, C)
+  if (K == 4) { SB_CONV_STEP(4); } else if (K == 3) { SB_CONV_STEP(3); } else { SB_CONV_STEP(2); }
+#undef SB_CONV_STEP
+  SB_CHECK_CUDA(cudaGetLastError());
+  return SB_OK;
+}
+
+// u / delta / out `[B, C]` contiguous, Bm / Cm `[B, N]` with row stride ld_bc, z `[B, C]` with row stride ldz, a_log `[C, N]`,
+// h `[B, C, N]` fp32 (updated), both 8-byte aligned. N in {8, 16, 32, 64, 128, 256}.
+extern "C" int sb_mamba_scan_step(const void* u, const void* delta, const float* a_log, const void* Bm, const void* Cm, long ld_bc,
+                                  const float* D, const void* z, long ldz, float* h, void* out, int B, int C, int N,
+                                  cudaStream_t st) {
+  using namespace sb;
+  SB_CHECK_ARG(B > 0 && B <= 65535 && C > 0);
+#define SB_SCAN_STEP(NN, SPL)                                                                                                  \
+  mamba_scan_step_kernel<NN, SPL><<<dim3((int)(((long)C * (NN / SPL) + 255) / 256), B), 256, 0, st>>>(                          \
+      (const __nv_bfloat16*)u, (const __nv_bfloat16*)delta, a_log, (const __nv_bfloat16*)Bm, (const __nv_bfloat16*)Cm, ld_bc, D, \
+      (const __nv_bfloat16*)z, ldz, h, (__nv_bfloat16*)out, C)
+  switch (N) {
+    case 8: SB_SCAN_STEP(8, 2); break;
+    case 16: SB_SCAN_STEP(16, 4); break;
+    case 32: SB_SCAN_STEP(32, 4); break;
+    case 64: SB_SCAN_STEP(64, 4); break;
+    case 128: SB_SCAN_STEP(128, 4); break;
+    case 256: SB_SCAN_STEP(256, 8); break;
+    default: return SB_ERR_ARG;
+  }
+#undef SB_SCAN_STEP
+  SB_CHECK_CUDA(cudaGetLastError());
+  return SB_OK;
+}
+
 // Steps between the state checkpoints that sb_scan_fwd writes and sb_scan_bwd reads.
 extern "C" int sb_scan_ckpt_interval() { return SCAN_SEG; }
 

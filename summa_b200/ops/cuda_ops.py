@@ -790,6 +790,38 @@ def selective_scan(u, delta, A, Bm, Cm, D, h0=None, need_final_state=False):
     return y, h
 
 
+N.register("sb_mamba_conv_step", [N.P, N.L, N.P, N.P, N.I, N.P, N.P] + [N.I] * 3 + [N.P])
+N.register("sb_mamba_scan_step", [N.P] * 5 + [N.L, N.P, N.P, N.L, N.P, N.P] + [N.I] * 3 + [N.P])
+
+
+def mamba_decode_usable(mixer) -> bool:
+    """Whether `mamba_decode_step` takes this mixer: bf16 projections, fp32 scan parameters, supported state and taps."""
+    w = mixer.conv1d.weight
+    small = (mixer.a_log, mixer.d, mixer.conv1d.bias)
+    return (mixer.d_state in _SCAN_STATES and 2 <= mixer.d_conv <= 4 and w.is_cuda and w.is_contiguous()
+            and w.dtype in (BF16, torch.float32) and all(t.dtype == torch.float32 and t.is_contiguous() for t in small)
+            and mixer.a_log.data_ptr() % 8 == 0
+            and all(getattr(p, "weight", None) is not None and p.weight.dtype == BF16
+                    for p in (mixer.in_proj, mixer.x_proj, mixer.dt_proj, mixer.out_proj)))
+
+
+def mamba_decode_step(mixer, xz, conv, h):
+    """One token of a Mamba mixer behind its in-projection: `xz` `[B, 2 d_inner]` -> `[B, d_inner]` in front of its
+    out-projection. `conv` `[B, d_inner, K-1]` (bf16) and `h` `[B, d_inner, N]` (fp32) are updated in place."""
+    B, C, Ns, r = xz.shape[0], mixer.d_inner, mixer.d_state, mixer.dt_rank
+    w = mixer.conv1d.weight
+    xc = torch.empty(B, C, device=xz.device, dtype=BF16)
+    N.call("sb_mamba_conv_step", xz.data_ptr(), xz.stride(0), conv.data_ptr(), w.data_ptr(), 1 if w.dtype == BF16 else 0,
+           mixer.conv1d.bias.data_ptr(), xc.data_ptr(), B, C, mixer.d_conv, N.stream())
+    proj = decode_linear(xc, mixer.x_proj.weight, mixer.x_proj.bias)
+    delta = decode_linear(proj[:, :r], mixer.dt_proj.weight, mixer.dt_proj.bias)
+    out = torch.empty(B, C, device=xz.device, dtype=BF16)
+    N.call("sb_mamba_scan_step", xc.data_ptr(), delta.data_ptr(), mixer.a_log.data_ptr(), proj[:, r:].data_ptr(),
+           proj[:, r + Ns:].data_ptr(), proj.stride(0), mixer.d.data_ptr(), xz[:, C:].data_ptr(), xz.stride(0), h.data_ptr(),
+           out.data_ptr(), B, C, Ns, N.stream())
+    return out
+
+
 # ------------------------------------------------------------------ mixture of experts
 
 N.register("sb_router_logits", [N.P, N.P, N.P, N.I, N.I, N.I, N.L, N.P])

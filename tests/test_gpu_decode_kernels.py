@@ -139,3 +139,91 @@ def test_rmsnorm_row_per_cta(rows, H):
             y = y[0]
         # one rounding to bf16 next to fp32 statistics
         assert bool(((y.double() - ref).abs() <= (2.0 ** -8 + 2.0 ** -18) * ref.abs() + 1e-30).all())
+
+
+def _hybrid(state_dim, taps, layers=3, hidden=256):
+    from summa_b200 import mal
+    src = f"""
+attention a {{ num_heads: {hidden // 128}  bias: false }}
+ssm s {{ state_dim: {state_dim}  conv_kernel: {taps}  expand: 2 }}
+ffn f {{ hidden_dim: 512  activation: swiglu  bias: false }}
+block ab {{ attention: a  ffn: f  norm: rmsnorm {{ eps: 1e-5 }}  norm_position: pre  residual: true }}
+block mb {{ ssm: s  ffn: f  norm: rmsnorm {{ eps: 1e-5 }}  norm_position: pre  residual: true }}
+model t {{ vocab_size: 512  max_seq_len: 64  hidden_size: {hidden}  num_layers: {layers}  block: ab  pattern: [mb, ab, mb] }}
+"""
+    return mal.parse_mal(src)
+
+
+@gpu
+@pytest.mark.parametrize("B,state_dim,taps", [(1, 8, 2), (3, 16, 4), (2, 32, 3), (8, 64, 4), (9, 128, 4), (1, 256, 4)])
+def test_mamba_decode_step_matches_the_general_path(B, state_dim, taps):
+    """Output and in-place states of the step against the mixer's own forward over one token (scan kernel). Both round at the
+    same places; fp32 sums in another order move single bf16 results by one step (2^-8)."""
+    from summa_b200.models import Transformer
+    from summa_b200.ops import cuda_ops
+    torch.manual_seed(state_dim + taps)
+    with torch.device("cuda"):
+        model = Transformer(_hybrid(state_dim, taps), init_std=0.1)
+    model.prepare_inference(torch.bfloat16)
+    mx = model.layers[0].ssm
+    with torch.no_grad():
+        mx.a_log.copy_(torch.rand_like(mx.a_log) * 3 - 1)
+    assert cuda_ops.mamba_decode_usable(mx)
+    x = torch.randn(B, 256, device="cuda").to(torch.bfloat16)
+    st = mx.make_state(B, "cuda", torch.bfloat16)
+    st.conv.normal_()
+    st.h.normal_()
+    conv, h = st.conv.clone(), st.h.clone()
+    with torch.no_grad():
+        want = mx(x.view(B, 1, 256), st).view(B, 256)
+        got = cuda_ops.decode_linear(cuda_ops.mamba_decode_step(mx, cuda_ops.decode_linear(x, mx.in_proj.weight), conv, h), mx.out_proj.weight)
+    assert torch.equal(conv, st.conv.view_as(conv)) or float((conv.float() - st.conv.float()).abs().max()) <= 2.0 ** -7 * float(st.conv.float().abs().max())
+    for a, b in ((h, st.h), (got, want)):
+        assert float((a.double() - b.double()).norm() / b.double().norm()) <= 2.0 ** -7
+
+
+@gpu
+@pytest.mark.parametrize("B", [1, 5, 9])
+def test_hybrid_graph_decode_against_eager(B):
+    """The captured step of a model with recurrent blocks: states after one token, repeated and continued requests."""
+    from summa_b200.models import Transformer
+    from summa_b200.models.engine import InferenceEngine
+    from summa_b200.ops import native
+    torch.manual_seed(B)
+    with torch.device("cuda"):
+        model = Transformer(_hybrid(16, 4), init_std=0.1)
+    model.prepare_inference(torch.bfloat16)
+    prompt = torch.randint(0, 512, (B, 7), device="cuda")
+
+    def after(use_graph, steps):
+        eng = InferenceEngine(model)
+        eng.use_graph = use_graph
+        eng.reset(B, 40)
+        first = eng.prefill(prompt)
+        eng.decode(first, steps)
+        assert (eng._graph is not None) == use_graph
+        return eng
+    g, e = after(True, 1), after(False, 1)
+    for a, b in zip(g.state.layers, e.state.layers):
+        for k in vars(b):
+            u, v = getattr(a, k), getattr(b, k)
+            if not torch.is_tensor(u):
+                assert u == v
+                continue
+            assert u.dtype == v.dtype and float((u.double() - v.double()).norm() / v.double().norm().clamp_min(1e-9)) <= 2e-2
+    # the same request again on the kept graph, and in two halves: identical
+    eng = after(True, 6)
+    assert eng._graph.graph is not None
+    runs = []
+    for split in ((6,), (6,), (2, 4)):
+        eng.reset(B, 40)
+        tok, out = eng.prefill(prompt), []
+        for n in split:
+            out.append(eng.decode(tok, n))
+            tok = out[-1][:, -1:]
+        runs.append((torch.cat(out, 1), [vars(s).copy() for s in eng.state.layers]))
+    for toks, states in runs[1:]:
+        assert torch.equal(toks, runs[0][0])
+        for a, b in zip(states, runs[0][1]):
+            assert "h" not in a or torch.equal(a["h"], b["h"])
+    assert native.read_error_flag() == 0
