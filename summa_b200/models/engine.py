@@ -131,7 +131,9 @@ class _GraphDecoder:
             elif (not isinstance(a, MultiHeadAttention) or a.head_dim != 128 or a.window is not None or a.q_norm is not None
                     or not a.use_rope or not a.causal or a.num_heads // a.num_kv_heads > 8):
                 return None
-        if cfgm.embeddings.scale is not None or model.stream_dtype != torch.bfloat16:
+        table = model.embedding.weight
+        if (cfgm.embeddings.scale is not None or model.stream_dtype != torch.bfloat16 or table.dtype != torch.bfloat16
+                or not table.is_contiguous() or table.shape[1] % 2):
             return None
         return cls(model, state, max_steps)
 
@@ -159,13 +161,19 @@ class _GraphDecoder:
             self.ws = torch.empty(need, dtype=torch.float32, device=dev)
         P, I, L, F = native.P, native.I, native.L, native.F
         native.register("sb_decode_rope_append", [P] * 6 + [I, I, I, I, L, P, I, P])
+        native.register("sb_decode_embed", [P, P, P, I, I, L, P, P, P])
+        native.register("sb_decode_pick", [P, P, I, I, L, I, P, P, L, P])
         native.register("sb_attention_decode_dyn", [P] * 5 + [I, I, I, P, I, I, I] + [P] * 4 + [F, I, P])
         self.graph = None
 
     def _step(self):
+        from ..ops import native
         from .quantized import QuantLinear, in_proj_swiglu
         m, B = self.model, self.B
-        h = torch.nn.functional.embedding(self.tok.view(-1), m.embedding.weight).to(torch.bfloat16)
+        table = m.embedding.weight
+        h = torch.empty(B, table.shape[1], dtype=torch.bfloat16, device=table.device)
+        native.call("sb_decode_embed", self.tok.data_ptr(), table.data_ptr(), h.data_ptr(), B, table.shape[1], table.shape[0],
+                    self.pos.data_ptr(), self.col.data_ptr(), native.stream())
         cos, sin = m.rope(h.device) or (None, None)
         for i, (blk, st) in enumerate(zip(m.layers, self.state.layers)):
             if blk.ssm is not None:
@@ -181,12 +189,12 @@ class _GraphDecoder:
                 u = self._norm_proj(blk.ffn_norm, ff.in_proj, h)
                 u = ops.gated_act(u, ff.act) if ff.gated else ops.activation(ff.act, u)
             h = self._proj_add(ff.down_proj, u, h)
-        logits = m.project_logits(m.final_norm(h))
-        nxt = ops.argmax(logits).view(B, 1)
-        self.out.scatter_(1, self.col.expand(B, 1), nxt)
-        self.tok.copy_(nxt)
-        self.pos += 1
-        self.col += 1
+        head = m.lm_head
+        logits = (m.project_logits(m.final_norm(h)) if head is None
+                  else self._norm_proj(m.final_norm, head, h)[..., :m.cfg.vocab_size])
+        native.call("sb_decode_pick", logits.data_ptr(), self.out.data_ptr(), B, logits.shape[1], logits.stride(0),
+                    1 if logits.dtype == torch.bfloat16 else 0, self.tok.data_ptr(), self.col.data_ptr(), self.out.stride(0),
+                    native.stream())
 
     def _attend(self, blk, st, h, cos, sin):
         """The attention branch of a block with its residual: qkv projection, RoPE, cache append, split-KV attention, o_proj."""
@@ -259,8 +267,8 @@ class _GraphDecoder:
             conv.copy_(self.state.layers[i].conv)
             hid.copy_(self.state.layers[i].h)
         self.tok.copy_(first)
-        self.pos.fill_(start)
-        self.col.zero_()
+        self.pos.fill_(start - 1)                         # the step's first kernel moves both on
+        self.col.fill_(-1)
         done = 0
         if self.graph is None:
             self._step()                                  # eager: warms every lazy allocation and attribute

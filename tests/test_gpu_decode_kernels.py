@@ -227,3 +227,18 @@ def test_hybrid_graph_decode_against_eager(B):
         for a, b in zip(states, runs[0][1]):
             assert "h" not in a or torch.equal(a["h"], b["h"])
     assert native.read_error_flag() == 0
+
+
+@gpu
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("rows,vocab,ld,off", [(1, 1, 8, 0), (3, 32000, 32064, 0), (2, 8191, 8192, 0), (2, 1003, 1003, 0), (2, 50, 64, 1)])
+def test_argmax_rows_vector_and_scalar(dtype, rows, vocab, ld, off):
+    """Aligned and unaligned rows against torch (lowest index among equals: values are drawn from few)."""
+    from summa_b200 import ops
+    torch.manual_seed(vocab)
+    buf = torch.randint(-9, 9, (rows * ld + off,), device="cuda").to(dtype)
+    x = buf[off:].view(rows, ld)[:, :vocab]
+    want = torch.tensor([int((r == r.max()).nonzero()[0]) for r in x.float().cpu()])
+    assert torch.equal(ops.argmax(x).cpu(), want)
+    x[0].fill_(float("-inf"))
+    assert int(ops.argmax(x)[0]) == 0
