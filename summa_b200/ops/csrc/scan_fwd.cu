@@ -1,9 +1,9 @@
 // Mamba-1 kernels, forward side: causal depthwise conv1d (+SiLU), the segmented
 // selective scan for training / prefill, and the single-token decode step.
 //
-// Scan layout: one thread owns 16 consecutive states of one channel and carries them in
-// registers for the whole sequence. A block covers 16 channels of one batch row with N / 16
-// state groups (two per warp) and walks the sequence in 16-step segments whose inputs
+// Scan layout: one thread owns 4..16 consecutive states of one channel and carries them in
+// registers for the whole sequence. A block covers 16 or 32 channels of one batch row with all
+// its state groups and walks the sequence in 16-step segments whose inputs
 // (softplus(delta), u, B_t, C_t) are fetched asynchronously one segment ahead and staged in
 // shared memory as fp32. At every segment start the state is written to a checkpoint tensor
 // for the backward pass. This removes the reference design's N <= 16 limit: N = 8 .. 256
@@ -395,12 +395,17 @@ extern "C" int sb_scan_fwd(const void* u, const void* delta, const float* A, con
   p.B = B; p.T = T; p.C = C; p.ld_u = ld_u; p.ld_d = ld_d; p.ld_b = ld_b; p.ld_c = ld_c;
   p.vec = C % 8 == 0 && ld_u % 8 == 0 && ld_d % 8 == 0 && ld_b % 8 == 0 && ld_c % 8 == 0 &&
           (((uintptr_t)u | (uintptr_t)delta | (uintptr_t)Bm | (uintptr_t)Cm) & 15) == 0;
+  // States per thread and channels per block. The sequence is serial, so the warps in flight are B C N / (32 states per
+  // thread) however long it is: few states per thread until there are about 20 warps per SM. N 16, 4 states instead of 16:
+  // B 27 T 1024 C 1024 396 -> 254 us, B 24 T 301 119 -> 78; N 128, 8 instead of 16: B 1 T 4096 C 3072 1136 -> 999 us (32
+  // channels, one block per SM at most), B 2 T 8192 2889 -> 2881 (16 channels; 3493 with 32, whose last round is short).
+  const bool one_round = (long)B * ((C + 31) / 32) <= num_sms();
   switch (N) {
-    case 8: return launch_scan_fwd<8, 8, 32>(p, st);
-    case 16: return launch_scan_fwd<16, 16, 32>(p, st);
-    case 32: return launch_scan_fwd<32, 16, 16>(p, st);
-    case 64: return launch_scan_fwd<64, 16, 16>(p, st);
-    case 128: return launch_scan_fwd<128, 16, 16>(p, st);
+    case 8: return launch_scan_fwd<8, 4, 32>(p, st);
+    case 16: return launch_scan_fwd<16, 4, 32>(p, st);
+    case 32: return launch_scan_fwd<32, 8, 32>(p, st);
+    case 64: return launch_scan_fwd<64, 8, 16>(p, st);
+    case 128: return one_round ? launch_scan_fwd<128, 8, 32>(p, st) : launch_scan_fwd<128, 8, 16>(p, st);
     case 256: return launch_scan_fwd<256, 16, 16>(p, st);
     default:
       fprintf(stderr, "summa_b200: selective scan supports d_state in {8,16,32,64,128,256}, got %d\n", N);
