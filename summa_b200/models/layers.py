@@ -182,7 +182,9 @@ class MambaMixer(nn.Module):
     def forward(self, x: torch.Tensor, state: Optional[MambaState] = None) -> torch.Tensor:
         B, T, _ = x.shape
         xz = self.in_proj(x)
-        xs, z = xz[..., :self.d_inner], xz[..., self.d_inner:]
+        # split, not slices: the backward of a split is one concatenation, of slices a zero-filled tensor, a copy and an
+        # addition per piece
+        xs, z = xz.split([self.d_inner, self.d_inner], dim=-1)
         conv_state = state.conv if state is not None else None
         if state is not None:
             K1 = self.d_conv - 1
@@ -190,9 +192,7 @@ class MambaMixer(nn.Module):
             new_conv = hist[..., -K1:].contiguous() if K1 > 0 else state.conv
         xc = ops.conv1d_silu(xs, self.conv1d.weight, self.conv1d.bias, conv_state)
         proj = self.x_proj(xc)
-        dt_in = proj[..., :self.dt_rank]
-        Bm = proj[..., self.dt_rank:self.dt_rank + self.d_state]
-        Cm = proj[..., self.dt_rank + self.d_state:]
+        dt_in, Bm, Cm = proj.split([self.dt_rank, self.d_state, self.d_state], dim=-1)
         delta = self.dt_proj(dt_in)
         A = -torch.exp(self.a_log.float())
         h0 = state.h if state is not None else None
