@@ -335,9 +335,9 @@ __device__ __forceinline__ void lane_group_reduce(float (&v)[V], int lane) {
 
 constexpr int SCANT_SUB = 4;       // replay depth of the tiled kernel
 
-// Tiled backward, N >= 16. A thread owns a 4-channel x 4-state tile (16 states and their gradients in registers
-// as 8 f32x2 pairs); a warp is 8 channel groups x 4 state groups = 32 channels x 16 states; a block is NB / 16
-// warps over NB <= 64 states (blockIdx.z picks the slice when N > NB). Compared with one channel per lane this
+// Tiled backward, N >= 16. A thread owns a 4-channel x SPT-state tile (SPT = 4: 16 states and their gradients in
+// registers as 8 f32x2 pairs); a warp is 8 channel groups x 4 state groups = 32 channels x 4 SPT states; a block is
+// NB / (4 SPT) warps over NB <= 64 states (blockIdx.z picks the slice when N > NB). Compared with one channel per lane this
 // puts both kinds of per-step sums partly inside the thread: the B_t / C_t gradients (sums over channels) are
 // accumulated over the thread's 4 channels by the fma that computes them and then reduced over 8 lanes
 // (7 shuffles for 8 values); the delta / u gradients (sums over states) likewise over 4 lanes (6 shuffles for
@@ -346,14 +346,14 @@ constexpr int SCANT_SUB = 4;       // replay depth of the tiled kernel
 // checkpoint in two levels: the states at steps 4, 8, 12 stay in registers, then every 4-step group is replayed
 // into a per-thread column of shared memory and swept in reverse. The next segment's inputs are fetched
 // asynchronously during the sweep.
-template <int N, int NB>
-__global__ void __launch_bounds__(2 * NB, NB == 64 ? 3 : 4)
+template <int N, int NB, int SPT>
+__global__ void __launch_bounds__(8 * NB / SPT, NB == 64 ? 3 : 512 / (8 * NB / SPT))
 selective_scan_bwd_tile_kernel(const ScanBwdParams p) {
-  constexpr int NW = NB / 16;
+  constexpr int NW = NB / (4 * SPT);
   constexpr int THREADS = 32 * NW;
   constexpr int SEG = SCAN_SEG, SUB = SCANT_SUB, NSUB = SEG / SUB;
   constexpr int CH = 32;
-  constexpr int NPR = 8;                   // f32x2 pairs per thread: pair 2 i + q = channel i, states 2 q, 2 q + 1
+  constexpr int NQ = SPT / 2, NPR = 4 * NQ;  // f32x2 pairs per thread: pair NQ i + q = channel i, states 2 q, 2 q + 1
   constexpr float LN2 = 0.6931471805599453f;
   extern __shared__ __align__(16) float sm[];
   float* s_dt = sm;                        // [SEG][CH] softplus(delta)
@@ -361,8 +361,8 @@ selective_scan_bwd_tile_kernel(const ScanBwdParams p) {
   float* s_dy = s_u + SEG * CH;
   float* s_B = s_dy + SEG * CH;            // [SEG][NB]
   float* s_C = s_B + SEG * NB;
-  float* s_po = s_C + SEG * NB;            // [NW][SEG][2 CH] per-warp sums over the warp's 16 states: ddt | du
-  uint64_t* s_hp = reinterpret_cast<uint64_t*>(s_po + NW * SEG * 2 * CH);   // [SUB][NPR][THREADS] pre-step states
+  float* s_po = s_C + SEG * NB;            // [2][NW][SUB][2 CH] per-warp sums over the warp's states: ddt | du
+  uint64_t* s_hp = reinterpret_cast<uint64_t*>(s_po + 2 * NW * SUB * 2 * CH);   // [SUB][NPR][THREADS] pre-step states
   __nv_bfloat16* r_dt = reinterpret_cast<__nv_bfloat16*>(s_hp + SUB * NPR * THREADS);   // raw staging
   __nv_bfloat16* r_u = r_dt + SEG * CH;
   __nv_bfloat16* r_dy = r_u + SEG * CH;
@@ -374,7 +374,7 @@ selective_scan_bwd_tile_kernel(const ScanBwdParams p) {
   const int c0 = blockIdx.x * CH;
   const int cb = c0 + 4 * lc;              // first channel of this thread
   const int nb0 = blockIdx.z * NB;
-  const int nl = 16 * w + 4 * ln;          // first state of this thread inside the block's slice
+  const int nl = 4 * SPT * w + SPT * ln;          // first state of this thread inside the block's slice
   const int n0 = nb0 + nl;
   const bool vec = p.vec != 0;
   uint64_t A2[NPR], dh[NPR], dAacc[NPR];
@@ -382,15 +382,15 @@ selective_scan_bwd_tile_kernel(const ScanBwdParams p) {
   for (int i = 0; i < 4; ++i) {
     const bool ok = cb + i < p.C;
 #pragma unroll
-    for (int q = 0; q < 2; ++q) {
+    for (int q = 0; q < NQ; ++q) {
       const long o = (long)(cb + i) * N + n0 + 2 * q;
-      A2[2 * i + q] = ok ? f2_pack(p.A[o] * 1.4426950408889634f, p.A[o + 1] * 1.4426950408889634f) : f2_pack(0.f, 0.f);
+      A2[NQ * i + q] = ok ? f2_pack(p.A[o] * 1.4426950408889634f, p.A[o + 1] * 1.4426950408889634f) : f2_pack(0.f, 0.f);
       const long od = ((long)b * p.C + cb + i) * N + n0 + 2 * q;
-      dh[2 * i + q] = (ok && p.dh_out) ? f2_pack(p.dh_out[od], p.dh_out[od + 1]) : f2_pack(0.f, 0.f);
-      dAacc[2 * i + q] = f2_pack(0.f, 0.f);
+      dh[NQ * i + q] = (ok && p.dh_out) ? f2_pack(p.dh_out[od], p.dh_out[od + 1]) : f2_pack(0.f, 0.f);
+      dAacc[NQ * i + q] = f2_pack(0.f, 0.f);
     }
   }
-  float dDacc = 0.f;                        // threads 0..31 of slice 0: channel c0 + tid
+  float dDacc = 0.f;                        // slice 0: channel c0 + lane, this warp's steps
   const int nseg = (p.T + SEG - 1) / SEG;
   auto stage = [&](int seg) {
     const long row0 = (long)b * p.T + seg * SEG;
@@ -402,29 +402,48 @@ selective_scan_bwd_tile_kernel(const ScanBwdParams p) {
     scan_stage_rows(smem_u32(r_C), r_C, p.Cm, p.ld_c, row0, rv, SEG, nb0, NB, NB, vec, tid, THREADS);
     cp_async_commit();
   };
-  // the segment's checkpoint: this thread's 4 x 4 tile as 8 pairs
+  // the segment's checkpoint: this thread's 4 x SPT tile
   auto load_ckpt = [&](int seg, uint64_t (&h)[NPR]) {
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-      float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (cb + i < p.C) v = *reinterpret_cast<const float4*>(p.ckpt + (((long)b * nseg + seg) * p.C + cb + i) * N + n0);
-      h[2 * i] = f2_pack(v.x, v.y);
-      h[2 * i + 1] = f2_pack(v.z, v.w);
+      const float* src = p.ckpt + (((long)b * nseg + seg) * p.C + cb + i) * N + n0;
+      if (SPT == 4) {
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (cb + i < p.C) v = *reinterpret_cast<const float4*>(src);
+        h[NQ * i] = f2_pack(v.x, v.y);
+        h[NQ * i + NQ - 1] = f2_pack(v.z, v.w);
+      } else {
+        float2 v = make_float2(0.f, 0.f);
+        if (cb + i < p.C) v = *reinterpret_cast<const float2*>(src);
+        h[NQ * i] = f2_pack(v.x, v.y);
+      }
     }
   };
-  // one forward step on all 8 pairs
+  // B_t or C_t of this thread's states
+  auto load_pairs = [&](const float* at, uint64_t (&v)[NQ]) {
+    if (SPT == 4) {
+      const ulonglong2 t = *reinterpret_cast<const ulonglong2*>(at);
+      v[0] = t.x;
+      v[NQ - 1] = t.y;
+    } else {
+      v[0] = *reinterpret_cast<const uint64_t*>(at);
+    }
+  };
+  // one forward step on all pairs
   auto fwd_step = [&](int tt, uint64_t (&h)[NPR]) {
     const float4 dt4 = *reinterpret_cast<const float4*>(s_dt + tt * CH + 4 * lc);
     const float4 u4 = *reinterpret_cast<const float4*>(s_u + tt * CH + 4 * lc);
-    const ulonglong2 bq = *reinterpret_cast<const ulonglong2*>(s_B + tt * NB + nl);
+    uint64_t bp[NQ];
+    load_pairs(s_B + tt * NB + nl, bp);
     const float dtv[4] = {dt4.x, dt4.y, dt4.z, dt4.w}, uv[4] = {u4.x, u4.y, u4.z, u4.w};
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       const uint64_t dt2 = f2_pack(dtv[i], dtv[i]);
       const float duv = dtv[i] * uv[i];
       const uint64_t du2 = f2_pack(duv, duv);
-      h[2 * i] = f2_fma(exp2_xu2_packed(f2_mul(dt2, A2[2 * i])), h[2 * i], f2_mul(du2, bq.x));
-      h[2 * i + 1] = f2_fma(exp2_xu2_packed(f2_mul(dt2, A2[2 * i + 1])), h[2 * i + 1], f2_mul(du2, bq.y));
+#pragma unroll
+      for (int q = 0; q < NQ; ++q)
+        h[NQ * i + q] = f2_fma(exp2_xu2_packed(f2_mul(dt2, A2[NQ * i + q])), h[NQ * i + q], f2_mul(du2, bp[q]));
     }
   };
   stage(nseg - 1);
@@ -433,6 +452,12 @@ selective_scan_bwd_tile_kernel(const ScanBwdParams p) {
     const int steps = min(SEG, p.T - t0);
     cp_async_wait_all();
     __syncthreads();      // staging complete; the previous segment's epilogue is done with s_po / s_dy / s_u
+    if (seg > 0) {          // the next checkpoint's lines on their way to L2
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        if (ln == 0 && cb + i < p.C)
+          asm volatile("prefetch.global.L2 [%0];" ::"l"(p.ckpt + (((long)b * nseg + seg - 1) * p.C + cb + i) * N + n0));
+    }
     for (int i = tid; i < SEG * CH; i += THREADS) {
       const int tt = i / CH, cc = i - tt * CH;
       const bool ok = tt < steps && c0 + cc < p.C;
@@ -487,12 +512,14 @@ selective_scan_bwd_tile_kernel(const ScanBwdParams p) {
         const float4 dt4 = *reinterpret_cast<const float4*>(s_dt + tt * CH + 4 * lc);
         const float4 u4 = *reinterpret_cast<const float4*>(s_u + tt * CH + 4 * lc);
         const float4 dy4 = *reinterpret_cast<const float4*>(s_dy + tt * CH + 4 * lc);
-        const ulonglong2 bq = *reinterpret_cast<const ulonglong2*>(s_B + tt * NB + nl);
-        const ulonglong2 cq = *reinterpret_cast<const ulonglong2*>(s_C + tt * NB + nl);
-        const uint64_t bp[2] = {bq.x, bq.y}, cp[2] = {cq.x, cq.y};
+        uint64_t bp[NQ], cp[NQ];
+        load_pairs(s_B + tt * NB + nl, bp);
+        load_pairs(s_C + tt * NB + nl, cp);
         const float dtv[4] = {dt4.x, dt4.y, dt4.z, dt4.w}, uv[4] = {u4.x, u4.y, u4.z, u4.w};
         const float dyv[4] = {dy4.x, dy4.y, dy4.z, dy4.w};
-        uint64_t dBa[2] = {f2_pack(0.f, 0.f), f2_pack(0.f, 0.f)}, dCa[2] = {f2_pack(0.f, 0.f), f2_pack(0.f, 0.f)};
+        uint64_t dBa[NQ], dCa[NQ];
+#pragma unroll
+        for (int q = 0; q < NQ; ++q) dBa[q] = dCa[q] = f2_pack(0.f, 0.f);
         float r2[8];                        // [0,4): ddt of the 4 channels, [4,8): du
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
@@ -501,8 +528,8 @@ selective_scan_bwd_tile_kernel(const ScanBwdParams p) {
           const uint64_t du2 = f2_pack(duv, duv);
           uint64_t sA = f2_pack(0.f, 0.f), sB = f2_pack(0.f, 0.f);
 #pragma unroll
-          for (int q = 0; q < 2; ++q) {
-            const int j = 2 * i + q;
+          for (int q = 0; q < NQ; ++q) {
+            const int j = NQ * i + q;
             const uint64_t dA = exp2_xu2_packed(f2_mul(dt2, A2[j]));
             const uint64_t hprev = s_hp[(k * NPR + j) * THREADS + tid];
             const uint64_t ht = f2_fma(dA, hprev, f2_mul(du2, bp[q]));      // h_t
@@ -522,46 +549,52 @@ selective_scan_bwd_tile_kernel(const ScanBwdParams p) {
           r2[i] = fmaf(LN2, a0 + a1, uv[i] * sb2);
           r2[4 + i] = dtv[i] * sb2;
         }
-        float r1[8];                        // [0,4): dB of the 4 states, [4,8): dC
-        f2_unpack(dBa[0], r1[0], r1[1]);
-        f2_unpack(dBa[1], r1[2], r1[3]);
-        f2_unpack(dCa[0], r1[4], r1[5]);
-        f2_unpack(dCa[1], r1[6], r1[7]);
-        lane_group_reduce<8, 8, 0>(r1, lane);     // over the 8 channel groups: one total per lane
+        float r1[2 * SPT];                  // [0, SPT): dB of the states, [SPT, 2 SPT): dC
+#pragma unroll
+        for (int q = 0; q < NQ; ++q) {
+          f2_unpack(dBa[q], r1[2 * q], r1[2 * q + 1]);
+          f2_unpack(dCa[q], r1[SPT + 2 * q], r1[SPT + 2 * q + 1]);
+        }
+        // over the 8 channel groups: one total per lane (SPT = 2: per pair of lanes, the second adds its half first)
+        if constexpr (SPT == 2) {
+#pragma unroll
+          for (int v = 0; v < 4; ++v) r1[v] += __shfl_xor_sync(0xffffffffu, r1[v], 4);
+          lane_group_reduce<4, 4, 0>(r1, lane);
+        } else {
+          lane_group_reduce<2 * SPT, 8, 0>(r1, lane);
+        }
         lane_group_reduce<8, 4, 3>(r2, lane);     // over the 4 state groups: two totals per lane
         {
-          const int idx = ((lane & 1) << 2) | (lane & 2) | ((lane >> 2) & 1);
-          const long o = (((long)blockIdx.x * p.B + b) * p.T + t0 + tt) * N + n0 + (idx & 3);
-          if (idx < 4) p.dB_part[o] = r1[0];
-          else p.dC_part[o] = r1[0];
+          const int idx = SPT == 4 ? ((lane & 1) << 2) | (lane & 2) | ((lane >> 2) & 1) : ((lane & 1) << 1) | ((lane >> 1) & 1);
+          const long o = (((long)blockIdx.x * p.B + b) * p.T + t0 + tt) * N + n0 + (idx & (SPT - 1));
+          if (SPT == 4 || !(lane & 4)) {
+            if (idx < SPT) p.dB_part[o] = r1[0];
+            else p.dC_part[o] = r1[0];
+          }
         }
         {
           const int idx = (((lane >> 3) & 1) << 2) | (((lane >> 4) & 1) << 1);     // even: values idx, idx + 1
-          float* o = s_po + (w * SEG + tt) * 2 * CH + (idx < 4 ? 0 : CH) + 4 * lc + (idx & 3);
+          float* o = s_po + (((sb_ & 1) * NW + w) * SUB + k) * 2 * CH + (idx < 4 ? 0 : CH) + 4 * lc + (idx & 3);
           *reinterpret_cast<float2*>(o) = make_float2(r2[0], r2[1]);
         }
       }
-    }
-    __syncthreads();
-    {
-      float* pd = p.ddt_part + ((long)blockIdx.z * p.B + b) * p.T * p.C;
-      float* pu = p.du_part + ((long)blockIdx.z * p.B + b) * p.T * p.C;
-      for (int i = tid; i < steps * CH; i += THREADS) {
-        const int tt = i / CH, cc = i - tt * CH;
-        if (c0 + cc < p.C) {
+      // the group's sums over the warps; the other buffer takes the next group meanwhile
+      __syncthreads();
+      for (int i = tid; i < SUB * CH; i += THREADS) {
+        const int k = i / CH, cc = i - k * CH, tt = sb_ * SUB + k;
+        if (tt < steps && c0 + cc < p.C) {
+          const float* po = s_po + ((sb_ & 1) * NW * SUB + k) * 2 * CH + cc;
           float a = 0.f, e = 0.f;
 #pragma unroll
           for (int ww = 0; ww < NW; ++ww) {
-            a += s_po[(ww * SEG + tt) * 2 * CH + cc];
-            e += s_po[(ww * SEG + tt) * 2 * CH + CH + cc];
+            a += po[ww * SUB * 2 * CH];
+            e += po[ww * SUB * 2 * CH + CH];
           }
-          const long o = ((long)t0 + tt) * p.C + c0 + cc;
-          pd[o] = a;
-          pu[o] = e;
+          const long o = (((long)blockIdx.z * p.B + b) * p.T + t0 + tt) * p.C + c0 + cc;
+          p.ddt_part[o] = a;
+          p.du_part[o] = e;
+          dDacc = fmaf(s_dy[tt * CH + cc], s_u[tt * CH + cc], dDacc);
         }
-      }
-      if (tid < CH && blockIdx.z == 0) {
-        for (int tt = 0; tt < steps; ++tt) dDacc = fmaf(s_dy[tt * CH + tid], s_u[tt * CH + tid], dDacc);
       }
     }
   }
@@ -569,10 +602,10 @@ selective_scan_bwd_tile_kernel(const ScanBwdParams p) {
   for (int i = 0; i < 4; ++i) {
     if (cb + i < p.C) {
 #pragma unroll
-      for (int q = 0; q < 2; ++q) {
+      for (int q = 0; q < NQ; ++q) {
         float a0, a1, d0, d1;
-        f2_unpack(dAacc[2 * i + q], a0, a1);
-        f2_unpack(dh[2 * i + q], d0, d1);
+        f2_unpack(dAacc[NQ * i + q], a0, a1);
+        f2_unpack(dh[NQ * i + q], d0, d1);
         atomicAdd(p.dA + (long)(cb + i) * N + n0 + 2 * q, a0);
         atomicAdd(p.dA + (long)(cb + i) * N + n0 + 2 * q + 1, a1);
         if (p.dh0) {
@@ -582,15 +615,15 @@ selective_scan_bwd_tile_kernel(const ScanBwdParams p) {
       }
     }
   }
-  if (tid < CH && blockIdx.z == 0 && c0 + tid < p.C) atomicAdd(p.dD + c0 + tid, dDacc);
+  if (blockIdx.z == 0 && c0 + lane < p.C) atomicAdd(p.dD + c0 + lane, dDacc);
 }
 
-template <int N, int NB>
+template <int N, int NB, int SPT>
 static int launch_scan_bwd_tile(const ScanBwdParams& p, cudaStream_t st) {
-  constexpr int NW = NB / 16, THREADS = 32 * NW;
-  const int smem = (3 * SCAN_SEG * 32 + 2 * SCAN_SEG * NB + NW * SCAN_SEG * 64) * sizeof(float) +
-                   SCANT_SUB * 8 * THREADS * sizeof(uint64_t) + (3 * SCAN_SEG * 32 + 2 * SCAN_SEG * NB) * sizeof(__nv_bfloat16);
-  auto kern = selective_scan_bwd_tile_kernel<N, NB>;
+  constexpr int NW = NB / (4 * SPT), THREADS = 32 * NW;
+  const int smem = (3 * SCAN_SEG * 32 + 2 * SCAN_SEG * NB + 2 * NW * SCANT_SUB * 64) * sizeof(float) +
+                   SCANT_SUB * 2 * SPT * THREADS * sizeof(uint64_t) + (3 * SCAN_SEG * 32 + 2 * SCAN_SEG * NB) * sizeof(__nv_bfloat16);
+  auto kern = selective_scan_bwd_tile_kernel<N, NB, SPT>;
   if (smem > 48 * 1024) SB_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
   dim3 grid((p.C + 31) / 32, p.B, N / NB);
   kern<<<grid, THREADS, smem, st>>>(p);
@@ -698,49 +731,52 @@ static int launch_scan_bwd(const ScanBwdParams& p, cudaStream_t st) {
 
 // ---------------------------------------------------------------------------- conv1d backward
 // dy is the gradient of silu(conv(x)+b) (or of the plain conv when silu == 0).
-// Thread = 8 channels x TT steps; block = 32 channel groups x 8 time chunks.
+// Thread = 4 channels x t_per_thread steps; block = 32 channel groups x 8 time chunks. What bounds it is the latency of
+// the two loads a step needs: with 8 channels per thread the windows took 200 registers (8 warps per SM, nothing in
+// flight): B 2 T 8192 C 3072 340 us against 45 us of traffic. Four channels, the loads of a step
+// issued two steps ahead: 120 us (B 27 T 1024 C 1024: 170 -> 66).
 template <int K, bool SILU>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, 2)
 conv1d_bwd_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict__ w, const float* __restrict__ bias,
                   const __nv_bfloat16* __restrict__ dy, __nv_bfloat16* __restrict__ dx, float* __restrict__ dw,
                   float* __restrict__ db, int B, int T, int C, long ldx, long lddx, int t_per_thread) {
+  constexpr int CPT = 4;
   const int lane = threadIdx.x & 31, wy = threadIdx.x >> 5;
-  const int cg = blockIdx.x * 32 + lane;
-  const int c0 = cg * 8;
+  const int c0 = (blockIdx.x * 32 + lane) * CPT;
   const int b = blockIdx.z;
   const int t_begin = (blockIdx.y * 8 + wy) * t_per_thread;
   const bool ok = c0 < C;
-  float wk[K][8], bs[8], gw[K][8], gb[8];
+  float wk[K][CPT], bs[CPT], gw[K][CPT], gb[CPT];
 #pragma unroll
-  for (int j = 0; j < 8; ++j) {
+  for (int j = 0; j < CPT; ++j) {
     bs[j] = (ok && bias) ? bias[c0 + j] : 0.f;
     gb[j] = 0.f;
 #pragma unroll
     for (int k = 0; k < K; ++k) { wk[k][j] = ok ? w[(c0 + j) * K + k] : 0.f; gw[k][j] = 0.f; }
   }
-  auto load8 = [&](const __nv_bfloat16* base, long ld, int t, float* o) {
-    if (ok && t >= 0 && t < T) {
-      const uint4 v = *reinterpret_cast<const uint4*>(base + ((long)b * T + t) * ld + c0);
-      o[0] = bf16_lo(v.x); o[1] = bf16_hi(v.x); o[2] = bf16_lo(v.y); o[3] = bf16_hi(v.y);
-      o[4] = bf16_lo(v.z); o[5] = bf16_hi(v.z); o[6] = bf16_lo(v.w); o[7] = bf16_hi(v.w);
-    } else {
-#pragma unroll
-      for (int j = 0; j < 8; ++j) o[j] = 0.f;
-    }
+  auto fetch = [&](const __nv_bfloat16* base, long ld, int t) {
+    return ok && t >= 0 && t < T ? *reinterpret_cast<const uint2*>(base + ((long)b * T + t) * ld + c0) : make_uint2(0u, 0u);
+  };
+  auto unpack = [](const uint2& v, float (&o)[CPT]) {
+    o[0] = bf16_lo(v.x); o[1] = bf16_hi(v.x); o[2] = bf16_lo(v.y); o[3] = bf16_hi(v.y);
   };
   // dpre[t] for t in [t_begin, t_begin + tpt + K - 1): needs x[t-K+1 .. t]
   // dx[t] = sum_k w[k] * dpre[t + (K-1-k)];  dw[k] += dpre[t] * x[t-(K-1-k)]
-  float xw[2 * K - 1][8];     // x window: xw[i] = x[t - (K-1) + i], i in [0, 2K-1) covers t..t+K-1 lookahead
-  float dp[K][8];             // dp[i] = dpre[t + i]
-  // initialise windows for t = t_begin
+  float xw[2 * K - 1][CPT];     // x window: xw[i] = x[t - (K-1) + i], i in [0, 2K-1) covers t..t+K-1 lookahead
+  float dp[K][CPT];             // dp[i] = dpre[t + i]
+  {
+    uint2 raw[2 * K - 1];
 #pragma unroll
-  for (int i = 0; i < 2 * K - 1; ++i) load8(x, ldx, t_begin - (K - 1) + i, xw[i]);
-  auto dpre_at = [&](int i, int t, float* o) {
-    // dpre at time t using x window positions i-(K-1)..i relative to xw index base
-    float g[8];
-    load8(dy, (long)C, t, g);
+    for (int i = 0; i < 2 * K - 1; ++i) raw[i] = fetch(x, ldx, t_begin - (K - 1) + i);
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
+    for (int i = 0; i < 2 * K - 1; ++i) unpack(raw[i], xw[i]);
+  }
+  auto dpre_of = [&](int i, const uint2& dyv, float (&o)[CPT]) {
+    // dpre using x window positions i .. i + K - 1
+    float g[CPT];
+    unpack(dyv, g);
+#pragma unroll
+    for (int j = 0; j < CPT; ++j) {
       float a = bs[j];
 #pragma unroll
       for (int k = 0; k < K; ++k) a = fmaf(wk[k][j], xw[i + k][j], a);
@@ -752,14 +788,26 @@ conv1d_bwd_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict__
       }
     }
   };
+  {
+    uint2 raw[K];
 #pragma unroll
-  for (int i = 0; i < K; ++i) dpre_at(i, t_begin + i, dp[i]);
+    for (int i = 0; i < K; ++i) raw[i] = fetch(dy, (long)C, t_begin + i);
+#pragma unroll
+    for (int i = 0; i < K; ++i) dpre_of(i, raw[i], dp[i]);
+  }
+  // loads of the step that enters the windows next, two steps ahead
+  uint2 nx[2] = {fetch(x, ldx, t_begin + K), fetch(x, ldx, t_begin + K + 1)};
+  uint2 nd[2] = {fetch(dy, (long)C, t_begin + K), fetch(dy, (long)C, t_begin + K + 1)};
+#pragma unroll 2
   for (int tt = 0; tt < t_per_thread; ++tt) {
     const int t = t_begin + tt;
     if (t >= T) break;
-    float o[8];
+    const uint2 cx = nx[tt & 1], cd = nd[tt & 1];
+    nx[tt & 1] = fetch(x, ldx, t + K + 2);
+    nd[tt & 1] = fetch(dy, (long)C, t + K + 2);
+    float o[CPT];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
+    for (int j = 0; j < CPT; ++j) {
       float a = 0.f;
 #pragma unroll
       for (int k = 0; k < K; ++k) a = fmaf(wk[k][j], dp[K - 1 - k][j], a);
@@ -768,40 +816,35 @@ conv1d_bwd_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict__
 #pragma unroll
       for (int k = 0; k < K; ++k) gw[k][j] = fmaf(dp[0][j], xw[k][j], gw[k][j]);
     }
-    if (ok) {
-      uint4 ov;
-      ov.x = pack_bf16(o[0], o[1]); ov.y = pack_bf16(o[2], o[3]); ov.z = pack_bf16(o[4], o[5]); ov.w = pack_bf16(o[6], o[7]);
-      *reinterpret_cast<uint4*>(dx + ((long)b * T + t) * lddx + c0) = ov;
-    }
+    if (ok) *reinterpret_cast<uint2*>(dx + ((long)b * T + t) * lddx + c0) = make_uint2(pack_bf16(o[0], o[1]), pack_bf16(o[2], o[3]));
     // slide both windows by one step
 #pragma unroll
     for (int i = 0; i < 2 * K - 2; ++i)
 #pragma unroll
-      for (int j = 0; j < 8; ++j) xw[i][j] = xw[i + 1][j];
-    load8(x, ldx, t + K, xw[2 * K - 2]);
+      for (int j = 0; j < CPT; ++j) xw[i][j] = xw[i + 1][j];
+    unpack(cx, xw[2 * K - 2]);
 #pragma unroll
     for (int i = 0; i < K - 1; ++i)
 #pragma unroll
-      for (int j = 0; j < 8; ++j) dp[i][j] = dp[i + 1][j];
-    dpre_at(K - 1, t + K, dp[K - 1]);
+      for (int j = 0; j < CPT; ++j) dp[i][j] = dp[i + 1][j];
+    dpre_of(K - 1, cd, dp[K - 1]);
   }
   // reduce the parameter gradients over the 8 time-chunk warps, then one atomic per value
-  __shared__ float red[8][32][8 * (K + 1) + 1];
+  __shared__ float red[8][32][CPT * (K + 1) + 1];
 #pragma unroll
-  for (int j = 0; j < 8; ++j) {
+  for (int j = 0; j < CPT; ++j) {
     red[wy][lane][j] = gb[j];
 #pragma unroll
-    for (int k = 0; k < K; ++k) red[wy][lane][8 + k * 8 + j] = gw[k][j];
+    for (int k = 0; k < K; ++k) red[wy][lane][CPT + k * CPT + j] = gw[k][j];
   }
   __syncthreads();
-  if (wy == 0 && ok) {
-    for (int v = 0; v < 8 * (K + 1); ++v) {
-      float a = 0.f;
+  for (int v = wy; v < CPT * (K + 1); v += 8) {
+    if (!ok) break;
+    float a = 0.f;
 #pragma unroll
-      for (int r = 0; r < 8; ++r) a += red[r][lane][v];
-      if (v < 8) atomicAdd(db + c0 + v, a);
-      else { const int k = (v - 8) / 8, j = (v - 8) % 8; atomicAdd(dw + (c0 + j) * K + k, a); }
-    }
+    for (int r = 0; r < 8; ++r) a += red[r][lane][v];
+    if (v < CPT) atomicAdd(db + c0 + v, a);
+    else { const int k = (v - CPT) / CPT, j = (v - CPT) % CPT; atomicAdd(dw + (c0 + j) * K + k, a); }
   }
 }
 
@@ -829,11 +872,13 @@ extern "C" int sb_scan_bwd(const void* u, const void* delta, const float* A, con
   int rc, ns = 1;
   switch (N) {
     case 8: rc = launch_scan_bwd<8, 8>(p, st); break;
-    case 16: rc = launch_scan_bwd_tile<16, 16>(p, st); break;
-    case 32: rc = launch_scan_bwd_tile<32, 32>(p, st); break;
-    case 64: rc = launch_scan_bwd_tile<64, 64>(p, st); break;
-    case 128: rc = launch_scan_bwd_tile<128, 64>(p, st); ns = 2; break;
-    case 256: rc = launch_scan_bwd_tile<256, 64>(p, st); ns = 4; break;
+    // Two states per thread where a block would be a single warp (N 16, B 27 T 1024 C 1024: 1281 -> 1084 us with the passes
+    // behind it); from N 32 on four are ahead (N 32 1478 us against 1725, N 128 B 2 T 8192 C 3072 9.8 ms against 12.2).
+    case 16: rc = launch_scan_bwd_tile<16, 16, 2>(p, st); break;
+    case 32: rc = launch_scan_bwd_tile<32, 32, 4>(p, st); break;
+    case 64: rc = launch_scan_bwd_tile<64, 64, 4>(p, st); break;
+    case 128: rc = launch_scan_bwd_tile<128, 64, 4>(p, st); ns = 2; break;
+    case 256: rc = launch_scan_bwd_tile<256, 64, 4>(p, st); ns = 4; break;
     default: return SB_ERR_ARG;
   }
   if (rc) return rc;
@@ -870,7 +915,7 @@ extern "C" int sb_conv1d_bwd(const void* x, const float* w, const float* bias, c
                              float* db, int B, int T, int C, int K, long ldx, long lddx, int silu, cudaStream_t st) {
   SB_CHECK_ARG(B > 0 && T > 0 && C % 8 == 0 && ldx % 8 == 0 && lddx % 8 == 0 && K >= 2 && K <= 4);
   const int tpt = 32;
-  dim3 grid((C / 8 + 31) / 32, (T + 8 * tpt - 1) / (8 * tpt), B);
+  dim3 grid((C / 4 + 31) / 32, (T + 8 * tpt - 1) / (8 * tpt), B);
 #define SB_CONVB(KK)                                                                                               \
   if (silu) conv1d_bwd_kernel<KK, true><<<grid, 256, 0, st>>>((const __nv_bfloat16*)x, w, bias, (const __nv_bfloat16*)dy, \
                                                               (__nv_bfloat16*)dx, dw, db, B, T, C, ldx, lddx, tpt);  \
