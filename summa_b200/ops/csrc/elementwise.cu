@@ -356,18 +356,16 @@ __global__ void qk_rope_kernel(const __nv_bfloat16* __restrict__ in, __nv_bfloat
                                const float* __restrict__ cos_t, const float* __restrict__ sin_t, int T, int S, int Hq,
                                int Hkv, int ld, int pos0, float eps) {
   constexpr int E = D / 32;   // elements per lane (2 or 4)
-  const int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   const int heads = Hq + Hkv;
-  const bool active = gw < T * heads;
-  float dg[E];
+  float dg[2][E];                                         // gain gradients of q and k over this warp's (token, head) items
 #pragma unroll
-  for (int i = 0; i < E; ++i) dg[i] = 0.f;
+  for (int i = 0; i < E; ++i) dg[0][i] = dg[1][i] = 0.f;
   const float* gamma = nullptr;
-  bool is_q = true;
-  if (active) {
+  const int nw = (gridDim.x * blockDim.x) >> 5;
+  for (int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; gw < T * heads; gw += nw) {
     const int t = gw / heads, h = gw - t * heads;
-    is_q = h < Hq;
+    const bool is_q = h < Hq;
     const size_t off = static_cast<size_t>(t) * ld + static_cast<size_t>(h) * D + lane * E;
     const int pos = pos0 + (t % S);
     float v[E], c[E / 2], s[E / 2];
@@ -427,7 +425,9 @@ __global__ void qk_rope_kernel(const __nv_bfloat16* __restrict__ in, __nv_bfloat
         for (int i = 0; i < E; ++i) {
           const float g = gamma[lane * E + i];
           dot += g * v[i] * x[i];
-          dg[i] = v[i] * x[i] * rstd;
+          const float d = v[i] * x[i] * rstd;
+          dg[0][i] += is_q ? d : 0.f;
+          dg[1][i] += is_q ? 0.f : d;
         }
         dot = warp_sum(dot);
         const float coef = dot * rstd * rstd * rstd / D;
@@ -446,9 +446,10 @@ __global__ void qk_rope_kernel(const __nv_bfloat16* __restrict__ in, __nv_bfloat
     __shared__ float acc[2][D];
     for (int i = threadIdx.x; i < 2 * D; i += blockDim.x) (&acc[0][0])[i] = 0.f;
     __syncthreads();
-    if (active) {
 #pragma unroll
-      for (int i = 0; i < E; ++i) atomicAdd(&acc[is_q ? 0 : 1][lane * E + i], dg[i]);
+    for (int i = 0; i < E; ++i) {
+      atomicAdd(&acc[0][lane * E + i], dg[0][i]);
+      atomicAdd(&acc[1][lane * E + i], dg[1][i]);
     }
     __syncthreads();
     for (int i = threadIdx.x; i < D; i += blockDim.x) {
@@ -881,6 +882,85 @@ __global__ void muon_apply_kernel(float* const* __restrict__ masters, __nv_bfloa
   }
 }
 
+// ------------------------------------------------------------------ column sums (bias gradients)
+// part[y][n] = sum of x[r][n] over the y-th chunk of rows; block = 32 x 8 threads over a 256-column strip, a thread eight
+// columns. The chunks are added in order by colsum_finish_kernel, so the result does not depend on scheduling. One read of
+// x (T 27648, N 1024: 57 MB, 21 us; a cast to fp32 and a library reduction took 123 us).
+__global__ void __launch_bounds__(256)
+colsum_kernel(const __nv_bfloat16* __restrict__ x, float* __restrict__ part, long rows, int N, long ld, long chunk) {
+  __shared__ float red[8][32][9];
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  const int c = (blockIdx.x * 32 + tx) * 8;
+  const long r0 = blockIdx.y * chunk, r1 = min(rows, r0 + chunk);
+  float a[8];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) a[j] = 0.f;
+  if (c < N) {
+#pragma unroll 4
+    for (long r = r0 + ty; r < r1; r += 8) {
+      bf16x8 v;
+      v.v = *reinterpret_cast<const uint4*>(x + r * ld + c);
+      float f[8];
+      v.unpack(f);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) a[j] += f[j];
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < 8; ++j) red[ty][tx][j] = a[j];
+  __syncthreads();
+  const int col = blockIdx.x * 256 + threadIdx.x, l = threadIdx.x >> 3, j = threadIdx.x & 7;
+  if (col < N) {
+    float v = 0.f;
+#pragma unroll
+    for (int y = 0; y < 8; ++y) v += red[y][l][j];
+    part[(long)blockIdx.y * N + col] = v;
+  }
+}
+
+__global__ void __launch_bounds__(256)
+colsum_finish_kernel(const float* __restrict__ part, float* __restrict__ out, int N, int chunks) {
+  const int c = blockIdx.x * 256 + threadIdx.x;
+  if (c >= N) return;
+  float v = 0.f;
+#pragma unroll 8
+  for (int y = 0; y < chunks; ++y) v += part[(long)y * N + c];
+  out[c] = v;
+}
+
+// ------------------------------------------------------------------ Newton-Schulz elementwise steps (Muon)
+// out = a x + b y, bf16 in and out, fp32 inside, rounded once
+__global__ void __launch_bounds__(256)
+axpby_kernel(const uint4* __restrict__ x, const uint4* __restrict__ y, uint4* __restrict__ out, long n8, float a, float b) {
+  for (long i = blockIdx.x * 256L + threadIdx.x; i < n8; i += gridDim.x * 256L) {
+    bf16x8 u, w;
+    u.v = x[i];
+    w.v = y[i];
+    float f[8], g[8];
+    u.unpack(f);
+    w.unpack(g);
+#pragma unroll
+    for (int k = 0; k < 8; ++k) f[k] = fmaf(a, f[k], b * g[k]);
+    u.pack(f);
+    out[i] = u.v;
+  }
+}
+// out[b] = x[b] / div[b] (bf16 divisor, one per matrix)
+__global__ void __launch_bounds__(256)
+matrix_div_kernel(const uint4* __restrict__ x, const __nv_bfloat16* __restrict__ div, uint4* __restrict__ out, long per8) {
+  const float d = __bfloat162float(div[blockIdx.y]);
+  for (long i = blockIdx.x * 256L + threadIdx.x; i < per8; i += gridDim.x * 256L) {
+    bf16x8 u;
+    u.v = x[blockIdx.y * per8 + i];
+    float f[8];
+    u.unpack(f);
+#pragma unroll
+    for (int k = 0; k < 8; ++k) f[k] = __fdiv_rn(f[k], d);
+    u.pack(f);
+    out[blockIdx.y * per8 + i] = u.v;
+  }
+}
+
 static inline int grid_for(long work_items, int block) {
   long g = (work_items + block - 1) / block;
   const long cap = static_cast<long>(num_sms()) * 16;
@@ -964,7 +1044,11 @@ extern "C" int sb_qk_rope(const void* in, void* out, const void* pre, const floa
   SB_CHECK_ARG(T > 0 && S > 0 && ld % 4 == 0);
   const bool norm = q_gamma != nullptr;
   const long warps = static_cast<long>(T) * (Hq + Hkv);
-  const int blocks = static_cast<int>((warps + 7) / 8);
+  SB_CHECK_ARG(warps <= 0x7fffffffL - 8L * 32 * num_sms());
+  // One warp per item, except where the gain gradients leave: one block per eight items put 128 atomics on the same
+  // addresses for each (T 27648, 12 heads of 64: 211 us); eight blocks per SM walk their items: 71 us.
+  int blocks = static_cast<int>((warps + 7) / 8);
+  if (norm && backward && blocks > 8 * num_sms()) blocks = 8 * num_sms();
 #define SB_ROPE(DD, NN, BB)                                                                                          \
   qk_rope_kernel<DD, NN, BB><<<blocks, 256, 0, st>>>((const __nv_bfloat16*)in, (__nv_bfloat16*)out,                   \
                                                      (const __nv_bfloat16*)pre, q_gamma, k_gamma, rstd, dq_gamma,      \
@@ -1103,6 +1187,43 @@ extern "C" int sb_muon_apply(const void* masters, const void* params, const void
   if (bx > 512) bx = 512;
   muon_apply_kernel<<<dim3(bx, n), 256, 0, st>>>((float* const*)masters, (__nv_bfloat16* const*)params,
                                                  (const __nv_bfloat16*)upd, per, step);
+  SB_CHECK_CUDA(cudaGetLastError());
+  return SB_OK;
+}
+
+// out[N] fp32 = column sums of x `[rows, N]` bf16 (row stride ld, multiple of 8; N % 8 == 0, 16-byte aligned). part: fp32
+// scratch of sb_colsum_chunks(rows, N) * N.
+extern "C" int sb_colsum_chunks(long rows, int N) {
+  const int strips = (N + 255) / 256;
+  long want = 4L * sb::num_sms() / strips;
+  if (want > (rows + 63) / 64) want = (rows + 63) / 64;
+  return want < 1 ? 1 : (want > 1024 ? 1024 : (int)want);
+}
+
+extern "C" int sb_colsum(const void* x, float* part, float* out, long rows, int N, long ld, cudaStream_t st) {
+  SB_CHECK_ARG(rows > 0 && N > 0 && N % 8 == 0 && ld % 8 == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0);
+  const int chunks = sb_colsum_chunks(rows, N);
+  const long chunk = (rows + chunks - 1) / chunks;
+  colsum_kernel<<<dim3((N + 255) / 256, chunks), 256, 0, st>>>((const __nv_bfloat16*)x, part, rows, N, ld, chunk);
+  colsum_finish_kernel<<<(N + 255) / 256, 256, 0, st>>>(part, out, N, chunks);
+  SB_CHECK_CUDA(cudaGetLastError());
+  return SB_OK;
+}
+
+// out = a x + b y over n bf16 elements (n % 8 == 0, 16-byte aligned); out may be x or y
+extern "C" int sb_axpby(const void* x, const void* y, void* out, long n, float a, float b, cudaStream_t st) {
+  SB_CHECK_ARG(n > 0 && n % 8 == 0);
+  axpby_kernel<<<grid_for(n / 8, 256), 256, 0, st>>>((const uint4*)x, (const uint4*)y, (uint4*)out, n / 8, a, b);
+  SB_CHECK_CUDA(cudaGetLastError());
+  return SB_OK;
+}
+
+// out[b, :] = x[b, :] / div[b] over `batch` matrices of `per` bf16 elements (per % 8 == 0, 16-byte aligned)
+extern "C" int sb_matrix_div(const void* x, const void* div, void* out, int batch, long per, cudaStream_t st) {
+  SB_CHECK_ARG(batch > 0 && batch <= 65535 && per > 0 && per % 8 == 0);
+  long bx = (per / 8 + 255) / 256, cap = (16L * num_sms() + batch - 1) / batch;
+  if (bx > cap) bx = cap;
+  matrix_div_kernel<<<dim3((int)bx, batch), 256, 0, st>>>((const uint4*)x, (const __nv_bfloat16*)div, (uint4*)out, per / 8);
   SB_CHECK_CUDA(cudaGetLastError());
   return SB_OK;
 }

@@ -135,8 +135,39 @@ class _Linear(torch.autograd.Function):
                                out_dtype=BF16 if weight.dtype == BF16 else torch.float32)
                     dw = dwt.t()
         if bias is not None and ctx.needs_input_grad[2]:
-            db = dy2.float().sum(dim=0).to(bias.dtype)
+            db = column_sum(dy2).to(bias.dtype)
         return dx, dw, db
+
+
+N.register("sb_colsum_chunks", [N.L, N.I])
+N.register("sb_colsum", [N.P, N.P, N.P, N.L, N.I, N.L, N.P])
+N.register("sb_axpby", [N.P, N.P, N.P, N.L, N.F, N.F, N.P])
+N.register("sb_matrix_div", [N.P, N.P, N.P, N.I, N.L, N.P])
+
+
+def column_sum(x: torch.Tensor) -> torch.Tensor:
+    """fp32 sums over the rows of a 2-D tensor (bias gradients)."""
+    rows, Nn = x.shape
+    if x.dtype != BF16 or rows == 0 or Nn % 8 or x.stride(1) != 1 or x.stride(0) % 8 or x.data_ptr() % 16:
+        return x.float().sum(dim=0)
+    part = torch.empty(N.call_value("sb_colsum_chunks", rows, Nn), Nn, device=x.device, dtype=torch.float32)
+    out = torch.empty(Nn, device=x.device, dtype=torch.float32)
+    N.call("sb_colsum", x.data_ptr(), part.data_ptr(), out.data_ptr(), rows, Nn, x.stride(0), N.stream())
+    return out
+
+
+def axpby(a: float, x: torch.Tensor, b: float, y: torch.Tensor) -> torch.Tensor:
+    """a x + b y of contiguous bf16 tensors in one pass, rounded once; numel % 8 == 0."""
+    out = torch.empty_like(x)
+    N.call("sb_axpby", x.data_ptr(), y.data_ptr(), out.data_ptr(), x.numel(), float(a), float(b), N.stream())
+    return out
+
+
+def matrix_div(x: torch.Tensor, div: torch.Tensor) -> torch.Tensor:
+    """x[b] / div[b] for contiguous bf16 matrices `[B, R, C]` and a bf16 divisor per matrix; R * C % 8 == 0."""
+    out = torch.empty_like(x)
+    N.call("sb_matrix_div", x.data_ptr(), div.data_ptr(), out.data_ptr(), x.shape[0], x[0].numel(), N.stream())
+    return out
 
 
 def linear(x, weight, bias=None):

@@ -40,11 +40,20 @@ def newton_schulz(G: torch.Tensor, steps: int = NS_STEPS) -> torch.Tensor:
     a, b, c = NS_COEFFS
     X = G.to(torch.bfloat16) if G.is_cuda else G.float()
     tall = X.shape[1] > X.shape[2]
-    X = X / (torch.linalg.vector_norm(X, dim=(1, 2), keepdim=True, dtype=torch.float32).to(X.dtype) + 1e-7)
+    div = torch.linalg.vector_norm(X, dim=(1, 2), keepdim=True, dtype=torch.float32).to(X.dtype) + 1e-7
+    device = X.is_cuda and X.shape[1] % 8 == 0 and X.shape[2] % 8 == 0       # then the products keep whole 16-byte rows too
+    if device:
+        from ..ops import cuda_ops
+        X, mix = cuda_ops.matrix_div(X.contiguous(), div), cuda_ops.axpby
+    else:
+        X = X / div
+
+        def mix(p, x, q, y):
+            return torch.add(p * x, y, alpha=q)
     for _ in range(steps):
         A = _bmm(X, X, False, trans_a=True) if tall else _bmm(X, X, True)      # X^T X  or  X X^T
-        Bm = torch.add(b * A, _bmm(A, A, True), alpha=c)
-        X = torch.add(_bmm(X, Bm, False) if tall else _bmm(Bm, X, False), X, alpha=a)
+        Bm = mix(b, A, c, _bmm(A, A, True))
+        X = mix(a, X, 1.0, _bmm(X, Bm, False) if tall else _bmm(Bm, X, False))
     return X if X.is_cuda else X.float()          # bf16 on the device: that is what the update consumes
 
 

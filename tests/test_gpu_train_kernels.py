@@ -45,3 +45,57 @@ def test_adamw_vector_and_scalar_ranges(n, off, copy):
         torch.testing.assert_close(a.double(), b, rtol=2e-5, atol=2e-6)
     if copy:
         assert torch.equal(pb, p.to(torch.bfloat16))
+
+
+@gpu
+@pytest.mark.parametrize("rows,N,ld", [(1, 8, 8), (63, 264, 264), (65, 256, 512), (5000, 1024, 1024), (27648, 40, 48), (7, 2048, 2048)])
+def test_column_sum(rows, N, ld):
+    """fp32 sums of bf16 values, deterministic: at most `rows` roundings of 2^-24 of the terms' sum."""
+    from summa_b200.ops import cuda_ops
+    torch.manual_seed(rows)
+    x = torch.randn(rows, ld, device="cuda").to(torch.bfloat16)[:, :N]
+    got = cuda_ops.column_sum(x)
+    tol = rows * 2.0 ** -24 * x.double().abs().sum(0) + 1e-30
+    assert bool(((got.double() - x.double().sum(0)).abs() <= tol).all())
+    assert torch.equal(got, cuda_ops.column_sum(x))
+
+
+@gpu
+@pytest.mark.parametrize("shape", [(1, 8, 8), (3, 40, 24), (5, 64, 1032)])
+def test_newton_schulz_elementwise_steps(shape):
+    """One rounding to bf16 of the fp32 result each."""
+    from summa_b200.ops import cuda_ops
+    torch.manual_seed(shape[2])
+    x, y = torch.randn(shape, device="cuda").to(torch.bfloat16), torch.randn(shape, device="cuda").to(torch.bfloat16)
+    want = 3.4445 * x.double() - 4.775 * y.double()
+    assert bool(((cuda_ops.axpby(3.4445, x, -4.775, y).double() - want).abs()
+                 <= 2.0 ** -8 * want.abs() + 2.0 ** -22 * (3.4445 * x.double().abs() + 4.775 * y.double().abs())).all())
+    d = torch.rand(shape[0], 1, 1, device="cuda").to(torch.bfloat16) + 0.5
+    assert torch.equal(cuda_ops.matrix_div(x, d), x / d)
+
+
+@gpu
+@pytest.mark.parametrize("T,Hq,Hkv,D", [(1, 1, 1, 64), (9, 3, 1, 128), (12000, 8, 4, 64)])
+def test_qk_norm_rope_backward_gains(T, Hq, Hkv, D):
+    """Input and gain gradients with fewer and more (token, head) items than one round of the grid, against fp64 autograd
+    (bf16 rounding between norm and rotation and of the result: 2^-8 of a term each)."""
+    from summa_b200.ops import cuda_ops, reference
+    torch.manual_seed(T)
+    W = (Hq + 2 * Hkv) * D
+    qkv = torch.randn(1, T, W, device="cuda").to(torch.bfloat16).requires_grad_()
+    qg, kg = [(1 + 0.1 * torch.randn(D, device="cuda")).requires_grad_() for _ in range(2)]
+    cos, sin = reference.rope_table(T, D, 10000.0, None, "cuda")
+    dout = torch.randn(1, T, W, device="cuda").to(torch.bfloat16)
+    out = cuda_ops.qkv_rope(qkv, qg, kg, 1e-5, cos, sin, Hq, Hkv, D)
+    out.backward(dout)
+    x = qkv.detach().double().requires_grad_()
+    g64 = [g.detach().double().requires_grad_() for g in (qg, kg)]
+    v = x.view(T, Hq + 2 * Hkv, D)
+    n = v[:, :Hq + Hkv] * torch.rsqrt(v[:, :Hq + Hkv].pow(2).mean(-1, keepdim=True) + 1e-5)
+    n = torch.cat([n[:, :Hq] * g64[0], n[:, Hq:] * g64[1]], 1)
+    c, s = cos.double().view(T, 1, D // 2), sin.double().view(T, 1, D // 2)
+    a, b = n[..., 0::2], n[..., 1::2]
+    r = torch.stack([a * c - b * s, a * s + b * c], -1).flatten(-2)
+    torch.cat([r, v[:, Hq + Hkv:]], 1).view(1, T, W).backward(dout.double())
+    for got, want in ((qkv.grad, x.grad), (qg.grad, g64[0].grad), (kg.grad, g64[1].grad)):
+        assert float((got.double() - want).norm() / want.norm()) <= 2.0 ** -7
