@@ -194,10 +194,9 @@ class MambaMixer(nn.Module):
         proj = self.x_proj(xc)
         dt_in, Bm, Cm = proj.split([self.dt_rank, self.d_state, self.d_state], dim=-1)
         delta = self.dt_proj(dt_in)
-        A = -torch.exp(self.a_log.float())
         h0 = state.h if state is not None else None
-        y, h_last = ops.selective_scan(xc, delta, A, Bm, Cm, self.d, h0,
-                                       need_final_state=state is not None)
+        y, h_last = ops.selective_scan_log(xc, delta, self.a_log, Bm, Cm, self.d, h0,
+                                           need_final_state=state is not None)
         if state is not None:
             state.conv = new_conv
             state.h = h_last
@@ -294,13 +293,13 @@ class SparseMoe(nn.Module):
         self.moe = _Moe(ffn, hidden, init_std)
         self.ep = None      # set by parallel.ep.shard_experts
 
-    def forward(self, x: torch.Tensor, extra_random_expert_seed: Optional[int] = None):
+    def forward(self, x: torch.Tensor, extra_random_expert_seed: Optional[int] = None, need_aux: bool = True):
         shape = x.shape
         flat = x.reshape(-1, shape[-1])
         logits = ops.router_logits(flat, self.moe.router.weight)
         idx, gates = ops.moe_route(logits, self.cfg.top_k)
         aux = ops.moe_aux_loss(logits, idx, self.cfg.experts, self.cfg.load_balance_loss_weight,
-                               self.cfg.router_z_loss_weight)
+                               self.cfg.router_z_loss_weight) if need_aux else None
         if extra_random_expert_seed is not None:
             idx, gates = _dream_routes(logits, idx, self.cfg.experts, extra_random_expert_seed)
         e = self.moe.experts

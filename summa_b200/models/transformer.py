@@ -135,7 +135,7 @@ class TransformerBlock(nn.Module):
                 and self.ffn_norm.kind == "rmsnorm" and not (self.dropout > 0.0 and self.training))
 
     def forward_deferred(self, x: torch.Tensor, pending: Optional[torch.Tensor], rope, state=None,
-                         dream_seed: Optional[int] = None):
+                         dream_seed: Optional[int] = None, need_aux: bool = True):
         """Same block with the residual adds fused into the following norm (`norm(x + y)` and
         `x + y` come out of one kernel). `pending` is the previous block's branch output that has
         not been added to `x` yet; returns (x, pending, aux) in the same convention."""
@@ -147,7 +147,7 @@ class TransformerBlock(nn.Module):
         n, x = self.ffn_norm(mix.to(x.dtype), x)
         aux = None
         if isinstance(self.feed_forward, SparseMoe):
-            y, aux = self.feed_forward(n, dream_seed)
+            y, aux = self.feed_forward(n, dream_seed, need_aux)
         else:
             y = self.feed_forward(n)
         return x, y, aux
@@ -278,9 +278,9 @@ class Transformer(nn.Module):
 
     # ------------------------------------------------------------------ stateless
     def forward_hidden(self, tokens: torch.Tensor, through_layer: Optional[int] = None,
-                       dream_seed: Optional[int] = None, final_norm: bool = True):
+                       dream_seed: Optional[int] = None, final_norm: bool = True, need_aux: bool = True):
         """Hidden states after `through_layer` blocks (all when None) and the summed
-        router auxiliary loss."""
+        router auxiliary loss (`need_aux=False`: the caller has no use for it)."""
         x = self.embed(tokens)
         rope = self.rope(tokens.device)
         aux_total = None
@@ -293,7 +293,7 @@ class Transformer(nn.Module):
             if hook is not None and hook.armed and x.requires_grad:
                 x = _GradReady.apply(x, hook, i)
             if fused:
-                x, pending, aux = self.layers[i].forward_deferred(x, pending, rope, None, seed)
+                x, pending, aux = self.layers[i].forward_deferred(x, pending, rope, None, seed, need_aux)
             else:
                 x, aux = self.layers[i](x, rope, None, seed)
             if aux is not None:
@@ -369,7 +369,7 @@ class Transformer(nn.Module):
                            layer: Optional[int] = None) -> torch.Tensor:
         """L2-normalised final-norm(hidden at end_positions) from 1-based `layer`
         (all layers when None), in fp32 (`transformer.rs:835-851`)."""
-        x, _ = self.forward_hidden(tokens, through_layer=layer)
+        x, _ = self.forward_hidden(tokens, through_layer=layer, need_aux=False)
         B = tokens.shape[0]
         sel = x[torch.arange(B, device=x.device), end_positions].float()
         return sel / sel.norm(dim=-1, keepdim=True).clamp_min(1e-12)

@@ -170,6 +170,13 @@ def selective_scan(u, delta, A, Bm, Cm, D, h0=None, need_final_state=False):
     return reference.selective_scan(u, delta, A, Bm, Cm, D, h0)
 
 
+def selective_scan_log(u, delta, a_log, Bm, Cm, D, h0=None, need_final_state=False):
+    """`selective_scan` with A = -exp(a_log)."""
+    if native_enabled(u) and not torch.is_grad_enabled():
+        return _cu().selective_scan_log(u, delta, a_log, Bm, Cm, D, h0, need_final_state)
+    return selective_scan(u, delta, -torch.exp(a_log.float()), Bm, Cm, D, h0, need_final_state)
+
+
 def mul_silu(y, z):
     """y * silu(z), fp32 math."""
     if native_enabled(y):

@@ -27,9 +27,10 @@ __device__ __forceinline__ float silu_f(float x) { return x / (1.f + __expf(-x))
 // A thread's 8 K weights and its K - 1 leading inputs are paid once per TT steps: 32 steps where there are enough of them to
 // fill the GPU (B 2 T 8192 C 3072: 142 -> 64 us of 30 us of traffic), 8 otherwise.
 template <int K, bool SILU, int TT>
-__global__ void __launch_bounds__(128, 4) conv1d_fwd_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict__ w,
+__global__ void __launch_bounds__(128, 4) conv1d_fwd_kernel(const __nv_bfloat16* __restrict__ x, const void* __restrict__ taps,
                                   const float* __restrict__ bias, const __nv_bfloat16* __restrict__ state,
                                   __nv_bfloat16* __restrict__ y, int B, int T, int C, long ldx, int w16) {
+  const float* w = static_cast<const float*>(taps);          // w16: 0 fp32, 1 fp32 on 16 bytes, 2 bf16
   const int c8 = C / 8;
   const long idx = blockIdx.x * (long)blockDim.x + threadIdx.x;
   const int tchunks = (T + TT - 1) / TT;
@@ -42,7 +43,10 @@ __global__ void __launch_bounds__(128, 4) conv1d_fwd_kernel(const __nv_bfloat16*
 #pragma unroll
   for (int j = 0; j < 8; ++j) {
     bs[j] = bias ? bias[c0 + j] : 0.f;
-    if (K == 4 && w16) {
+    if (w16 == 2) {
+#pragma unroll
+      for (int k = 0; k < K; ++k) wk[k][j] = __bfloat162float(static_cast<const __nv_bfloat16*>(taps)[(c0 + j) * K + k]);
+    } else if (K == 4 && w16) {
       const float4 q = *reinterpret_cast<const float4*>(w + (long)(c0 + j) * K);
       wk[0][j] = q.x; wk[1 % K][j] = q.y; wk[2 % K][j] = q.z; wk[3 % K][j] = q.w;
     } else {
@@ -115,6 +119,7 @@ struct ScanFwdParams {
   int B, T, C;
   long ld_u, ld_d, ld_b, ld_c;
   int vec;                     // every row of u / delta / B / C starts 16-byte aligned
+  int a_is_log;                // A holds a_log: the decay rate is -exp(a_log)
 };
 
 // Thread = one channel x NPT consecutive states, carried in registers as f32x2 pairs for the whole sequence.
@@ -151,9 +156,13 @@ selective_scan_fwd_kernel(const ScanFwdParams p) {
   uint64_t A2[NP], h[NP];
 #pragma unroll
   for (int j = 0; j < NP; ++j) {
-    const float a0 = c_ok ? p.A[(long)c * N + n0 + 2 * j] * 1.4426950408889634f : 0.f;
-    const float a1 = c_ok ? p.A[(long)c * N + n0 + 2 * j + 1] * 1.4426950408889634f : 0.f;
-    A2[j] = f2_pack(a0, a1);
+    float a0 = c_ok ? p.A[(long)c * N + n0 + 2 * j] : 0.f;
+    float a1 = c_ok ? p.A[(long)c * N + n0 + 2 * j + 1] : 0.f;
+    if (p.a_is_log) {          // (once per thread and launch; in 64 bits, so that A is as exact as a library exponential)
+      a0 = -static_cast<float>(exp(static_cast<double>(a0)));
+      a1 = -static_cast<float>(exp(static_cast<double>(a1)));
+    }
+    A2[j] = f2_pack(a0 * 1.4426950408889634f, a1 * 1.4426950408889634f);
     const float h0a = (c_ok && p.h0) ? p.h0[((long)b * p.C + c) * N + n0 + 2 * j] : 0.f;
     const float h0b = (c_ok && p.h0) ? p.h0[((long)b * p.C + c) * N + n0 + 2 * j + 1] : 0.f;
     h[j] = f2_pack(h0a, h0b);
@@ -263,10 +272,10 @@ static int launch_scan_fwd(const ScanFwdParams& p, cudaStream_t st) {
 using namespace sb;
 
 // y = [silu](causal depthwise conv(x) + bias). K in 2..4. C % 8 == 0, ldx % 8 == 0.
-extern "C" int sb_conv1d_fwd(const void* x, const float* w, const float* bias, const void* state, void* y, int B, int T,
-                             int C, int K, long ldx, int silu, cudaStream_t st) {
+static int conv1d_fwd(int w_is_bf16, const void* x, const void* w, const float* bias, const void* state, void* y, int B, int T,
+                      int C, int K, long ldx, int silu, cudaStream_t st) {
   SB_CHECK_ARG(B > 0 && T > 0 && C % 8 == 0 && ldx % 8 == 0 && K >= 2 && K <= 4);
-  const int w16 = (reinterpret_cast<uintptr_t>(w) & 15) == 0;      // K = 4: a channel's taps in one load
+  const int w16 = w_is_bf16 ? 2 : ((reinterpret_cast<uintptr_t>(w) & 15) == 0 ? 1 : 0);      // K = 4: a channel's taps in one load
   const long long_items = (long)B * ((T + 31) / 32) * (C / 8), short_items = (long)B * ((T + 7) / 8) * (C / 8);
   const bool many = long_items >= 512L * num_sms();
   const int blocks = (int)(((many ? long_items : short_items) + 127) / 128);
@@ -281,6 +290,17 @@ extern "C" int sb_conv1d_fwd(const void* x, const float* w, const float* bias, c
 #undef SB_CONV_ARGS
   SB_CHECK_CUDA(cudaGetLastError());
   return SB_OK;
+}
+
+extern "C" int sb_conv1d_fwd(const void* x, const float* w, const float* bias, const void* state, void* y, int B, int T,
+                             int C, int K, long ldx, int silu, cudaStream_t st) {
+  return conv1d_fwd(0, x, w, bias, state, y, B, T, C, K, ldx, silu, st);
+}
+
+// The same with bf16 taps.
+extern "C" int sb_conv1d_fwd_bf16w(const void* x, const void* w, const float* bias, const void* state, void* y, int B, int T,
+                                   int C, int K, long ldx, int silu, cudaStream_t st) {
+  return conv1d_fwd(1, x, w, bias, state, y, B, T, C, K, ldx, silu, st);
 }
 
 // ---------------------------------------------------------------------------- single-token decode step
@@ -404,15 +424,15 @@ extern "C" int sb_scan_ckpt_interval() { return SCAN_SEG; }
 
 // Selective scan forward. N in {8,16,32,64,128,256}, C even. ckpt `[B, ceil(T / sb_scan_ckpt_interval()), C, N]` fp32 is
 // written when non-null (training); h_out `[B,C,N]` receives the final state when non-null.
-extern "C" int sb_scan_fwd(const void* u, const void* delta, const float* A, const void* Bm, const void* Cm,
-                           const float* D, const float* h0, void* y, float* ckpt, float* h_out, int B, int T, int C,
-                           int N, long ld_u, long ld_d, long ld_b, long ld_c, cudaStream_t st) {
+static int scan_fwd(int a_is_log, const void* u, const void* delta, const float* A, const void* Bm, const void* Cm,
+                    const float* D, const float* h0, void* y, float* ckpt, float* h_out, int B, int T, int C,
+                    int N, long ld_u, long ld_d, long ld_b, long ld_c, cudaStream_t st) {
   SB_CHECK_ARG(B > 0 && T > 0 && C > 0 && C % 2 == 0);
   ScanFwdParams p;
   p.u = (const __nv_bfloat16*)u; p.delta = (const __nv_bfloat16*)delta; p.A = A;
   p.Bm = (const __nv_bfloat16*)Bm; p.Cm = (const __nv_bfloat16*)Cm; p.D = D; p.h0 = h0;
   p.y = (__nv_bfloat16*)y; p.ckpt = ckpt; p.h_out = h_out;
-  p.B = B; p.T = T; p.C = C; p.ld_u = ld_u; p.ld_d = ld_d; p.ld_b = ld_b; p.ld_c = ld_c;
+  p.B = B; p.T = T; p.C = C; p.ld_u = ld_u; p.ld_d = ld_d; p.ld_b = ld_b; p.ld_c = ld_c; p.a_is_log = a_is_log;
   p.vec = C % 8 == 0 && ld_u % 8 == 0 && ld_d % 8 == 0 && ld_b % 8 == 0 && ld_c % 8 == 0 &&
           (((uintptr_t)u | (uintptr_t)delta | (uintptr_t)Bm | (uintptr_t)Cm) & 15) == 0;
   // States per thread and channels per block. The sequence is serial, so the warps in flight are B C N / (32 states per
@@ -431,4 +451,17 @@ extern "C" int sb_scan_fwd(const void* u, const void* delta, const float* A, con
       fprintf(stderr, "summa_b200: selective scan supports d_state in {8,16,32,64,128,256}, got %d\n", N);
       return SB_ERR_ARG;
   }
+}
+
+extern "C" int sb_scan_fwd(const void* u, const void* delta, const float* A, const void* Bm, const void* Cm,
+                           const float* D, const float* h0, void* y, float* ckpt, float* h_out, int B, int T, int C,
+                           int N, long ld_u, long ld_d, long ld_b, long ld_c, cudaStream_t st) {
+  return scan_fwd(0, u, delta, A, Bm, Cm, D, h0, y, ckpt, h_out, B, T, C, N, ld_u, ld_d, ld_b, ld_c, st);
+}
+
+// The same with a_log in the place of A = -exp(a_log).
+extern "C" int sb_scan_fwd_log(const void* u, const void* delta, const float* a_log, const void* Bm, const void* Cm,
+                               const float* D, const float* h0, void* y, float* ckpt, float* h_out, int B, int T, int C,
+                               int N, long ld_u, long ld_d, long ld_b, long ld_c, cudaStream_t st) {
+  return scan_fwd(1, u, delta, a_log, Bm, Cm, D, h0, y, ckpt, h_out, B, T, C, N, ld_u, ld_d, ld_b, ld_c, st);
 }

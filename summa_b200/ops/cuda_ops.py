@@ -700,6 +700,8 @@ def linear_cross_entropy(hidden, weight, bias, targets, vocab_size, chunks=4):
 N.register("sb_conv1d_fwd", [N.P, N.P, N.P, N.P, N.P, N.I, N.I, N.I, N.I, N.L, N.I, N.P])
 N.register("sb_conv1d_bwd", [N.P, N.P, N.P, N.P, N.P, N.P, N.P, N.I, N.I, N.I, N.I, N.L, N.L, N.I, N.P])
 N.register("sb_scan_fwd", [N.P] * 10 + [N.I] * 4 + [N.L] * 4 + [N.P])
+N.register("sb_scan_fwd_log", [N.P] * 10 + [N.I] * 4 + [N.L] * 4 + [N.P])
+N.register("sb_conv1d_fwd_bf16w", [N.P, N.P, N.P, N.P, N.P, N.I, N.I, N.I, N.I, N.L, N.I, N.P])
 N.register("sb_scan_bwd", [N.P] * 20 + [N.I] * 4 + [N.L] * 7 + [N.P])
 N.register("sb_scan_ckpt_interval", [])
 
@@ -721,11 +723,12 @@ class _Conv1dSilu(torch.autograd.Function):
         B, T, C = x.shape
         K = weight.shape[-1]
         xs, ldx = _btc(x)
-        w32 = weight.reshape(C, K).float().contiguous()
+        w16 = weight.dtype == BF16 and weight.is_contiguous()      # the kernel widens bf16 taps itself
+        w32 = weight if w16 else weight.reshape(C, K).float().contiguous()
         b32 = bias.float().contiguous() if bias is not None else None
         y = torch.empty(B, T, C, device=x.device, dtype=BF16)
         st = state.to(BF16).contiguous() if state is not None else None
-        N.call("sb_conv1d_fwd", xs.data_ptr(), w32.data_ptr(), N.ptr(b32), N.ptr(st), y.data_ptr(), B, T, C, K, ldx,
+        N.call("sb_conv1d_fwd_bf16w" if w16 else "sb_conv1d_fwd", xs.data_ptr(), w32.data_ptr(), N.ptr(b32), N.ptr(st), y.data_ptr(), B, T, C, K, ldx,
                1, N.stream())
         ctx.save_for_backward(x, weight, bias)
         ctx.has_state = state is not None
@@ -814,6 +817,25 @@ class _SelectiveScan(torch.autograd.Function):
         return du, dd, dA.to(A.dtype), dBm, dCm, dD.to(D.dtype), None, None
 
 
+def selective_scan_log(u, delta, a_log, Bm, Cm, D, h0=None, need_final_state=False):
+    """`selective_scan` with A = -exp(a_log) formed inside the kernel; no gradients."""
+    B, T, C = u.shape
+    Ns = a_log.shape[1]
+    if Ns not in _SCAN_STATES or C % 2:
+        return reference.selective_scan(u, delta, -torch.exp(a_log.float()), Bm, Cm, D, h0)
+    us, ld_u = _btc(u)
+    ds, ld_d = _btc(delta)
+    bs, ld_b = _btc(Bm)
+    cs, ld_c = _btc(Cm)
+    A32, D32 = a_log.detach().float().contiguous(), D.detach().float().contiguous()
+    y = torch.empty(B, T, C, device=u.device, dtype=BF16)
+    h_out = torch.empty(B, C, Ns, device=u.device, dtype=torch.float32) if need_final_state else None
+    h0c = h0.float().contiguous() if h0 is not None else None
+    N.call("sb_scan_fwd_log", us.data_ptr(), ds.data_ptr(), A32.data_ptr(), bs.data_ptr(), cs.data_ptr(), D32.data_ptr(),
+           N.ptr(h0c), y.data_ptr(), None, N.ptr(h_out), B, T, C, Ns, ld_u, ld_d, ld_b, ld_c, N.stream())
+    return y, h_out
+
+
 def selective_scan(u, delta, A, Bm, Cm, D, h0=None, need_final_state=False):
     if A.shape[1] not in _SCAN_STATES or u.shape[-1] % 2:
         return reference.selective_scan(u, delta, A, Bm, Cm, D, h0)
@@ -857,6 +879,8 @@ def mamba_decode_step(mixer, xz, conv, h):
 
 N.register("sb_router_logits", [N.P, N.P, N.P, N.I, N.I, N.I, N.L, N.P])
 N.register("sb_moe_plan", [N.P] * 7 + [N.I] * 4 + [N.P])
+N.register("sb_moe_plan_gates", [N.P] * 9 + [N.I] * 4 + [N.P])
+N.register("sb_moe_gates_bwd", [N.P] * 4 + [N.I] * 3 + [N.P])
 N.register("sb_moe_gather", [N.P, N.P, N.P, N.P, N.I, N.I, N.I, N.L, N.I, N.P])
 N.register("sb_moe_combine", [N.P, N.P, N.P, N.P, N.I, N.I, N.I, N.P])
 N.register("sb_moe_combine_bwd", [N.P] * 7 + [N.I] * 4 + [N.P])
@@ -911,7 +935,7 @@ def router_logits(x, w):
 class RoutePlan:
     """Device-resident routing plan of one MoE layer call (no host synchronisation)."""
 
-    def __init__(self, logits: torch.Tensor, k: int):
+    def __init__(self, logits: torch.Tensor, k: int, gates: Optional[torch.Tensor] = None, idx64: Optional[torch.Tensor] = None):
         T, E = logits.shape
         dev = logits.device
         self.T, self.E, self.k = T, E, k
@@ -923,9 +947,9 @@ class RoutePlan:
         self.dest = torch.empty(T * k, device=dev, dtype=torch.int32)
         self.row_route = torch.empty(self.max_rows, device=dev, dtype=torch.int32)
         lg = logits.detach().float().contiguous()
-        N.call("sb_moe_plan", lg.data_ptr(), self.idx.data_ptr(), self.counts.data_ptr(), self.meta.data_ptr(),
-               self.tile_expert.data_ptr(), self.dest.data_ptr(), self.row_route.data_ptr(), T, E, k, self.max_rows,
-               N.stream())
+        N.call("sb_moe_plan_gates", lg.data_ptr(), self.idx.data_ptr(), self.counts.data_ptr(), self.meta.data_ptr(),
+               self.tile_expert.data_ptr(), self.dest.data_ptr(), self.row_route.data_ptr(), N.ptr(gates), N.ptr(idx64), T, E, k,
+               self.max_rows, N.stream())
 
     @property
     def num_m_tiles_ptr(self) -> int:
@@ -976,14 +1000,46 @@ def moe_aux_loss(logits, idx, num_experts, lb_weight, z_weight):
     return _MoeAuxLoss.apply(logits, counts, idx.shape[1], max(lb_weight, 0.0), max(z_weight, 0.0))
 
 
+class _MoeRoute(torch.autograd.Function):
+    """Top-k routing: int64 indices, the softmax over the selected logits and the device plan of one launch sequence; the
+    backward writes the full row of logit gradients in one launch."""
+
+    @staticmethod
+    def forward(ctx, logits, k, out):
+        T, E = logits.shape
+        gates = torch.empty(T, k, device=logits.device, dtype=torch.float32)
+        idx = torch.empty(T, k, device=logits.device, dtype=torch.int64)
+        out.append(RoutePlan(logits, k, gates, idx))
+        ctx.save_for_backward(out[0].idx, gates, logits)
+        ctx.meta = (T, E, k, logits.dtype)
+        ctx.mark_non_differentiable(idx)
+        return idx, gates
+
+    @staticmethod
+    def backward(ctx, _, dg):
+        idx, gates, logits = ctx.saved_tensors
+        T, E, k, dtype = ctx.meta
+        if torch.is_grad_enabled():                  # a second derivative is wanted: the same in differentiable ops
+            g = torch.softmax(torch.gather(logits.float(), 1, idx.long()), dim=-1)
+            d = g * (dg - (g * dg).sum(-1, keepdim=True))
+            return torch.zeros(T, E, device=d.device, dtype=d.dtype).scatter(1, idx.long(), d).to(dtype), None, None
+        dl = torch.empty(T, E, device=gates.device, dtype=torch.float32)
+        d = dg.float().contiguous()
+        N.call("sb_moe_gates_bwd", idx.data_ptr(), gates.data_ptr(), d.data_ptr(), dl.data_ptr(), T, E, k, N.stream())
+        return dl.to(dtype), None, None
+
+
 def moe_route(logits, top_k):
-    """(indices [T,k] int64, gates [T,k] fp32 = softmax over the selected logits). The
-    selection runs in the top-k kernel; the gate softmax is differentiable torch math on
-    the tiny `[T, k]` gather."""
-    plan = RoutePlan(logits, top_k)
-    idx = plan.idx.long()
-    gates = torch.softmax(torch.gather(logits.float(), 1, idx), dim=-1)
-    idx._sb_plan = plan
+    """(indices [T,k] int64, gates [T,k] fp32 = softmax over the selected logits, differentiable)."""
+    if torch.autograd.forward_ad._current_level >= 0:        # forward-mode derivatives: differentiable ops for the gates
+        plan = RoutePlan(logits, top_k)
+        idx = plan.idx.long()
+        gates = torch.softmax(torch.gather(logits.float(), 1, idx), dim=-1)
+        idx._sb_plan = plan
+        return idx, gates
+    plan = []
+    idx, gates = _MoeRoute.apply(logits, top_k, plan)
+    idx._sb_plan = plan[0]
     return idx, gates
 
 

@@ -99,3 +99,59 @@ def test_qk_norm_rope_backward_gains(T, Hq, Hkv, D):
     torch.cat([r, v[:, Hq + Hkv:]], 1).view(1, T, W).backward(dout.double())
     for got, want in ((qkv.grad, x.grad), (qg.grad, g64[0].grad), (kg.grad, g64[1].grad)):
         assert float((got.double() - want).norm() / want.norm()) <= 2.0 ** -7
+
+
+@gpu
+@pytest.mark.parametrize("T,E,k", [(1, 2, 1), (5, 8, 2), (300, 33, 8), (2049, 64, 4), (2100, 256, 3)])
+def test_moe_route_gates_and_plan(T, E, k):
+    """Indices, gates and their gradient against the torch ops they stand for (fp32 rounding of 64-bit results), the packed
+    plan against a stable sort, with fewer and more routes than a round of the packing block; also a second derivative."""
+    from summa_b200 import ops
+    torch.manual_seed(T + E)
+    logits = torch.randn(T, E, device="cuda").requires_grad_()
+    idx, gates = ops.moe_route(logits, k)
+    val, want = logits.detach().topk(k, dim=-1)
+    assert torch.equal(logits.detach().gather(1, idx), val) and idx.dtype == torch.int64
+    ref = logits.detach().double().requires_grad_()
+    rg = torch.softmax(ref.gather(1, idx), -1)
+    torch.testing.assert_close(gates.double(), rg, rtol=2.0 ** -23, atol=1e-30)
+    dg = torch.randn_like(gates)
+    (d1,) = torch.autograd.grad(gates, logits, dg, retain_graph=True)
+    (r1,) = torch.autograd.grad(rg, ref, dg.double(), retain_graph=True)
+    torch.testing.assert_close(d1.double(), r1, rtol=1e-5, atol=1e-6)
+    (d2,) = torch.autograd.grad((torch.autograd.grad(gates, logits, dg, create_graph=True)[0] ** 2).sum(), logits)
+    (r2,) = torch.autograd.grad((torch.autograd.grad(rg, ref, dg.double(), create_graph=True)[0] ** 2).sum(), ref)
+    torch.testing.assert_close(d2.double(), r2, rtol=1e-4, atol=1e-5)
+    plan = idx._sb_plan
+    flat, meta = idx.view(-1).cpu(), plan.meta.cpu()
+    counts = torch.bincount(flat, minlength=E)
+    assert torch.equal(plan.counts.cpu().long(), counts)
+    row_route, dest = plan.row_route.cpu(), plan.dest.cpu()
+    for e in range(E):
+        lo, hi, n = int(meta[e]), int(meta[e + 1]), int(counts[e])
+        routes = (flat == e).nonzero().view(-1)
+        assert hi - lo == -(-n // 128) * 128
+        assert torch.equal(row_route[lo:lo + n].long(), routes) and bool((row_route[lo + n:hi] == -1).all())
+        assert torch.equal(dest[routes].long(), torch.arange(lo, lo + n))
+
+
+@gpu
+def test_scan_and_convolution_inference_forms():
+    """a_log and bf16 taps inside the kernels against the same kernels on prepared operands."""
+    from summa_b200 import ops
+    from summa_b200.ops import cuda_ops
+    torch.manual_seed(0)
+    for B, T, C, Ns in ((2, 37, 64, 16), (1, 5, 96, 128)):
+        u, d, Bm, Cm = [torch.randn(*s, device="cuda").to(torch.bfloat16) for s in ((B, T, C), (B, T, C), (B, T, Ns), (B, T, Ns))]
+        a_log, D = torch.rand(C, Ns, device="cuda") * 3 - 1, torch.randn(C, device="cuda")
+        h0 = torch.randn(B, C, Ns, device="cuda")
+        with torch.no_grad():
+            y, h = ops.selective_scan_log(u, d, a_log, Bm, Cm, D, h0, True)
+            yr, hr = cuda_ops.selective_scan(u, d, -torch.exp(a_log), Bm, Cm, D, h0, True)
+        torch.testing.assert_close(h, hr, rtol=1e-5, atol=1e-5)
+        torch.testing.assert_close(y.float(), yr.float(), rtol=2.0 ** -7, atol=2.0 ** -7)
+        for K in (2, 3, 4):
+            w, b = torch.randn(C, 1, K, device="cuda").to(torch.bfloat16), torch.randn(C, device="cuda")
+            assert torch.equal(cuda_ops.conv1d_silu(u, w, b), cuda_ops.conv1d_silu(u, w.float(), b))
+            v = torch.empty(C * K + 1, device="cuda")[1:].view(C, 1, K).copy_(w.float())      # taps that are not 16-byte aligned
+            assert torch.equal(cuda_ops.conv1d_silu(u, v, b), cuda_ops.conv1d_silu(u, w.float(), b))
