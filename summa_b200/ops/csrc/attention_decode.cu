@@ -27,14 +27,18 @@ constexpr int DEC_D = 128;
 constexpr int DEC_N = 8;                           // padded query heads per kv head
 constexpr int DEC_THREADS = 192;
 constexpr int DEC_TILE = 128 * DEC_D * 2;          // 32 KB
-constexpr int DEC_NS = 3;
 constexpr int DEC_OFF_K = 0;
-constexpr int DEC_OFF_V = DEC_NS * DEC_TILE;
-constexpr int DEC_OFF_Q = 2 * DEC_NS * DEC_TILE;   // 8 rows x 256 B (two swizzle atoms)
-constexpr int DEC_OFF_P = DEC_OFF_Q + 2048;        // 2 buffers x 2 KB
-constexpr int DEC_OFF_RED = DEC_OFF_P + 4096;      // [2][4 warps][8] floats
-constexpr int DEC_OFF_BAR = DEC_OFF_RED + 256;
-constexpr int DEC_SMEM = DEC_OFF_BAR + 256 + 1024;
+// K/V ring stages: 3 for few (batch, kv head) pairs, where one CTA per SM has to keep HBM busy by itself; 1 when there are
+// more pairs than SMs, where three CTAs per SM hide each other's loads and softmax steps instead (64 sequences x 8 kv heads,
+// 150 cached tokens: 22.8 us and a merge of 3.4 with 3 stages and 3.5 rounds of CTAs, 17.4 with 1).
+template <int NS> struct DecLayout {
+  static constexpr int OFF_V = NS * DEC_TILE;
+  static constexpr int OFF_Q = 2 * NS * DEC_TILE;    // 8 rows x 256 B (two swizzle atoms)
+  static constexpr int OFF_P = OFF_Q + 2048;         // 2 buffers x 2 KB
+  static constexpr int OFF_RED = OFF_P + 4096;       // [2][4 warps][8] floats
+  static constexpr int OFF_BAR = OFF_RED + 256;
+  static constexpr int SMEM = OFF_BAR + 256 + 1024;
+};
 
 struct DecParams {
   int B, Hq, Hkv, Sk, splits, blocks_per_split;
@@ -46,12 +50,18 @@ struct DecParams {
   float* part_o;              // [B, Hkv, splits, 8, D]
   float* part_m;              // [B, Hkv, splits, 8]  (log2 domain)
   float* part_l;              // [B, Hkv, splits, 8]
+  __nv_bfloat16* o;           // one split: the normalised output goes straight here, strides o_sb / o_sh
+  long o_sb, o_sh;
   unsigned int* err;
 };
 
-__global__ void __launch_bounds__(DEC_THREADS, 1)
+template <int NS>
+__global__ void __launch_bounds__(DEC_THREADS, NS == 1 ? 3 : 1)
 attention_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV, const DecParams p) {
+  constexpr int DEC_NS = NS, DEC_OFF_V = DecLayout<NS>::OFF_V, DEC_OFF_Q = DecLayout<NS>::OFF_Q, DEC_OFF_P = DecLayout<NS>::OFF_P;
+  constexpr int DEC_OFF_RED = DecLayout<NS>::OFF_RED, DEC_OFF_BAR = DecLayout<NS>::OFF_BAR;
   extern __shared__ uint8_t smem_raw[];
+  if (p.o != nullptr) asm volatile("griddepcontrol.launch_dependents;");   // (the merge kernel's signal otherwise)
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + DEC_OFF_BAR);
   uint64_t* kv_full = bars + 0;    // [3]
@@ -128,7 +138,7 @@ attention_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_co
       bool ok = mbar_wait(&kv_full[0], 0, abort_flag, p.err);
       if (ok) { tc_fence_after(); issue_s(0); }
       for (int i = 0; i < nblk && ok; ++i) {
-        if (i + 1 < nblk) {
+        if (NS > 1 && i + 1 < nblk) {
           // S^T buffer (i+1)&1 was read by the threads in block i-1, before their p_full(i-1)
           if (!mbar_wait(&kv_full[(i + 1) % DEC_NS], ((i + 1) / DEC_NS) & 1, abort_flag, p.err)) { ok = false; break; }
           tc_fence_after();
@@ -145,6 +155,11 @@ attention_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_co
         }
         umma_commit(&kv_empty[s]);
         umma_commit(o_done);
+        if (NS == 1 && i + 1 < nblk) {               // one stage: the next block is loaded once this one is consumed
+          if (!mbar_wait(&kv_full[0], (i + 1) & 1, abort_flag, p.err)) { ok = false; break; }
+          tc_fence_after();
+          issue_s(i + 1);
+        }
       }
     }
     __syncwarp();
@@ -226,7 +241,7 @@ attention_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_co
     }
     asm volatile("bar.sync 1, 128;" ::: "memory");
     const size_t pbase = ((static_cast<size_t>(b) * p.Hkv + kv_head) * p.splits + split) * DEC_N;
-    if (t < DEC_N) {
+    if (p.o == nullptr && t < DEC_N) {
       p.part_l[pbase + t] = red[t] + red[8 + t] + red[16 + t] + red[24 + t];
       float mr = -INFINITY;
 #pragma unroll
@@ -240,8 +255,17 @@ attention_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_co
       tmem_ld_32x32b_x8(tmem_base + COL_O + lane_sel, o16);
       tmem_ld_wait();
     }
+    if (p.o != nullptr) {
 #pragma unroll
-    for (int g = 0; g < DEC_N; ++g) p.part_o[(pbase + g) * DEC_D + t] = have ? __uint_as_float(o16[g]) : 0.f;
+      for (int g = 0; g < DEC_N; ++g) {
+        const float l = red[g] + red[8 + g] + red[16 + g] + red[24 + g];
+        if (g < G)
+          p.o[b * p.o_sb + (long)(kv_head * G + g) * p.o_sh + t] = __float2bfloat16(have && l > 0.f ? __uint_as_float(o16[g]) / l : 0.f);
+      }
+    } else {
+#pragma unroll
+      for (int g = 0; g < DEC_N; ++g) p.part_o[(pbase + g) * DEC_D + t] = have ? __uint_as_float(o16[g]) : 0.f;
+    }
   }
   tc_fence_before();
   __syncthreads();
@@ -321,16 +345,22 @@ static int decode_launch(const void* q, const void* k, const void* v, void* o, f
   p.part_o = work; p.part_m = work + n8 * DEC_D; p.part_l = p.part_m + n8;
   p.err = error_word();
   if (!p.err) return SB_ERR_CUDA;
-  static bool attr_set[64] = {false};
+  p.o = splits == 1 ? (__nv_bfloat16*)o : nullptr;
+  p.o_sb = o_strides[0]; p.o_sh = o_strides[1];
+  const bool many = (long)splits * Hkv * B > 2L * num_sms();
+  auto kern = many ? attention_decode_kernel<1> : attention_decode_kernel<3>;
+  const int smem = many ? DecLayout<1>::SMEM : DecLayout<3>::SMEM;
+  static bool attr_set[2][64] = {{false}};
   int dev = 0;
   SB_CHECK_CUDA(cudaGetDevice(&dev));
-  if (!attr_set[dev & 63]) {
-    SB_CHECK_CUDA(cudaFuncSetAttribute(attention_decode_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, DEC_SMEM));
-    attr_set[dev & 63] = true;
+  if (!attr_set[many][dev & 63]) {
+    SB_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    attr_set[many][dev & 63] = true;
   }
-  attention_decode_kernel<<<dim3(splits, Hkv, B), DEC_THREADS, DEC_SMEM, st>>>(tmK, tmV, p);
-  attention_decode_merge_kernel<<<dim3(Hq, B), DEC_D, 0, st>>>(p.part_o, p.part_m, p.part_l, (__nv_bfloat16*)o,
-                                                               o_strides[0], o_strides[1], Hq, Hkv, splits);
+  kern<<<dim3(splits, Hkv, B), DEC_THREADS, smem, st>>>(tmK, tmV, p);
+  if (splits > 1)
+    attention_decode_merge_kernel<<<dim3(Hq, B), DEC_D, 0, st>>>(p.part_o, p.part_m, p.part_l, (__nv_bfloat16*)o,
+                                                                 o_strides[0], o_strides[1], Hq, Hkv, splits);
   SB_CHECK_CUDA(cudaGetLastError());
   return SB_OK;
 }

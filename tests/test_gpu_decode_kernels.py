@@ -242,3 +242,21 @@ def test_argmax_rows_vector_and_scalar(dtype, rows, vocab, ld, off):
     assert torch.equal(ops.argmax(x).cpu(), want)
     x[0].fill_(float("-inf"))
     assert int(ops.argmax(x)[0]) == 0
+
+
+@gpu
+@pytest.mark.parametrize("B,Hq,Hkv,Sk", [(38, 16, 8, 1), (40, 32, 8, 127), (64, 8, 8, 129), (75, 12, 4, 300), (37, 64, 8, 513), (5, 8, 8, 140)])
+def test_decode_attention_many_sequences(B, Hq, Hkv, Sk):
+    """More (sequence, kv head) pairs than two rounds of SMs: the one-stage kernel, which writes the output itself when the keys
+    are not split; the last case stays on the split form. bf16 probabilities and values: 2^-8 of the weighted sum's terms."""
+    from summa_b200.ops import cuda_ops, native
+    torch.manual_seed(B + Sk)
+    q = torch.randn(B, 1, Hq, 128, device="cuda").to(torch.bfloat16)
+    kc, vc = [torch.randn(B, Sk + 9, Hkv, 128, device="cuda").to(torch.bfloat16) for _ in range(2)]
+    with torch.no_grad():
+        o = cuda_ops.decode_attention(q, kc[:, :Sk], vc[:, :Sk], True, None, Sk - 1)
+    k, v = [t[:, :Sk].double().repeat_interleave(Hq // Hkv, 2).transpose(1, 2) for t in (kc, vc)]
+    p = torch.softmax(q.double().transpose(1, 2) @ k.transpose(-1, -2) / 128 ** 0.5, -1)
+    want = (p @ v).transpose(1, 2)
+    assert bool(((o.double() - want).abs() <= 2.0 ** -7 * (p @ v.abs()).transpose(1, 2) + 2.0 ** -8 * want.abs()).all())
+    assert native.read_error_flag() == 0
