@@ -346,14 +346,14 @@ constexpr int SCANT_SUB = 4;       // replay depth of the tiled kernel
 // checkpoint in two levels: the states at steps 4, 8, 12 stay in registers, then every 4-step group is replayed
 // into a per-thread column of shared memory and swept in reverse. The next segment's inputs are fetched
 // asynchronously during the sweep.
-template <int N, int NB, int SPT>
-__global__ void __launch_bounds__(8 * NB / SPT, NB == 64 ? 3 : 512 / (8 * NB / SPT))
+template <int N, int NB, int SPT, int CPT>
+__global__ void __launch_bounds__(8 * NB / SPT, NB == 64 ? 3 : (CPT == 2 ? 768 : 512) / (8 * NB / SPT))
 selective_scan_bwd_tile_kernel(const ScanBwdParams p) {
   constexpr int NW = NB / (4 * SPT);
   constexpr int THREADS = 32 * NW;
   constexpr int SEG = SCAN_SEG, SUB = SCANT_SUB, NSUB = SEG / SUB;
-  constexpr int CH = 32;
-  constexpr int NQ = SPT / 2, NPR = 4 * NQ;  // f32x2 pairs per thread: pair NQ i + q = channel i, states 2 q, 2 q + 1
+  constexpr int CH = 8 * CPT;
+  constexpr int NQ = SPT / 2, NPR = CPT * NQ;  // f32x2 pairs per thread: pair NQ i + q = channel i, states 2 q, 2 q + 1
   constexpr float LN2 = 0.6931471805599453f;
   extern __shared__ __align__(16) float sm[];
   float* s_dt = sm;                        // [SEG][CH] softplus(delta)
@@ -372,14 +372,14 @@ selective_scan_bwd_tile_kernel(const ScanBwdParams p) {
   const int lc = lane & 7, ln = lane >> 3;
   const int b = blockIdx.y;
   const int c0 = blockIdx.x * CH;
-  const int cb = c0 + 4 * lc;              // first channel of this thread
+  const int cb = c0 + CPT * lc;              // first channel of this thread
   const int nb0 = blockIdx.z * NB;
   const int nl = 4 * SPT * w + SPT * ln;          // first state of this thread inside the block's slice
   const int n0 = nb0 + nl;
   const bool vec = p.vec != 0;
   uint64_t A2[NPR], dh[NPR], dAacc[NPR];
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
+  for (int i = 0; i < CPT; ++i) {
     const bool ok = cb + i < p.C;
 #pragma unroll
     for (int q = 0; q < NQ; ++q) {
@@ -390,7 +390,7 @@ selective_scan_bwd_tile_kernel(const ScanBwdParams p) {
       dAacc[NQ * i + q] = f2_pack(0.f, 0.f);
     }
   }
-  float dDacc = 0.f;                        // slice 0: channel c0 + lane, this warp's steps
+  float dDacc = 0.f;                        // slice 0: channel c0 + lane % CH, this lane's steps
   const int nseg = (p.T + SEG - 1) / SEG;
   auto stage = [&](int seg) {
     const long row0 = (long)b * p.T + seg * SEG;
@@ -405,7 +405,7 @@ selective_scan_bwd_tile_kernel(const ScanBwdParams p) {
   // the segment's checkpoint: this thread's 4 x SPT tile
   auto load_ckpt = [&](int seg, uint64_t (&h)[NPR]) {
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
+    for (int i = 0; i < CPT; ++i) {
       const float* src = p.ckpt + (((long)b * nseg + seg) * p.C + cb + i) * N + n0;
       if (SPT == 4) {
         float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -417,6 +417,15 @@ selective_scan_bwd_tile_kernel(const ScanBwdParams p) {
         if (cb + i < p.C) v = *reinterpret_cast<const float2*>(src);
         h[NQ * i] = f2_pack(v.x, v.y);
       }
+    }
+  };
+  auto load_channels = [](const float* at, float (&v)[CPT]) {
+    if constexpr (CPT == 4) {
+      const float4 t = *reinterpret_cast<const float4*>(at);
+      v[0] = t.x; v[1] = t.y; v[2] = t.z; v[3] = t.w;
+    } else {
+      const float2 t = *reinterpret_cast<const float2*>(at);
+      v[0] = t.x; v[1] = t.y;
     }
   };
   // B_t or C_t of this thread's states
@@ -431,13 +440,13 @@ selective_scan_bwd_tile_kernel(const ScanBwdParams p) {
   };
   // one forward step on all pairs
   auto fwd_step = [&](int tt, uint64_t (&h)[NPR]) {
-    const float4 dt4 = *reinterpret_cast<const float4*>(s_dt + tt * CH + 4 * lc);
-    const float4 u4 = *reinterpret_cast<const float4*>(s_u + tt * CH + 4 * lc);
+    float dtv[CPT], uv[CPT];
+    load_channels(s_dt + tt * CH + CPT * lc, dtv);
+    load_channels(s_u + tt * CH + CPT * lc, uv);
     uint64_t bp[NQ];
     load_pairs(s_B + tt * NB + nl, bp);
-    const float dtv[4] = {dt4.x, dt4.y, dt4.z, dt4.w}, uv[4] = {u4.x, u4.y, u4.z, u4.w};
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
+    for (int i = 0; i < CPT; ++i) {
       const uint64_t dt2 = f2_pack(dtv[i], dtv[i]);
       const float duv = dtv[i] * uv[i];
       const uint64_t du2 = f2_pack(duv, duv);
@@ -454,7 +463,7 @@ selective_scan_bwd_tile_kernel(const ScanBwdParams p) {
     __syncthreads();      // staging complete; the previous segment's epilogue is done with s_po / s_dy / s_u
     if (seg > 0) {          // the next checkpoint's lines on their way to L2
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
+      for (int i = 0; i < CPT; ++i)
         if (ln == 0 && cb + i < p.C)
           asm volatile("prefetch.global.L2 [%0];" ::"l"(p.ckpt + (((long)b * nseg + seg - 1) * p.C + cb + i) * N + n0));
     }
@@ -509,20 +518,19 @@ selective_scan_bwd_tile_kernel(const ScanBwdParams p) {
       for (int k = SUB - 1; k >= 0; --k) {
         const int tt = sb_ * SUB + k;
         if (tt >= steps) continue;          // uniform across the block
-        const float4 dt4 = *reinterpret_cast<const float4*>(s_dt + tt * CH + 4 * lc);
-        const float4 u4 = *reinterpret_cast<const float4*>(s_u + tt * CH + 4 * lc);
-        const float4 dy4 = *reinterpret_cast<const float4*>(s_dy + tt * CH + 4 * lc);
+        float dtv[CPT], uv[CPT], dyv[CPT];
+        load_channels(s_dt + tt * CH + CPT * lc, dtv);
+        load_channels(s_u + tt * CH + CPT * lc, uv);
+        load_channels(s_dy + tt * CH + CPT * lc, dyv);
         uint64_t bp[NQ], cp[NQ];
         load_pairs(s_B + tt * NB + nl, bp);
         load_pairs(s_C + tt * NB + nl, cp);
-        const float dtv[4] = {dt4.x, dt4.y, dt4.z, dt4.w}, uv[4] = {u4.x, u4.y, u4.z, u4.w};
-        const float dyv[4] = {dy4.x, dy4.y, dy4.z, dy4.w};
         uint64_t dBa[NQ], dCa[NQ];
 #pragma unroll
         for (int q = 0; q < NQ; ++q) dBa[q] = dCa[q] = f2_pack(0.f, 0.f);
-        float r2[8];                        // [0,4): ddt of the 4 channels, [4,8): du
+        float r2[2 * CPT];                  // [0, CPT): ddt of the channels, [CPT, 2 CPT): du
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
+        for (int i = 0; i < CPT; ++i) {
           const uint64_t dt2 = f2_pack(dtv[i], dtv[i]), dy2 = f2_pack(dyv[i], dyv[i]);
           const float duv = dtv[i] * uv[i];
           const uint64_t du2 = f2_pack(duv, duv);
@@ -547,7 +555,7 @@ selective_scan_bwd_tile_kernel(const ScanBwdParams p) {
           f2_unpack(sB, b0, b1);
           const float sb2 = b0 + b1;
           r2[i] = fmaf(LN2, a0 + a1, uv[i] * sb2);
-          r2[4 + i] = dtv[i] * sb2;
+          r2[CPT + i] = dtv[i] * sb2;
         }
         float r1[2 * SPT];                  // [0, SPT): dB of the states, [SPT, 2 SPT): dC
 #pragma unroll
@@ -563,7 +571,7 @@ selective_scan_bwd_tile_kernel(const ScanBwdParams p) {
         } else {
           lane_group_reduce<2 * SPT, 8, 0>(r1, lane);
         }
-        lane_group_reduce<8, 4, 3>(r2, lane);     // over the 4 state groups: two totals per lane
+        lane_group_reduce<2 * CPT, 4, 3>(r2, lane);     // over the 4 state groups: CPT / 2 totals per lane
         {
           const int idx = SPT == 4 ? ((lane & 1) << 2) | (lane & 2) | ((lane >> 2) & 1) : ((lane & 1) << 1) | ((lane >> 1) & 1);
           const long o = (((long)blockIdx.x * p.B + b) * p.T + t0 + tt) * N + n0 + (idx & (SPT - 1));
@@ -573,9 +581,11 @@ selective_scan_bwd_tile_kernel(const ScanBwdParams p) {
           }
         }
         {
-          const int idx = (((lane >> 3) & 1) << 2) | (((lane >> 4) & 1) << 1);     // even: values idx, idx + 1
-          float* o = s_po + (((sb_ & 1) * NW + w) * SUB + k) * 2 * CH + (idx < 4 ? 0 : CH) + 4 * lc + (idx & 3);
-          *reinterpret_cast<float2*>(o) = make_float2(r2[0], r2[1]);
+          // values idx .. idx + CPT / 2 - 1 of (ddt | du)
+          const int idx = ((lane >> 3) & 1) * CPT + ((lane >> 4) & 1) * (CPT / 2);
+          float* o = s_po + (((sb_ & 1) * NW + w) * SUB + k) * 2 * CH + (idx < CPT ? 0 : CH) + CPT * lc + (idx & (CPT - 1));
+          if (CPT == 4) *reinterpret_cast<float2*>(o) = make_float2(r2[0], r2[1]);
+          else *o = r2[0];
         }
       }
       // the group's sums over the warps; the other buffer takes the next group meanwhile
@@ -599,7 +609,7 @@ selective_scan_bwd_tile_kernel(const ScanBwdParams p) {
     }
   }
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
+  for (int i = 0; i < CPT; ++i) {
     if (cb + i < p.C) {
 #pragma unroll
       for (int q = 0; q < NQ; ++q) {
@@ -615,17 +625,17 @@ selective_scan_bwd_tile_kernel(const ScanBwdParams p) {
       }
     }
   }
-  if (blockIdx.z == 0 && c0 + lane < p.C) atomicAdd(p.dD + c0 + lane, dDacc);
+  if (blockIdx.z == 0 && c0 + lane % CH < p.C) atomicAdd(p.dD + c0 + lane % CH, dDacc);
 }
 
-template <int N, int NB, int SPT>
+template <int N, int NB, int SPT, int CPT>
 static int launch_scan_bwd_tile(const ScanBwdParams& p, cudaStream_t st) {
-  constexpr int NW = NB / (4 * SPT), THREADS = 32 * NW;
-  const int smem = (3 * SCAN_SEG * 32 + 2 * SCAN_SEG * NB + 2 * NW * SCANT_SUB * 64) * sizeof(float) +
-                   SCANT_SUB * 2 * SPT * THREADS * sizeof(uint64_t) + (3 * SCAN_SEG * 32 + 2 * SCAN_SEG * NB) * sizeof(__nv_bfloat16);
-  auto kern = selective_scan_bwd_tile_kernel<N, NB, SPT>;
+  constexpr int NW = NB / (4 * SPT), THREADS = 32 * NW, CH = 8 * CPT;
+  const int smem = (3 * SCAN_SEG * CH + 2 * SCAN_SEG * NB + 2 * NW * SCANT_SUB * 2 * CH) * sizeof(float) +
+                   SCANT_SUB * (CPT * SPT / 2) * THREADS * sizeof(uint64_t) + (3 * SCAN_SEG * CH + 2 * SCAN_SEG * NB) * sizeof(__nv_bfloat16);
+  auto kern = selective_scan_bwd_tile_kernel<N, NB, SPT, CPT>;
   if (smem > 48 * 1024) SB_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-  dim3 grid((p.C + 31) / 32, p.B, N / NB);
+  dim3 grid((p.C + CH - 1) / CH, p.B, N / NB);
   kern<<<grid, THREADS, smem, st>>>(p);
   SB_CHECK_CUDA(cudaGetLastError());
   return SB_OK;
@@ -852,7 +862,11 @@ conv1d_bwd_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict__
 
 using namespace sb;
 
-// Scan backward. Scratch (fp32): dB_part/dC_part `[ceil(C/32)][B][T][N]`, ddt_part/du_part
+// Channels per partial tile of the B / C gradients.
+static bool few_channels(int N, int B, int C) { return N == 16 && (long)B * ((C + 31) / 32) <= 2L * num_sms(); }
+extern "C" int sb_scan_bwd_tile_channels(int N, int B, int C) { return few_channels(N, B, C) ? 16 : 32; }
+
+// Scan backward. Scratch (fp32): dB_part/dC_part `[ceil(C / sb_scan_bwd_tile_channels(N, B, C))][B][T][N]`, ddt_part/du_part
 // `[max(1, N/64)][B][T][C]`. dA/dD accumulate (zero them first). du/ddelta are bf16
 // `[B,T,C]` contiguous; dBm/dCm bf16 `[B,T,N]` with row strides ld_db / ld_dc.
 extern "C" int sb_scan_bwd(const void* u, const void* delta, const float* A, const void* Bm, const void* Cm,
@@ -873,16 +887,17 @@ extern "C" int sb_scan_bwd(const void* u, const void* delta, const float* A, con
   switch (N) {
     case 8: rc = launch_scan_bwd<8, 8>(p, st); break;
     // Two states per thread where a block would be a single warp (N 16, B 27 T 1024 C 1024: 1281 -> 1084 us with the passes
-    // behind it); from N 32 on four are ahead (N 32 1478 us against 1725, N 128 B 2 T 8192 C 3072 9.8 ms against 12.2).
-    case 16: rc = launch_scan_bwd_tile<16, 16, 2>(p, st); break;
-    case 32: rc = launch_scan_bwd_tile<32, 32, 4>(p, st); break;
-    case 64: rc = launch_scan_bwd_tile<64, 64, 4>(p, st); break;
-    case 128: rc = launch_scan_bwd_tile<128, 64, 4>(p, st); ns = 2; break;
-    case 256: rc = launch_scan_bwd_tile<256, 64, 4>(p, st); ns = 4; break;
+    // behind it), and two channels as well while there are few blocks (B 4: 918 -> 592 us against 737 with four; B 27: 1215
+    // against 1084); from N 32 on four by four is ahead (N 32 1478 us against 1725, N 128 B 2 T 8192 C 3072 9.8 ms against 12.2).
+    case 16: rc = few_channels(N, B, C) ? launch_scan_bwd_tile<16, 16, 2, 2>(p, st) : launch_scan_bwd_tile<16, 16, 2, 4>(p, st); break;
+    case 32: rc = launch_scan_bwd_tile<32, 32, 4, 4>(p, st); break;
+    case 64: rc = launch_scan_bwd_tile<64, 64, 4, 4>(p, st); break;
+    case 128: rc = launch_scan_bwd_tile<128, 64, 4, 4>(p, st); ns = 2; break;
+    case 256: rc = launch_scan_bwd_tile<256, 64, 4, 4>(p, st); ns = 4; break;
     default: return SB_ERR_ARG;
   }
   if (rc) return rc;
-  const int tiles = (C + 31) / 32;
+  const int tiles = (C + sb_scan_bwd_tile_channels(N, B, C) - 1) / sb_scan_bwd_tile_channels(N, B, C);
   const long per_tile = (long)B * T * N;
   const int cap = num_sms() * 8;
   auto blocks_for = [&](long items) { return (int)((items + 255) / 256 < cap ? (items + 255) / 256 : cap); };

@@ -704,6 +704,7 @@ N.register("sb_scan_fwd_log", [N.P] * 10 + [N.I] * 4 + [N.L] * 4 + [N.P])
 N.register("sb_conv1d_fwd_bf16w", [N.P, N.P, N.P, N.P, N.P, N.I, N.I, N.I, N.I, N.L, N.I, N.P])
 N.register("sb_scan_bwd", [N.P] * 20 + [N.I] * 4 + [N.L] * 7 + [N.P])
 N.register("sb_scan_ckpt_interval", [])
+N.register("sb_scan_bwd_tile_channels", [N.I, N.I, N.I])
 
 _SCAN_STATES = (8, 16, 32, 64, 128, 256)
 
@@ -796,7 +797,7 @@ class _SelectiveScan(torch.autograd.Function):
         dys, ld_dy = _btc(dy)
         A32 = A.float().contiguous()
         D32 = D.float().contiguous()
-        tiles = -(-C // 32)
+        tiles = -(-C // N.call_value("sb_scan_bwd_tile_channels", Ns, B, C))
         ns = max(1, Ns // 64)
         dev = u.device
         part_dt = torch.empty(ns, B, T, C, device=dev, dtype=torch.float32)

@@ -155,3 +155,28 @@ def test_scan_and_convolution_inference_forms():
             assert torch.equal(cuda_ops.conv1d_silu(u, w, b), cuda_ops.conv1d_silu(u, w.float(), b))
             v = torch.empty(C * K + 1, device="cuda")[1:].view(C, 1, K).copy_(w.float())      # taps that are not 16-byte aligned
             assert torch.equal(cuda_ops.conv1d_silu(u, v, b), cuda_ops.conv1d_silu(u, w.float(), b))
+
+
+@gpu
+@pytest.mark.parametrize("B,T,C,Ns", [(1, 17, 40, 16), (2, 33, 34, 16), (75, 5, 128, 16), (2, 19, 72, 32), (1, 18, 64, 64), (1, 21, 36, 128)])
+def test_scan_backward_tiles(B, T, C, Ns):
+    """Every gradient for ragged channel tiles and segments, on both sides of the channel-tile rule (75 x 128 / 32 blocks are
+    more than two per SM), against fp64 autograd of the recurrence. bf16 outputs round to 2^-9 and the inputs of dA and dD
+    are sums of B T products in fp32."""
+    from summa_b200.ops import cuda_ops
+    torch.manual_seed(B + T + C)
+    u, d, Bm, Cm = [torch.randn(*s, device="cuda").to(torch.bfloat16) for s in ((B, T, C), (B, T, C), (B, T, Ns), (B, T, Ns))]
+    A, D = -torch.rand(C, Ns, device="cuda") - 0.1, torch.randn(C, device="cuda")
+    dy = torch.randn(B, T, C, device="cuda").to(torch.bfloat16)
+    lo = [t.detach().clone().requires_grad_() for t in (u, d, A, Bm, Cm, D)]
+    y, _ = cuda_ops.selective_scan(*lo)
+    y.backward(dy)
+    hi = [t.detach().double().requires_grad_() for t in (u, d, A, Bm, Cm, D)]
+    dt = torch.nn.functional.softplus(hi[1])
+    h, ys = torch.zeros(B, C, Ns, device="cuda", dtype=torch.float64), []
+    for t in range(T):
+        h = torch.exp(dt[:, t, :, None] * hi[2]) * h + (dt[:, t] * hi[0][:, t])[..., None] * hi[3][:, t, None]
+        ys.append((h * hi[4][:, t, None]).sum(-1) + hi[5] * hi[0][:, t])
+    torch.stack(ys, 1).backward(dy.double())
+    for a, b in zip(lo, hi):
+        assert float((a.grad.double() - b.grad).norm() / b.grad.norm()) <= 2.0 ** -8
