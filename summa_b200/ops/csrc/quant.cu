@@ -116,10 +116,7 @@ template <int MPMAX, int G> struct WqCfg {
   static constexpr int DQ = G;
   static constexpr int THREADS = 128 * DQ + 64;
   static constexpr int NA = 4;                              // expanded weight buffers in tensor memory (32 columns each)
-  // a group skips blocks, so it does not see every phase of a buffer's `free` barrier; a parity wait stays
-  // unambiguous because the ring bounds how far the MMA can lag: block i is only loaded once block i - NS has been
-  // consumed, and i - NS >= i - 2 NA
-  static_assert(DQ == 1 || NS <= 2 * NA, "ring deeper than two rounds of weight buffers: free-barrier parity would alias");
+  static_assert(NS > NA, "the stage's barrier must still be in the phase of block i - NA when block i is expanded");
 };
 
 struct W4Params {
@@ -142,10 +139,12 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + WQ_NS * WQ_STAGE);
   uint64_t* full = bars;                 // [NS]
-  uint64_t* empty = bars + WQ_NS;        // [NS]
+  // [NS] a block's products are complete: frees its ring stage and its expanded weight buffer. One commit per block instead
+  // of one for each of the two; K 4096, N 28672: 12 rows 41.4 -> 39.9 us, 64 rows 43.7 -> 42.1 us, 512 rows 158.9 ->
+  // 153.1 us; K 14336, N 4096, 512 rows 65.0 -> 60.5 us.
+  uint64_t* done = bars + WQ_NS;
   uint64_t* a_full = bars + 2 * WQ_NS;   // [NA] one arrival per dequant thread
-  uint64_t* a_free = a_full + NA;        // [NA]
-  uint64_t* d_full = a_free + NA;
+  uint64_t* d_full = a_full + NA;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(d_full + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -154,8 +153,8 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
   const int kb0 = blockIdx.y * p.kb_per_split;
   const int nkb = max(0, min(p.kb_per_split, kblocks - kb0));
   if (threadIdx.x == 0) {
-    for (int s = 0; s < WQ_NS; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
-    for (int s = 0; s < NA; ++s) { mbar_init(&a_full[s], 128); mbar_init(&a_free[s], 1); }
+    for (int s = 0; s < WQ_NS; ++s) { mbar_init(&full[s], 1); mbar_init(&done[s], 1); }
+    for (int s = 0; s < NA; ++s) mbar_init(&a_full[s], 128);
     mbar_init(d_full, 1);
     *abort_flag = 0;
     fence_barrier_init();
@@ -178,7 +177,7 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
     if (lane == 0) {
       for (int i = 0; i < nkb; ++i) {
         const int s = i % WQ_NS;
-        if (!mbar_wait(&empty[s], ((i / WQ_NS) & 1) ^ 1, abort_flag, p.err)) break;
+        if (!mbar_wait(&done[s], ((i / WQ_NS) & 1) ^ 1, abort_flag, p.err)) break;
         mbar_expect_tx(&full[s], WQ_WBYTES + p.MP * 128);
         tma_load_2d(smem + s * WQ_STAGE, &tmW, &full[s], n0, (kb0 + i) * 8);
         tma_load_2d(smem + s * WQ_STAGE + WQ_WBYTES, &tmX, &full[s], (kb0 + i) * 64, m0);
@@ -200,8 +199,7 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
         for (int kk = 0; kk < 4; ++kk)
           umma_bf16_ta(tmem_base + COL_D, tmem_base + COL_A + 32 * b + 8 * kk,
                        make_smem_desc_sw128(x_base + kk * 32, 16, 1024), idesc, (i > 0 || kk > 0) ? 1u : 0u);
-        umma_commit(&a_free[b]);
-        umma_commit(&empty[s]);
+        umma_commit(&done[s]);
       }
       if (ok) umma_commit(d_full);
     }
@@ -243,7 +241,10 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
           r[4 * jj + q] = *reinterpret_cast<uint32_t*>(&v);
         }
       }
-      if (i >= NA && !mbar_wait(&a_free[b], ((i / NA) - 1) & 1, abort_flag, p.err)) { ok = false; break; }
+      // Buffer b was last read by block i - NA. The parity is unambiguous: block i is loaded, so block i - NS and with it
+      // every earlier phase of this barrier is complete, and its next phase (block i - NA + NS > i) cannot be before block
+      // i is handed over.
+      if (i >= NA && !mbar_wait(&done[(i - NA) % WQ_NS], ((i - NA) / WQ_NS) & 1, abort_flag, p.err)) { ok = false; break; }
       tc_fence_after();
       tmem_st_32x32b_x32(tmem_base + COL_A + 32 * b + lane_sel, r);
       tmem_st_wait();
