@@ -230,6 +230,32 @@ def test_hybrid_graph_decode_against_eager(B):
 
 
 @gpu
+@pytest.mark.parametrize("short", [False, True])
+def test_decode_capture_empties_the_cache_only_when_memory_is_short(short, monkeypatch):
+    """Whole numbers: both ways of capturing give the same tokens as the eager decode."""
+    from summa_b200.models import Transformer
+    from summa_b200.models.engine import InferenceEngine
+    torch.manual_seed(3)
+    with torch.device("cuda"):
+        model = Transformer(_hybrid(16, 4), init_std=0.1)
+    model.prepare_inference(torch.bfloat16)
+    eng = InferenceEngine(model)
+    eng.reset(2, 24)
+    prompt = torch.randint(0, 512, (2, 7), device="cuda")
+    first = eng.prefill(prompt)
+    free, calls, empty_cache = 0 if short else 1 << 40, [], torch.cuda.empty_cache
+    monkeypatch.setattr(torch.cuda, "mem_get_info", lambda *a: (free, 1 << 40))
+    monkeypatch.setattr(torch.cuda, "empty_cache", lambda: (calls.append(1), empty_cache()))
+    tokens = eng.decode(first, 6)
+    assert eng._graph is not None and eng._graph.graph is not None and len(calls) == int(short)
+    plain = InferenceEngine(model)
+    plain.use_graph = False
+    plain.reset(2, 24)
+    again = plain.prefill(prompt)
+    assert torch.equal(first, again) and torch.equal(tokens, plain.decode(again, 6))
+
+
+@gpu
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("rows,vocab,ld,off", [(1, 1, 8, 0), (3, 32000, 32064, 0), (2, 8191, 8192, 0), (2, 1003, 1003, 0), (2, 50, 64, 1)])
 def test_argmax_rows_vector_and_scalar(dtype, rows, vocab, ld, off):
