@@ -2,8 +2,8 @@
 ternary codecs (`HQuantLinear`), plus the loader of a quantised archive.
 
 `QuantLinear` holds a `[d_in, d_out]` weight as packed int4 codes (group 128 along d_in,
-bf16 scales). Decode-sized inputs (<= 64 rows) run the weight-streaming GEMV kernel, which
-reads the packed weight once; inputs of up to 512 rows (short prefill chunks, speculative batches) run the
+bf16 scales). Decode-sized inputs (<= 64 rows) run the weight-streaming kernel (few rows)
+or the fused dequant-GEMM, which read the packed weight once; inputs of up to 512 rows (short prefill chunks, speculative batches) run the
 fused dequant-GEMM, which expands each 4-bit weight tile in registers on its way into tensor memory (no bf16
 copy of the weight exists); longer prefill expands the weight once into a reused bf16 workspace and runs the
 plain tensor-core GEMM, which is the faster form there (numbers beside `PREFILL_FUSED_MAX_ROWS`). The reference has only a host-side oracle for

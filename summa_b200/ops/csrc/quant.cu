@@ -96,7 +96,7 @@ int4_gemv_kernel(const __nv_bfloat16* __restrict__ x, const uint8_t* __restrict_
 // one CTA per SM, no K split: the weight tile is expanded once per 128 x MP output tile, in registers, on its
 // way into tensor memory, and never exists in global memory.
 constexpr int WQ_WBYTES = 8 * 128 * 4;           // repacked weight tile
-// Decode rows run three expanding groups too: 64 rows, N 28672 52.8 -> 44.4 us against one group, N 6144 18.8 -> 16.9,
+// Decode rows run three expanding groups too: 64 rows, N 28672 52.8 -> 44.4 us against one group (when the change was made; 42.1 now), N 6144 18.8 -> 16.9,
 // K 14336 N 4096 27.2 -> 25.6, N 4096 level (12.6 / 12.7).
 constexpr int W4A16_GROUPS = 3;
 template <int MPMAX, int G> struct WqCfg {

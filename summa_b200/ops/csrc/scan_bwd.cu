@@ -1,7 +1,7 @@
 // Mamba-1 kernels, backward side: segmented selective-scan backward and the depthwise
 // conv1d (+SiLU) backward.
 //
-// Scan backward, N >= 16: the tiled kernel (a thread owns 4 channels x 4 states; see
+// Scan backward, N >= 16: the tiled kernel (a thread owns 4 channels x 4 states, at N 16 fewer; see
 // selective_scan_bwd_tile_kernel). N = 8 keeps the one-channel-per-lane kernel: lane = channel,
 // warp = 8 states, state and its gradient in registers. Both visit the 16-step segments last to
 // first; each segment starts from the forward pass's checkpoint and rebuilds its states in two

@@ -1263,7 +1263,7 @@ def int4_gemv_swiglu(x, packed_k8, scales, norm=None):
 
 def int4_gemv(x, packed, scales, residual=None, packed_k8=None, norm=None):
     """x `[M <= 64, K]` @ dequant(W) (+ residual). With the repacked weight (`reference.repack_int4_k8`)
-    the product runs on the tensor cores (M > 4) or as the one-launch cluster GEMV (M <= 4);
+    the product runs on the streaming integer-mma kernel (few rows) or the tcgen05 W4A16 kernel;
     otherwise on the CUDA-core weight-streaming kernel. `norm=(gamma fp32 [K], eps)` applies RMSNorm
     to x first (fused into the GEMV for M <= 4)."""
     M, K = x.shape
@@ -1285,7 +1285,7 @@ def int4_gemv(x, packed, scales, residual=None, packed_k8=None, norm=None):
         return y
     if (packed_k8 is not None and M <= (8 if use_mma else 4) and ldx % 8 == 0 and x2.data_ptr() % 16 == 0
             and K % 128 == 0 and Nn % 4 == 0 and K <= (98304 if use_mma else 20480)):
-        # batch 1..8 decode: one launch, K split over a thread-block cluster, no accumulator pass
+        # few rows: one launch (streaming kernel, or the older bf16-mma form), no accumulator pass
         fuse = norm is not None and norm[0].dtype == torch.float32 and norm[0].is_contiguous()
         if norm is not None and not fuse:
             x2 = rmsnorm(x2, norm[0], norm[1])
