@@ -45,7 +45,6 @@ __device__ __forceinline__ void w4s_copy8(uint32_t dst_smem, const void* src) {
 __device__ __forceinline__ uint32_t w4s_lo(uint32_t w) { return ((w << 4) & 0xF0F0F0F0u) ^ 0x80808080u; }
 __device__ __forceinline__ uint32_t w4s_hi(uint32_t w) { return (w & 0xF0F0F0F0u) ^ 0x80808080u; }
 
-template <int MT> constexpr int W4S_X_BYTES = MT == 0 ? 84 * 1024 : 104 * 1024;     // digits of x of one K pass
 template <int MT> constexpr int W4S_DEPTH = MT == 0 ? 6 : 4;
 constexpr int W4S_MAGIC = 0x4B400000;        // float bits of 1.5 * 2^23: adding a small integer to the bits adds it to the value
 
@@ -405,25 +404,38 @@ w4_stream_kernel(const W4StreamArgs p, const int tile_base, const int tiles, con
   for (int q = max(handed - 2, 0); q < handed; ++q) epilogue(q);
 }
 
+// How a call is cut: scale groups per K pass and column tiles per launch. The digits of a pass stay in shared memory while the
+// CTA walks its tiles; K goes in passes when they do not all fit next to the rings and buffers. Partial sums then wait in
+// shared memory (at least W4S_PSUM_TILES tiles per CTA, or all of them), what does not fit goes to further launches.
+constexpr int W4S_PSUM_TILES = 8;
+struct W4SPlan { int pass_groups, tiles_per_cta; };             // tiles_per_cta: tiles of a launch per CTA, 0 = all at once
+static bool w4s_plan(int M, int K, int tiles, int sms, bool norm, W4SPlan& out) {
+  const int rows = 8, depth = M <= 2 ? W4S_DEPTH<0> : W4S_DEPTH<1>, groups = K / 128;
+  auto bytes = [&](int pass_groups, int psum_tiles) { return w4s_layout(rows, depth, M, pass_groups, groups, norm, psum_tiles).total; };
+  if (bytes(groups, 0) <= W4S_SMEM) {
+    out = {groups, 0};
+    return true;
+  }
+  const int all = (tiles + sms - 1) / sms, kept = all < W4S_PSUM_TILES ? all : W4S_PSUM_TILES;
+  const int fit = (W4S_SMEM - bytes(0, kept)) / (bytes(1, 0) - bytes(0, 0));
+  if (fit < 1) return false;
+  const int passes = (groups + fit - 1) / fit;
+  int pass_groups = ((groups + passes - 1) / passes + W4S_WARPS - 1) / W4S_WARPS * W4S_WARPS;      // whole rounds of the warps
+  if (pass_groups > fit) pass_groups = fit < W4S_WARPS ? fit : fit / W4S_WARPS * W4S_WARPS;
+  const int room = (W4S_SMEM - bytes(pass_groups, 0)) / (M * W4S_TILE * 4);
+  out = {pass_groups, room < all ? room : all};
+  return true;
+}
+
 template <int MT, int MODE>
 static int w4s_launch(const W4StreamArgs& a, cudaStream_t st) {
   constexpr int ROWS = MT == 0 ? 8 : 8 * MT;
   const int groups = a.K / 128;
   const bool norm = a.gamma != nullptr;
   const int tiles = MODE == W4S_GATED ? (a.N / 2 + 7) / 8 : (a.N + W4S_TILE - 1) / W4S_TILE;
-  // K passes: the digits of a pass stay in shared memory while the CTA walks its tiles
-  const int fit = W4S_X_BYTES<MT> / (a.M * 3 * 128);
-  const int passes = (groups + fit - 1) / fit;
-  int pass_groups = (groups + passes - 1) / passes;
-  if (passes > 1) {             // whole rounds of the warps
-    pass_groups = (pass_groups + W4S_WARPS - 1) / W4S_WARPS * W4S_WARPS;
-    if (pass_groups > fit) pass_groups = fit < W4S_WARPS ? fit : fit / W4S_WARPS * W4S_WARPS;
-  }
-  const int base_smem = w4s_layout(ROWS, W4S_DEPTH<MT>, a.M, pass_groups, groups, norm, 0).total;
-  int most = tiles;
-  if (pass_groups < groups)     // partial sums wait in shared memory: as many tiles per CTA as fit, the rest in further launches
-    most = (W4S_SMEM - base_smem) / (a.M * W4S_TILE * 4) * num_sms();
-  SB_CHECK_ARG(base_smem <= W4S_SMEM && most > 0);
+  W4SPlan plan;
+  SB_CHECK_ARG(w4s_plan(a.M, a.K, tiles, num_sms(), norm, plan));
+  const int pass_groups = plan.pass_groups, most = plan.tiles_per_cta > 0 ? plan.tiles_per_cta * num_sms() : tiles;
   unsigned int* err = error_word();
   if (!err) return SB_ERR_CUDA;
   auto kern = w4_stream_kernel<MT, MODE>;
@@ -455,7 +467,10 @@ static int w4s_launch(const W4StreamArgs& a, cudaStream_t st) {
   return SB_OK;
 }
 
-bool w4_stream_one_pass(int M, int K) { return (long)M * 3 * K <= (M <= 2 ? W4S_X_BYTES<0> : W4S_X_BYTES<1>); }
+bool w4_stream_one_pass(int M, int K) {
+  W4SPlan plan;
+  return w4s_plan(M, K, 1, 1, false, plan) && plan.pass_groups == K / 128;
+}
 
 int launch_w4_stream(const W4StreamArgs& a, W4StreamMode mode, cudaStream_t st) {
   SB_CHECK_ARG(a.M >= 1 && a.M <= W4S_MAX_ROWS && a.K > 0 && a.K % 128 == 0 && a.N > 0 && a.N % 4 == 0 && a.ldx % 8 == 0);
@@ -473,3 +488,16 @@ int launch_w4_stream(const W4StreamArgs& a, W4StreamMode mode, cudaStream_t st) 
 }
 
 }  // namespace sb
+
+// Host check of the cut of a call on a GPU of `sms` SMs: dynamic shared memory of its largest launch in bytes, -1 when the call
+// would be refused. passes receives the number of K passes.
+extern "C" int sb_w4_stream_smem(int M, int N, int K, int norm, int sms, int* passes) {
+  using namespace sb;
+  const int groups = K / 128;
+  W4SPlan plan;
+  if (!w4s_plan(M, K, (N + W4S_TILE - 1) / W4S_TILE, sms, norm != 0, plan)) return -1;
+  *passes = (groups + plan.pass_groups - 1) / plan.pass_groups;
+  if (*passes > 1 && plan.tiles_per_cta < 1) return -1;
+  const int bytes = w4s_layout(8, M <= 2 ? W4S_DEPTH<0> : W4S_DEPTH<1>, M, plan.pass_groups, groups, norm != 0, plan.tiles_per_cta).total;
+  return bytes <= W4S_SMEM ? bytes : -1;
+}

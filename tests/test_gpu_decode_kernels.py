@@ -13,8 +13,24 @@ def _w4(K, N, seed):
     return packed, scales, reference.repack_int4_k8(packed), reference.dequantize_int4_g128(packed.cpu(), scales.cpu()).double().cuda()
 
 
+@pytest.mark.parametrize("norm", [0, 1])
+@pytest.mark.parametrize("M", range(1, 9))
+def test_w4_stream_cuts_every_k_to_fit_shared_memory(M, norm):
+    """The host's cut of a call, without a GPU: whatever K, rows, columns and SMs, its launches fit the 220 KB of a CTA."""
+    import ctypes
+    from summa_b200.ops import native
+    passes, seen = ctypes.c_int(0), set()
+    for K in list(range(128, 131072, 128)) + [196608, 262144]:
+        for N, sms in ((4, 148), (4096, 148), (152064, 148), (28672, 20)):
+            got = native.lib().sb_w4_stream_smem(M, N, K, norm, sms, ctypes.byref(passes))
+            assert 0 < got <= 220 * 1024 and passes.value >= 1, (K, N, sms)
+            seen.add(passes.value)
+    assert 1 in seen and 2 in seen
+
+
 @gpu
 @pytest.mark.parametrize("M,K,N", [
+    (1, 28032, 20), (1, 28672, 40), (2, 28672, 24), (1, 53376, 12), (1, 86016, 8),  # one row around the last K of one pass
     (1, 128, 4), (2, 256, 20), (3, 2048, 16), (1, 2176, 132), (8, 1920, 68),        # one group; fewer and more than 16 groups; ragged tiles
     (2, 14464, 36), (1, 20480, 28), (4, 9088, 44), (8, 4352, 2400),                 # K in passes / the last that fits one pass
     (8, 4736, 52), (5, 14336, 40)])                                                 # rows 5..8 beyond one pass: the other kernel
