@@ -1,15 +1,12 @@
 // 4-bit projection of a decode step, y[M,N] = x[M,K] @ dequant(W) for few rows (weights in the k8-repacked form of
-// quant.cu), as a register-prefetched weight stream feeding warp-level integer mma.
+// quant.cu), as a weight stream through per-warp rings of asynchronous copies feeding warp-level mma.
 //
 // What bounds it: the weight bytes, if the code words can be consumed in few instructions and enough of them are in
 // flight. Measured on a B200: a kernel that only loads the words of a 4096 x 28672 weight takes 14.0 us (6.3 TB/s plus
 // 4.6 us of launch and ramp) with 16 warps x 4 KB in flight per SM, and 20 us with 8 warps.
-//   * x is quantised EXACTLY ENOUGH instead of the weights being widened: per scale group of 128 k, x becomes a 22-bit
-//     fixed-point number (power-of-two step below 2^-21 of the group's largest magnitude, so every bf16 within a factor
-//     2^13 of it is exact) in three signed base-256 digits. A code word then needs one shift and two LOP3 to be the s8
-//     operands 16 (q - 8) of 8 k, against seven instructions for bf16 pairs, and ONE mma.m16n8k32 (s8, s32 accumulation,
-//     exact) takes 16 columns x 32 k of weights against 8 columns of digits. The products of a group are whole numbers;
-//     only the combination over groups rounds (fp32).
+//   * x stays bf16 and a code word becomes the eight bf16 values q - 8 (three shifts, four LOP3, four subtractions, all
+//     exact), so every product is exact whatever the range of x, and the sums of a scale group are fp32. Two
+//     mma.m16n8k16 take 16 columns x 32 k of a word row against all 8 rows of x.
 //   * one CTA per SM walks 16-column tiles over the whole K range; its 16 warps take the scale groups
 //     round robin, each through a ring of its own in shared memory that asynchronous copies fill D groups (D KB) ahead,
 //     across tiles; no barrier, no producer. (A ring in registers is held up by whatever touches a loaded register
@@ -18,10 +15,6 @@
 //     turn it is adds them and runs the epilogue two tiles later (mbarriers both ways). With one block barrier and an
 //     immediate epilogue per tile its latency was paid per tile. No cluster, no atomics.
 //   * the weights depend on nothing, so the first groups are requested before `griddepcontrol.wait`.
-// Measured against the CUDA-core cluster kernel it replaces (weights from HBM, graph of launches, one row): K 4096 N 6144
-// 12.0 -> 7.3 us, N 4096 7.4 -> 5.8, N 28672 29.0 -> 20.2 (gated with norm 32.9 -> 22.2), N 32000 30.1 -> 22.4, K 14336
-// N 4096 20.0 -> 12.5; four rows: 20.0 -> 9.5, 14.6 -> 8.0, 60.4 -> 25.7, 66.7 -> 27.6, 41.6 -> 22.8. Relative error
-// against 64 bits: the same 0.00165 (the rounding of y to bf16).
 #include "host_util.h"
 #include "sm100.cuh"
 #include "w4_stream.h"
@@ -31,59 +24,50 @@ namespace sb {
 constexpr int W4S_WARPS = 16, W4S_THREADS = 512, W4S_TILE = 16, W4S_NB = 4;
 constexpr int W4S_SMEM = 220 * 1024;
 
-__device__ __forceinline__ void w4s_mma(int (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
+__device__ __forceinline__ void w4s_mma(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
                                         uint32_t b1) {
-  asm volatile("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, "
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, "
                "{%0, %1, %2, %3};"
-               : "+r"(d[0]), "+r"(d[1]), "+r"(d[2]), "+r"(d[3])
+               : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
                : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 __device__ __forceinline__ void w4s_copy8(uint32_t dst_smem, const void* src) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst_smem), "l"(reinterpret_cast<uint64_t>(src)) : "memory");
 }
-// codes of k 0,4,1,5 / 2,6,3,7 of a word as s8 bytes 16 (q - 8)
-__device__ __forceinline__ uint32_t w4s_lo(uint32_t w) { return ((w << 4) & 0xF0F0F0F0u) ^ 0x80808080u; }
-__device__ __forceinline__ uint32_t w4s_hi(uint32_t w) { return (w & 0xF0F0F0F0u) ^ 0x80808080u; }
+// codes of k 2 i, 2 i + 1 of a word as the bf16 pair q - 8 (0x4300 | q is 128 + q; both steps exact)
+__device__ __forceinline__ uint32_t w4s_pair(uint32_t w, int i) {
+  const uint32_t u = ((w >> (4 * i)) & 0x000F000Fu) | 0x43004300u;
+  const __nv_bfloat162 v = __hsub2(*reinterpret_cast<const __nv_bfloat162*>(&u), __float2bfloat162_rn(136.f));
+  return *reinterpret_cast<const uint32_t*>(&v);
+}
 
-template <int MT> constexpr int W4S_DEPTH = MT == 0 ? 6 : 4;
-constexpr int W4S_MAGIC = 0x4B400000;        // float bits of 1.5 * 2^23: adding a small integer to the bits adds it to the value
-
-// MT = 0: up to two rows, their 3 M digits are the columns of one mma. MT = 1: up to eight rows, one mma per digit.
 constexpr int W4S_SLOT = 1024 + 32;           // a group of a tile: 16 k8 rows x 64 bytes (chunks swizzled), 16 scales
-struct W4SLayout {                           // shared memory, in bytes
-  int ring, pitch, sx, red, psum, gsq, total;   // pitch: digit row of x (32 mod 128: conflict-free B loads)
+struct W4SLayout {                           // shared memory, in bytes; x comes first
+  int pitch, ring, red, psum, gsq, total;    // pitch: row of x (64 mod 128: conflict-free 16-byte B loads)
 };
-__host__ __device__ inline W4SLayout w4s_layout(int rows, int depth, int M, int pass_groups, int groups, bool norm, int psum_tiles) {
+__host__ __device__ inline W4SLayout w4s_layout(int depth, int M, int pass_groups, int groups, bool norm, int psum_tiles) {
   W4SLayout l;
-  l.ring = 3 * M * (pass_groups * 128 + 32);                       // [warps][depth] slots
-  l.pitch = pass_groups * 128 + 32;
-  l.sx = l.ring + W4S_WARPS * depth * W4S_SLOT;                                           // [pass_groups][rows] fp32
-  l.red = l.sx + pass_groups * rows * 4;                            // [buffers][warps][rows][16] fp32
-  l.psum = l.red + W4S_NB * W4S_WARPS * rows * W4S_TILE * 4;             // [psum_tiles][M][16] fp32 (more than one K pass)
-  l.gsq = l.psum + psum_tiles * M * W4S_TILE * 4;                   // [M] rstd, [M][groups] sums of squares
+  l.pitch = pass_groups * 256 + 64;
+  l.ring = M * l.pitch;                                                       // [warps][depth] slots
+  l.red = l.ring + W4S_WARPS * depth * W4S_SLOT;                              // [buffers][warps][rows][16] fp32, rows in pairs
+  l.psum = l.red + W4S_NB * W4S_WARPS * ((M + 1) & ~1) * W4S_TILE * 4;        // [psum_tiles][M][16] fp32 (more than one K pass)
+  l.gsq = l.psum + psum_tiles * M * W4S_TILE * 4;                             // [M] rstd, [M][groups] sums of squares
   l.total = l.gsq + (norm ? (M + M * groups) * 4 : 0);
   return l;
 }
 
-template <int MT, int MODE>
+template <int D, int MODE>                   // D: scale groups in flight per warp
 __global__ void __launch_bounds__(W4S_THREADS, 1)
 w4_stream_kernel(const W4StreamArgs p, const int tile_base, const int tiles, const int pass_groups, const int psum_tiles,
                  unsigned int* err) {
-  constexpr bool COMPACT = MT == 0;
-  constexpr int SETS = COMPACT ? 1 : MT;      // accumulator sets (8 columns of digits or 8 rows each)
-  constexpr int DIG = COMPACT ? 1 : 3;
-  constexpr int ROWS = 8 * SETS;
-  constexpr int D = W4S_DEPTH<MT>;            // units (scale groups) in flight per warp
   extern __shared__ __align__(128) unsigned char w4s_smem[];
   __shared__ uint64_t full[W4S_NB], empty[W4S_NB];
   __shared__ int abort_flag;
   asm volatile("griddepcontrol.launch_dependents;");
-  const int M = p.M, N = p.N, K = p.K;
+  const int M = p.M, N = p.N, K = p.K, RP = (p.M + 1) & ~1;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gq = lane >> 2, tq = lane & 3;
   const int groups = K >> 7;
-  const W4SLayout L = w4s_layout(ROWS, D, M, pass_groups, groups, p.gamma != nullptr, psum_tiles);
-  unsigned char* xq = w4s_smem;
-  float* sx = reinterpret_cast<float*>(w4s_smem + L.sx);
+  const W4SLayout L = w4s_layout(D, M, pass_groups, groups, p.gamma != nullptr, psum_tiles);
   float* red = reinterpret_cast<float*>(w4s_smem + L.red);
   float* psum = reinterpret_cast<float*>(w4s_smem + L.psum);
   float* rstd = reinterpret_cast<float*>(w4s_smem + L.gsq);
@@ -112,7 +96,7 @@ w4_stream_kernel(const W4StreamArgs p, const int tile_base, const int tiles, con
     const int chunk = (warp - local) & (W4S_WARPS - 1);
     if (chunk >= chunks) return;
     const bool last = pass + 1 == passes;
-    const float* rb = red + (q & (W4S_NB - 1)) * W4S_WARPS * ROWS * W4S_TILE;
+    const float* rb = red + (q & (W4S_NB - 1)) * W4S_WARPS * RP * W4S_TILE;
     const int o = chunk * 32 + lane, m = o >> 4, c = o & 15;
     const bool row = m < M;
     const int mm = row ? m : 0;
@@ -123,14 +107,7 @@ w4_stream_kernel(const W4StreamArgs p, const int tile_base, const int tiles, con
     if (!mbar_wait(&full[q & (W4S_NB - 1)], (q / W4S_NB) & 1, &abort_flag, err)) return;
     float v = 0.f;
 #pragma unroll
-    for (int w = 0; w < W4S_WARPS; ++w) {
-      if (COMPACT) {
-        const float* r = rb + (w * ROWS + 3 * mm) * W4S_TILE + c;
-        v += r[0] + r[W4S_TILE] + r[2 * W4S_TILE];
-      } else {
-        v += rb[(w * ROWS + mm) * W4S_TILE + c];
-      }
-    }
+    for (int w = 0; w < W4S_WARPS; ++w) v += rb[(w * RP + mm) * W4S_TILE + c];
     if (passes > 1) {
       float* ps = psum + (local * M + mm) * W4S_TILE + c;
       if (pass > 0 && row) v += *ps;
@@ -219,7 +196,7 @@ w4_stream_kernel(const W4StreamArgs p, const int tile_base, const int tiles, con
     rewind(g0);
     lslot = 0;
     for (int d = 0; d < D; ++d) load(g0);
-    // ---- x: (fused norm) -> digits and steps of this pass; half a warp takes one (row, group)
+    // ---- the rows of x of this pass, normed on the way; half a warp takes one (row, group)
     const int l16 = threadIdx.x & 15;
     uint4 v[4];
     bool kept = false;                        // v holds this half-warp's items already
@@ -254,10 +231,9 @@ w4_stream_kernel(const W4StreamArgs p, const int tile_base, const int tiles, con
           s = warp_sum(s);
           if (lane == 0) rstd[m] = rsqrtf(s / static_cast<float>(K) + p.eps);
         }
+        __syncthreads();
       }
     }
-    for (int i = threadIdx.x; i < ng * ROWS; i += 32 * W4S_WARPS) sx[i] = 0.f;    // rows beyond M
-    __syncthreads();                                                             // (pass > 0: nobody reads the old digits any more)
     for (int i1 = 2 * warp; i1 < M * ng; i1 += 4 * 32) {
       const int i0 = i1 + (lane >> 4);
 #pragma unroll
@@ -267,55 +243,26 @@ w4_stream_kernel(const W4StreamArgs p, const int tile_base, const int tiles, con
       }
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
-        if (i1 + 32 * q >= M * ng) break;
-        const int i = min(i0 + 32 * q, M * ng - 1), m = i / ng, gl = i - m * ng;
-        uint32_t u[4] = {v[q].x, v[q].y, v[q].z, v[q].w};
+        const int i = i0 + 32 * q, m = i / ng, gl = i - m * ng;
+        if (i >= M * ng) break;
+        uint4 u = v[q];
         if (p.gamma != nullptr) {
           const float r = rstd[m];
           const float2* gp = reinterpret_cast<const float2*>(p.gamma + (g0 + gl) * 128 + 8 * l16);
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            const float2 gm = __ldg(gp + e);
-            u[e] = pack_bf16(bf16_lo(u[e]) * r * gm.x, bf16_hi(u[e]) * r * gm.y);
-          }
+          const float2 a = __ldg(gp), b = __ldg(gp + 1), c = __ldg(gp + 2), d = __ldg(gp + 3);
+          u.x = pack_bf16(bf16_lo(u.x) * r * a.x, bf16_hi(u.x) * r * a.y);
+          u.y = pack_bf16(bf16_lo(u.y) * r * b.x, bf16_hi(u.y) * r * b.y);
+          u.z = pack_bf16(bf16_lo(u.z) * r * c.x, bf16_hi(u.z) * r * c.y);
+          u.w = pack_bf16(bf16_lo(u.w) * r * d.x, bf16_hi(u.w) * r * d.y);
         }
-        // largest magnitude of the group, as bf16 bits (NaN > Inf > finite as unsigned numbers)
-        uint32_t mx = __vmaxu2(__vmaxu2(u[0] & 0x7FFF7FFFu, u[1] & 0x7FFF7FFFu), __vmaxu2(u[2] & 0x7FFF7FFFu, u[3] & 0x7FFF7FFFu));
-        mx = max(mx & 0xFFFFu, mx >> 16);
-#pragma unroll
-        for (int o = 8; o > 0; o >>= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-        const bool finite = mx < 0x7F80u;
-        const uint32_t E = max(mx >> 7, 27u);                       // biased exponent; |x| < 2^(E - 126)
-        const float inv = __uint_as_float((274u - min(E, 254u)) << 23);          // 2^(20 - (E - 127)): |x inv| < 2^21
-        uint32_t y[8];
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const float a = finite ? bf16_lo(u[e]) : 0.f, b = finite ? bf16_hi(u[e]) : 0.f;
-          y[2 * e] = (__float_as_uint(fmaf(a, inv, 12582912.f)) - (uint32_t)W4S_MAGIC + 0x808080u) ^ 0x808080u;
-          y[2 * e + 1] = (__float_as_uint(fmaf(b, inv, 12582912.f)) - (uint32_t)W4S_MAGIC + 0x808080u) ^ 0x808080u;
-        }
-        if (i0 + 32 * q < M * ng) {
-#pragma unroll
-          for (int d = 0; d < 3; ++d) {
-            const uint32_t sel = d | ((4 + d) << 4);
-            const uint32_t b0 = __byte_perm(__byte_perm(y[0], y[4], sel), __byte_perm(y[1], y[5], sel), 0x5410);
-            const uint32_t b1 = __byte_perm(__byte_perm(y[2], y[6], sel), __byte_perm(y[3], y[7], sel), 0x5410);
-            *reinterpret_cast<uint2*>(xq + (3 * m + d) * L.pitch + gl * 128 + 8 * l16) = make_uint2(b0, b1);
-          }
-          const float step = finite ? __uint_as_float((E - 24u) << 23) : __uint_as_float(0x7FC00000u);   // 2^(E - 127 - 20) / 16
-          if (l16 < (COMPACT ? 3 : 1))
-            sx[gl * ROWS + (COMPACT ? 3 * m + l16 : m)] = step * (l16 == 0 ? 1.f : (l16 == 1 ? 256.f : 65536.f));
-        }
+        *reinterpret_cast<uint4*>(w4s_smem + m * L.pitch + gl * 256 + 16 * l16) = u;
       }
     }
     __syncthreads();
 
     // ---- the stream
-    float acc[SETS][4];
-#pragma unroll
-    for (int n = 0; n < SETS; ++n)
-#pragma unroll
-      for (int c = 0; c < 4; ++c) acc[n][c] = 0.f;
+    float acc[4] = {0.f, 0.f, 0.f, 0.f};      // first column, x rows 2 t, 2 t + 1; second column
+    const unsigned char* xr = w4s_smem + gq * L.pitch + 16 * tq;
     int ci = 0;                               // consume cursor: unit of the tile
     uint32_t slot = 0;
     for (int it = 0; it < total; ++it) {
@@ -324,13 +271,7 @@ w4_stream_kernel(const W4StreamArgs p, const int tile_base, const int tiles, con
       if (ci < mine) {
         const unsigned char* sl = w4s_smem + L.ring + (warp * D + slot) * W4S_SLOT;
         const int gl = warp + W4S_WARPS * ci;
-        int dd[SETS][DIG][4];
-#pragma unroll
-        for (int n = 0; n < SETS; ++n)
-#pragma unroll
-          for (int q = 0; q < DIG; ++q)
-#pragma unroll
-            for (int c = 0; c < 4; ++c) dd[n][q][c] = W4S_MAGIC;
+        float d[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
           uint32_t w0, w1;
@@ -342,17 +283,9 @@ w4_stream_kernel(const W4StreamArgs p, const int tile_base, const int tiles, con
             w0 = w.x;
             w1 = w.y;
           }
-          const uint32_t a0 = w4s_lo(w0), a1 = w4s_lo(w1), a2 = w4s_hi(w0), a3 = w4s_hi(w1);
-#pragma unroll
-          for (int n = 0; n < SETS; ++n) {
-#pragma unroll
-            for (int q = 0; q < DIG; ++q) {
-              const int row = COMPACT ? gq : 3 * (8 * n + gq) + q;
-              const uint2 xb = row < 3 * M ? *reinterpret_cast<const uint2*>(xq + row * L.pitch + gl * 128 + 8 * (4 * j + tq))
-                                           : make_uint2(0u, 0u);
-              w4s_mma(dd[n][q], a0, a1, a2, a3, xb.x, xb.y);
-            }
-          }
+          const uint4 xv = gq < M ? *reinterpret_cast<const uint4*>(xr + gl * 256 + 64 * j) : make_uint4(0u, 0u, 0u, 0u);
+          w4s_mma(d, w4s_pair(w0, 0), w4s_pair(w1, 0), w4s_pair(w0, 1), w4s_pair(w1, 1), xv.x, xv.y);
+          w4s_mma(d, w4s_pair(w0, 2), w4s_pair(w1, 2), w4s_pair(w0, 3), w4s_pair(w1, 3), xv.z, xv.w);
         }
         float s0, s1;
         if (MODE == W4S_GATED) {
@@ -363,21 +296,10 @@ w4_stream_kernel(const W4StreamArgs p, const int tile_base, const int tiles, con
           s0 = bf16_lo(w);
           s1 = bf16_hi(w);
         }
-#pragma unroll
-        for (int n = 0; n < SETS; ++n) {
-          const float2 st = *reinterpret_cast<const float2*>(sx + gl * ROWS + 8 * n + 2 * tq);
-          float f[4];
-#pragma unroll
-          for (int c = 0; c < 4; ++c) {
-            f[c] = __int_as_float(dd[n][DIG - 1][c]) - 12582912.f;
-#pragma unroll
-            for (int q = DIG - 2; q >= 0; --q) f[c] = fmaf(f[c], 256.f, __int_as_float(dd[n][q][c]) - 12582912.f);
-          }
-          acc[n][0] = fmaf(f[0], s0 * st.x, acc[n][0]);            // first column, x columns 2 t, 2 t + 1
-          acc[n][1] = fmaf(f[1], s0 * st.y, acc[n][1]);
-          acc[n][2] = fmaf(f[2], s1 * st.x, acc[n][2]);            // second column
-          acc[n][3] = fmaf(f[3], s1 * st.y, acc[n][3]);
-        }
+        acc[0] = fmaf(d[0], s0, acc[0]);
+        acc[1] = fmaf(d[1], s0, acc[1]);
+        acc[2] = fmaf(d[2], s1, acc[2]);
+        acc[3] = fmaf(d[3], s1, acc[3]);
       }
       __syncwarp();                         // everyone has read the slot
       load(g0);
@@ -386,59 +308,56 @@ w4_stream_kernel(const W4StreamArgs p, const int tile_base, const int tiles, con
       // ---- tile done: hand this warp's sums over
       ci = 0;
       const int hb = handed & (W4S_NB - 1);
-      if (handed >= W4S_NB && !mbar_wait(&empty[hb], ((handed / W4S_NB) - 1) & 1, &abort_flag, err)) return;
-#pragma unroll
-      for (int n = 0; n < SETS; ++n) {
-        float* r = red + ((hb * W4S_WARPS + warp) * ROWS + 8 * n + 2 * tq) * W4S_TILE + 2 * gq;
-        *reinterpret_cast<float2*>(r) = make_float2(acc[n][0], acc[n][2]);
-        *reinterpret_cast<float2*>(r + W4S_TILE) = make_float2(acc[n][1], acc[n][3]);
-        acc[n][0] = acc[n][1] = acc[n][2] = acc[n][3] = 0.f;
+      if (handed >= W4S_NB && !mbar_wait(&empty[hb], ((handed / W4S_NB) - 1) & 1, &abort_flag, err)) {
+        cp_async_wait_all();
+        return;
       }
+      if (2 * tq < M) {
+        float* r = red + ((hb * W4S_WARPS + warp) * RP + 2 * tq) * W4S_TILE + 2 * gq;
+        *reinterpret_cast<float2*>(r) = make_float2(acc[0], acc[2]);
+        *reinterpret_cast<float2*>(r + W4S_TILE) = make_float2(acc[1], acc[3]);
+      }
+      acc[0] = acc[1] = acc[2] = acc[3] = 0.f;
       __syncwarp();
       if (lane == 0) mbar_arrive(&full[hb]);
       if (++handed > 2) epilogue(handed - 3);
     }
     cp_async_wait_all();
-    if (pass + 1 < passes) __syncthreads();   // every warp is done with the digits
+    if (pass + 1 < passes) __syncthreads();   // every warp is done with x
   }
   for (int q = max(handed - 2, 0); q < handed; ++q) epilogue(q);
 }
 
-// How a call is cut: scale groups per K pass and column tiles per launch. The digits of a pass stay in shared memory while the
-// CTA walks its tiles; K goes in passes when they do not all fit next to the rings and buffers. Partial sums then wait in
-// shared memory (at least W4S_PSUM_TILES tiles per CTA, or all of them), what does not fit goes to further launches.
+// How a call is cut: ring depth, scale groups per K pass, column tiles per launch. The rows of x of a pass stay in shared
+// memory while the CTA walks its tiles. Six groups in flight per warp while that leaves room for all of x, four otherwise;
+// K in passes when that is not enough either: partial sums then wait in shared memory (at least W4S_PSUM_TILES tiles per CTA,
+// or all of them), what does not fit goes to further launches.
 constexpr int W4S_PSUM_TILES = 8;
-struct W4SPlan { int pass_groups, tiles_per_cta; };             // tiles_per_cta: tiles of a launch per CTA, 0 = all at once
+struct W4SPlan { int depth, pass_groups, tiles_per_cta; };       // tiles_per_cta: tiles of a launch per CTA, 0 = all at once
 static bool w4s_plan(int M, int K, int tiles, int sms, bool norm, W4SPlan& out) {
-  const int rows = 8, depth = M <= 2 ? W4S_DEPTH<0> : W4S_DEPTH<1>, groups = K / 128;
-  auto bytes = [&](int pass_groups, int psum_tiles) { return w4s_layout(rows, depth, M, pass_groups, groups, norm, psum_tiles).total; };
-  if (bytes(groups, 0) <= W4S_SMEM) {
-    out = {groups, 0};
-    return true;
-  }
+  const int groups = K / 128;
+  for (int depth = 6; depth >= 4; depth -= 2)
+    if (w4s_layout(depth, M, groups, groups, norm, 0).total <= W4S_SMEM) {
+      out = {depth, groups, 0};
+      return true;
+    }
   const int all = (tiles + sms - 1) / sms, kept = all < W4S_PSUM_TILES ? all : W4S_PSUM_TILES;
-  const int fit = (W4S_SMEM - bytes(0, kept)) / (bytes(1, 0) - bytes(0, 0));
+  const int fit = (W4S_SMEM - w4s_layout(4, M, 0, groups, norm, kept).total) / (M * 256);
   if (fit < 1) return false;
   const int passes = (groups + fit - 1) / fit;
   int pass_groups = ((groups + passes - 1) / passes + W4S_WARPS - 1) / W4S_WARPS * W4S_WARPS;      // whole rounds of the warps
   if (pass_groups > fit) pass_groups = fit < W4S_WARPS ? fit : fit / W4S_WARPS * W4S_WARPS;
-  const int room = (W4S_SMEM - bytes(pass_groups, 0)) / (M * W4S_TILE * 4);
-  out = {pass_groups, room < all ? room : all};
+  const int room = (W4S_SMEM - w4s_layout(4, M, pass_groups, groups, norm, 0).total) / (M * W4S_TILE * 4);
+  out = {4, pass_groups, room < all ? room : all};
   return true;
 }
 
-template <int MT, int MODE>
-static int w4s_launch(const W4StreamArgs& a, cudaStream_t st) {
-  constexpr int ROWS = MT == 0 ? 8 : 8 * MT;
+template <int D, int MODE>
+static int w4s_launch(const W4StreamArgs& a, const W4SPlan& plan, int tiles, cudaStream_t st) {
   const int groups = a.K / 128;
-  const bool norm = a.gamma != nullptr;
-  const int tiles = MODE == W4S_GATED ? (a.N / 2 + 7) / 8 : (a.N + W4S_TILE - 1) / W4S_TILE;
-  W4SPlan plan;
-  SB_CHECK_ARG(w4s_plan(a.M, a.K, tiles, num_sms(), norm, plan));
-  const int pass_groups = plan.pass_groups, most = plan.tiles_per_cta > 0 ? plan.tiles_per_cta * num_sms() : tiles;
   unsigned int* err = error_word();
   if (!err) return SB_ERR_CUDA;
-  auto kern = w4_stream_kernel<MT, MODE>;
+  auto kern = w4_stream_kernel<D, MODE>;
   static bool attr_set[64] = {false};
   int dev = 0;
   SB_CHECK_CUDA(cudaGetDevice(&dev));
@@ -446,14 +365,15 @@ static int w4s_launch(const W4StreamArgs& a, cudaStream_t st) {
     SB_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, W4S_SMEM));
     attr_set[dev & 63] = true;
   }
+  const int most = plan.tiles_per_cta > 0 ? plan.tiles_per_cta * num_sms() : tiles;
   for (int t0 = 0; t0 < tiles; t0 += most) {
     const int nt = tiles - t0 < most ? tiles - t0 : most;
     const int grid = nt < num_sms() ? nt : num_sms();
-    const int psum_tiles = pass_groups < groups ? (nt + grid - 1) / grid : 0;
+    const int psum_tiles = plan.tiles_per_cta > 0 ? (nt + grid - 1) / grid : 0;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid, 1, 1);
     cfg.blockDim = dim3(W4S_THREADS, 1, 1);
-    cfg.dynamicSmemBytes = w4s_layout(ROWS, W4S_DEPTH<MT>, a.M, pass_groups, groups, norm, psum_tiles).total;
+    cfg.dynamicSmemBytes = w4s_layout(D, a.M, plan.pass_groups, groups, a.gamma != nullptr, psum_tiles).total;
     cfg.stream = st;
     cudaLaunchAttribute attr[1];
     // programmatic dependent launch: this grid may start while its predecessor in the stream still runs; before
@@ -462,7 +382,7 @@ static int w4s_launch(const W4StreamArgs& a, cudaStream_t st) {
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    SB_CHECK_CUDA(cudaLaunchKernelEx(&cfg, kern, a, t0, nt, pass_groups, psum_tiles, err));
+    SB_CHECK_CUDA(cudaLaunchKernelEx(&cfg, kern, a, t0, nt, plan.pass_groups, psum_tiles, err));
   }
   return SB_OK;
 }
@@ -472,32 +392,34 @@ bool w4_stream_one_pass(int M, int K) {
   return w4s_plan(M, K, 1, 1, false, plan) && plan.pass_groups == K / 128;
 }
 
+template <int MODE>
+static int w4s_planned(const W4StreamArgs& a, cudaStream_t st) {
+  const int tiles = MODE == W4S_GATED ? (a.N / 2 + 7) / 8 : (a.N + W4S_TILE - 1) / W4S_TILE;
+  W4SPlan plan;
+  SB_CHECK_ARG(w4s_plan(a.M, a.K, tiles, num_sms(), a.gamma != nullptr, plan));
+  return plan.depth == 6 ? w4s_launch<6, MODE>(a, plan, tiles, st) : w4s_launch<4, MODE>(a, plan, tiles, st);
+}
+
 int launch_w4_stream(const W4StreamArgs& a, W4StreamMode mode, cudaStream_t st) {
-  SB_CHECK_ARG(a.M >= 1 && a.M <= W4S_MAX_ROWS && a.K > 0 && a.K % 128 == 0 && a.N > 0 && a.N % 4 == 0 && a.ldx % 8 == 0);
+  SB_CHECK_ARG(a.M >= 1 && a.M <= (mode == W4S_PLAIN ? W4S_MAX_ROWS : 4) && a.K > 0 && a.K % 128 == 0 && a.N > 0 && a.N % 4 == 0 && a.ldx % 8 == 0);
   SB_CHECK_ARG(((reinterpret_cast<uintptr_t>(a.wk8) | reinterpret_cast<uintptr_t>(a.x)) & 15) == 0 && (reinterpret_cast<uintptr_t>(a.scales) & 7) == 0);
   if (mode == W4S_GATED) {
-    SB_CHECK_ARG(a.M <= 8 && a.N % 8 == 0);
-    return a.M <= 2 ? w4s_launch<0, W4S_GATED>(a, st) : w4s_launch<1, W4S_GATED>(a, st);
+    SB_CHECK_ARG(a.N % 8 == 0);
+    return w4s_planned<W4S_GATED>(a, st);
   }
-  if (mode == W4S_ROPE) {
-    SB_CHECK_ARG(a.M <= 8);
-    return a.M <= 2 ? w4s_launch<0, W4S_ROPE>(a, st) : w4s_launch<1, W4S_ROPE>(a, st);
-  }
-  if (a.M <= 2) return w4s_launch<0, W4S_PLAIN>(a, st);
-  return w4s_launch<1, W4S_PLAIN>(a, st);
+  return mode == W4S_ROPE ? w4s_planned<W4S_ROPE>(a, st) : w4s_planned<W4S_PLAIN>(a, st);
 }
 
 }  // namespace sb
 
 // Host check of the cut of a call on a GPU of `sms` SMs: dynamic shared memory of its largest launch in bytes, -1 when the call
-// would be refused. passes receives the number of K passes.
+// would be refused. passes (may be null) receives the number of K passes.
 extern "C" int sb_w4_stream_smem(int M, int N, int K, int norm, int sms, int* passes) {
   using namespace sb;
-  const int groups = K / 128;
+  const int groups = K / 128, tiles = (N + W4S_TILE - 1) / W4S_TILE;
   W4SPlan plan;
-  if (!w4s_plan(M, K, (N + W4S_TILE - 1) / W4S_TILE, sms, norm != 0, plan)) return -1;
-  *passes = (groups + plan.pass_groups - 1) / plan.pass_groups;
-  if (*passes > 1 && plan.tiles_per_cta < 1) return -1;
-  const int bytes = w4s_layout(8, M <= 2 ? W4S_DEPTH<0> : W4S_DEPTH<1>, M, plan.pass_groups, groups, norm != 0, plan.tiles_per_cta).total;
-  return bytes <= W4S_SMEM ? bytes : -1;
+  if (!w4s_plan(M, K, tiles, sms, norm != 0, plan)) return -1;
+  if (passes) *passes = (groups + plan.pass_groups - 1) / plan.pass_groups;
+  const int bytes = w4s_layout(plan.depth, M, plan.pass_groups, groups, norm != 0, plan.tiles_per_cta).total;
+  return bytes <= W4S_SMEM && plan.tiles_per_cta >= (plan.pass_groups < groups ? 1 : 0) ? bytes : -1;
 }

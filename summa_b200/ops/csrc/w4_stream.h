@@ -34,7 +34,7 @@ struct W4StreamArgs {
 };
 
 constexpr int W4S_MAX_ROWS = 8;
-// Whether the digits of x fit shared memory at once (otherwise K is walked in passes, each with its own staging).
+// Whether the rows of x fit shared memory at once (otherwise K is walked in passes, each with its own staging).
 bool w4_stream_one_pass(int M, int K);
 int launch_w4_stream(const W4StreamArgs& a, W4StreamMode mode, cudaStream_t st);
 

@@ -1209,8 +1209,8 @@ N.register("sb_w4_gemv_small", [N.P] * 5 + [N.I, N.I, N.I, N.L, N.P])
 N.register("sb_w4_gemv_cluster", [N.P] * 5 + [N.I, N.I, N.I, N.L, N.P, N.F, N.P])
 N.register("sb_w4_gemv_mma", [N.P] * 5 + [N.I, N.I, N.I, N.L, N.P, N.F, N.P])
 N.register("sb_w4_gemv_stream", [N.P] * 5 + [N.I, N.I, N.I, N.L, N.P, N.F, N.I, N.P])
-# "cluster" (default): the streaming integer-mma kernel (w4_stream.cu); "mma" / "stream": the older bf16-mma forms, which
-# expand every code to bf16 (slower at every decode shape; kept as independent implementations for the tests).
+# "cluster" (default; the name of the form it replaced): the streaming kernel (w4_stream.cu); "mma" / "stream": older forms
+# (slower at every decode shape; kept as independent implementations for the tests).
 W4_GEMV_KERNEL = os.environ.get("SUMMA_W4_GEMV", "cluster")
 N.register("sb_w4_gemv_cluster_swiglu", [N.P] * 4 + [N.I, N.I, N.I, N.L, N.P, N.F, N.P])
 
@@ -1263,7 +1263,7 @@ def int4_gemv_swiglu(x, packed_k8, scales, norm=None):
 
 def int4_gemv(x, packed, scales, residual=None, packed_k8=None, norm=None):
     """x `[M <= 64, K]` @ dequant(W) (+ residual). With the repacked weight (`reference.repack_int4_k8`)
-    the product runs on the streaming integer-mma kernel (few rows) or the tcgen05 W4A16 kernel;
+    the product runs on the streaming kernel (few rows) or the tcgen05 W4A16 kernel;
     otherwise on the CUDA-core weight-streaming kernel. `norm=(gamma fp32 [K], eps)` applies RMSNorm
     to x first (fused into the GEMV for M <= 4)."""
     M, K = x.shape

@@ -36,31 +36,60 @@ def test_w4_stream_cuts_every_k_to_fit_shared_memory(M, norm):
     (8, 4736, 52), (5, 14336, 40)])                                                 # rows 5..8 beyond one pass: the other kernel
 @pytest.mark.parametrize("spread", [0, 24])
 def test_w4_projection_against_fp64(M, K, N, spread):
-    """x spreads over 2^-spread .. 1: a group's fixed-point step is 2^-21 of its largest magnitude, so a product is off by at
-    most 2^-21 max|x| |w| per term, next to fp32 sums (2^-20 of the terms' sum is above both) and one rounding to bf16."""
+    """x spreads over 2^-spread .. 1. Exact products, fp32 sums (2^-18 of the terms' sum) and one rounding to bf16."""
+    import ctypes
     from summa_b200 import ops
+    from summa_b200.ops import native
     packed, scales, k8, wq = _w4(K, N, M + K + N)
     x = (torch.randn(M, K, device="cuda") * torch.exp2(-spread * torch.rand(M, K, device="cuda"))).to(torch.bfloat16)
     res = torch.randn(M, N, device="cuda").to(torch.bfloat16)
     ref = x.double() @ wq
-    big = x.double().view(M, K // 128, 128).abs().amax(-1, keepdim=True).expand(M, K // 128, 128).reshape(M, K)
-    slack = 2.0 ** -20 * (big @ wq.abs())
-    if M > 4 and 3 * M * K > 104 * 1024:                                            # that kernel rounds the weights to bf16
-        slack += 2.0 ** -9 * (x.double().abs() @ wq.abs())
+    passes = ctypes.c_int(0)
+    native.lib().sb_w4_stream_smem(M, N, K, 0, 148, ctypes.byref(passes))
+    # rows 5..8 beyond one pass: that kernel rounds the weights to bf16
+    slack = (2.0 ** -9 if M > 4 and passes.value > 1 else 2.0 ** -18) * (x.double().abs() @ wq.abs())
     for got, want in ((ops.int4_gemv(x, packed, scales, None, k8), ref), (ops.int4_gemv(x, packed, scales, res, k8), ref + res.double())):
         assert bool(((got.double() - want).abs() <= 2.0 ** -8 * want.abs() + slack + 1e-30).all())
 
 
 @gpu
-def test_w4_projection_keeps_nan_and_inf_in_their_row():
+@pytest.mark.parametrize("M,N", [(1, 36), (2, 16), (4, 52), (8, 20)])
+@pytest.mark.parametrize("big", [12, 40])
+def test_w4_projection_keeps_small_elements_beside_an_outlier(M, N, big):
+    """One element of a scale group is 2^big, its weights are zero: the columns are what the other elements make of them, at
+    the same precision (exact products, fp32 sums: 2^-18 of the terms' sum, one rounding to bf16)."""
+    from summa_b200 import ops
+    from summa_b200.ops import reference
+    torch.manual_seed(M + N)
+    w = torch.randn(512, N) * 0.05
+    w[5::128] = 0
+    packed, scales = reference.quantize_int4_g128(w)
+    wq = reference.dequantize_int4_g128(packed, scales).double().cuda()
+    assert float(wq[5::128].abs().max()) == 0
+    packed, scales = packed.cuda(), scales.cuda()
+    x = torch.randn(M, 512, device="cuda")
+    x[:, 5::128] = 2.0 ** big
+    x = x.to(torch.bfloat16)
+    ref = x.double() @ wq
+    got = ops.int4_gemv(x, packed, scales, None, reference.repack_int4_k8(packed))
+    assert bool(((got.double() - ref).abs() <= 2.0 ** -8 * ref.abs() + 2.0 ** -18 * (x.double().abs() @ wq.abs())).all())
+
+
+@gpu
+@pytest.mark.parametrize("M", [4, 8])
+def test_w4_projection_keeps_nan_and_inf_in_their_row(M):
+    """An infinite element makes a column infinite, of the sign of its weight, or NaN where that is zero, and a NaN makes the row
+    NaN, as IEEE sums do; the other rows do not see either."""
     from summa_b200 import ops
     packed, scales, k8, wq = _w4(512, 40, 3)
-    x = torch.randn(4, 512, device="cuda").to(torch.bfloat16)
+    x = torch.randn(M, 512, device="cuda").to(torch.bfloat16)
     clean = ops.int4_gemv(x, packed, scales, None, k8)
     x[1, 7], x[2, 300] = float("inf"), float("nan")
     got = ops.int4_gemv(x, packed, scales, None, k8)
-    assert bool(got[1].isnan().all()) and bool(got[2].isnan().all())
-    assert torch.equal(got[0], clean[0]) and torch.equal(got[3], clean[3])
+    torch.testing.assert_close(got[1].float(), float("inf") * wq[7].float(), rtol=0, atol=0, equal_nan=True)
+    assert bool((wq[7] == 0).any()) and bool(got[2].isnan().all())
+    for m in (0, *range(3, M)):
+        assert torch.equal(got[m], clean[m])
 
 
 @gpu
