@@ -203,9 +203,9 @@ class _GraphDecoder:
         cs = (ctypes.c_long * 3)(st.k.stride(0), st.k.stride(1), st.k.stride(2))
         if self._rope_fusable(blk, h):
             from ..ops import cuda_ops
-            qkv = cuda_ops.int4_gemv_rope_append(h, a.qkv_proj.packed_k8(), a.qkv_proj.scales,
-                                                 (blk.attn_norm.gamma, blk.attn_norm.eps), cos, sin, st.k, st.v,
-                                                 self.pos, a.num_heads, a.num_kv_heads, a.head_dim, self.cap)
+            k8, scales, settled = a.qkv_proj.decode_operands()
+            qkv = cuda_ops.int4_gemv_rope_append(h, k8, scales, (blk.attn_norm.gamma, blk.attn_norm.eps), cos, sin, st.k, st.v,
+                                                 self.pos, a.num_heads, a.num_kv_heads, a.head_dim, self.cap, settled)
         else:
             qkv = self._norm_proj(blk.attn_norm, a.qkv_proj, h)
             native.call("sb_decode_rope_append", qkv.data_ptr(), cos.data_ptr(), sin.data_ptr(), st.k.data_ptr(),

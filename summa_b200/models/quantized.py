@@ -40,11 +40,24 @@ class QuantLinear(nn.Module):
         self.register_buffer("scales", scales.contiguous())
         self.register_buffer("bias", bias)
         self._k8 = None           # repacked copy for the tensor-core decode kernel (built on first use)
+        self._scales8 = None      # aligned copy of scales that start off an 8-byte boundary (built on first use)
 
     def packed_k8(self) -> torch.Tensor:
         if self._k8 is None or self._k8.device != self.packed.device:
             self._k8 = reference.repack_int4_k8(self.packed)
         return self._k8
+
+    def decode_operands(self):
+        """(codes, scales, settled) for the decode kernels: the repacked codes, the scales on the 8-byte boundary that those need
+        (a view that starts elsewhere is copied once, here), and whether both were there before this call, i.e. nothing in
+        flight writes them."""
+        settled = self._k8 is not None and self._k8.device == self.packed.device
+        k8, scales = self.packed_k8(), self.scales
+        if scales.is_cuda and scales.data_ptr() % 8:
+            if self._scales8 is None or self._scales8.device != scales.device:
+                self._scales8, settled = scales.clone(), False
+            scales = self._scales8
+        return k8, scales, settled
 
     @staticmethod
     def from_linear(lin: Linear) -> "QuantLinear":
@@ -65,10 +78,11 @@ class QuantLinear(nn.Module):
         x2 = x.reshape(-1, self.d_in)
         if x2.is_cuda and x2.dtype == torch.bfloat16:
             if x2.shape[0] <= 64:
+                k8, scales, settled = self.decode_operands()
                 if residual is not None and self.bias is None:
-                    return ops.int4_gemv(x2, self.packed, self.scales, residual.reshape(-1, self.d_out),
-                                         self.packed_k8(), norm).view(*lead, self.d_out)
-                y = ops.int4_gemv(x2, self.packed, self.scales, None, self.packed_k8(), norm)
+                    return ops.int4_gemv(x2, self.packed, scales, residual.reshape(-1, self.d_out), k8, norm,
+                                         settled).view(*lead, self.d_out)
+                y = ops.int4_gemv(x2, self.packed, scales, None, k8, norm, settled)
             else:
                 if norm is not None:
                     x2 = ops.rmsnorm(x2, norm[0], norm[1])
@@ -103,7 +117,8 @@ def in_proj_swiglu(lin, x: torch.Tensor, norm=None) -> torch.Tensor:
     x2 = x.reshape(-1, x.shape[-1])
     if _swiglu_fusable(lin, x2):
         from ..ops import cuda_ops
-        return cuda_ops.int4_gemv_swiglu(x2, lin.packed_k8(), lin.scales, norm).view(*x.shape[:-1], lin.d_out // 2)
+        k8, scales, settled = lin.decode_operands()
+        return cuda_ops.int4_gemv_swiglu(x2, k8, scales, norm, settled).view(*x.shape[:-1], lin.d_out // 2)
     if norm is not None:
         u = lin(x, norm=norm) if isinstance(lin, QuantLinear) else lin(ops.rmsnorm(x, norm[0], norm[1]))
     else:

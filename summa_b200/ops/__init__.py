@@ -269,12 +269,13 @@ def linear_cross_entropy(hidden, weight, bias, targets, vocab_size, chunks=4):
     return reference.linear_cross_entropy(hidden, weight, bias, targets, vocab_size, chunks)
 
 
-def int4_gemv(x, packed, scales, residual=None, packed_k8=None, norm=None):
+def int4_gemv(x, packed, scales, residual=None, packed_k8=None, norm=None, static_w=False):
     """x `[M<=64, K]` bf16 @ dequant(packed `[K/2, N]`, scales `[K/128, N]`) → `[M, N]` bf16.
     `packed_k8` (`reference.repack_int4_k8(packed)`) selects the tensor-core kernel (M > 4) or the
-    one-launch weight-streaming kernel (few rows) on CUDA; `norm=(gamma, eps)` applies RMSNorm to x first."""
+    one-launch weight-streaming kernel (few rows) on CUDA; `norm=(gamma, eps)` applies RMSNorm to x first.
+    `static_w`: no work in flight on the stream writes `packed_k8` or `scales` (the kernel may then read them early)."""
     if x.is_cuda:
-        return _cu().int4_gemv(x, packed, scales, residual, packed_k8, norm)
+        return _cu().int4_gemv(x, packed, scales, residual, packed_k8, norm, static_w)
     if norm is not None:
         x = rmsnorm(x, norm[0], norm[1])
     y = reference.int4_linear(x, packed, scales)

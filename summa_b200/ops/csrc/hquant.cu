@@ -478,12 +478,11 @@ w4_gemv_cluster_kernel(const __nv_bfloat16* __restrict__ x, const uint32_t* __re
       else w[r][0] = __ldcs(p);
     }
   };
-  // The weights do not depend on the preceding kernel: under programmatic dependent launch the first
-  // group is already on its way while that kernel finishes; x is only read after the wait.
+  // The weights may have been repacked or copied by the preceding kernel: nothing is read before the wait.
+  asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;");
   int g = g_lo + warp;
   if (live && g < g_hi) load_group(wcur, g);
-  asm volatile("griddepcontrol.wait;" ::: "memory");
   // the previous call of this kernel has completed (and bumped the call number) once the wait returns
   const uint32_t ar_epoch = ar.world > 1 ? *reinterpret_cast<volatile unsigned int*>(ar.epoch_word) + 1u : 0u;
   // ---- stage my slice of x
@@ -665,23 +664,25 @@ static int launch_w4_cluster(const void* x, const void* wk8, const void* scales,
 
 }  // namespace sb
 
-// y[M,N] bf16 = x[M,K] @ dequant(k8-repacked int4 g128 weights) (+ residual), M <= 4, on the streaming kernel
+// y[M,N] bf16 = x[M,K] @ dequant(k8-repacked int4 g128 weights) (+ residual), M <= 8, on the streaming kernel
 // (w4_stream.cu). gamma (fp32 [K]) != null fuses y = rmsnorm(x; gamma, eps) @ W. x and wk8 16-byte, scales 8-byte aligned.
+// static_w != 0: nothing in flight on the stream writes wk8 or scales (they may be read before the preceding kernel is done).
 extern "C" int sb_w4_gemv_cluster(const void* x, const void* wk8, const void* scales, const void* residual, void* y,
-                                  int M, int N, int K, long ldx, const float* gamma, float eps, cudaStream_t st) {
-  SB_CHECK_ARG(M >= 1 && M <= 4 && K > 0 && K % 128 == 0 && N > 0 && N % 4 == 0 && ldx % 8 == 0);
+                                  int M, int N, int K, long ldx, const float* gamma, float eps, int static_w,
+                                  cudaStream_t st) {
+  SB_CHECK_ARG(M >= 1 && M <= sb::W4S_MAX_ROWS && K > 0 && K % 128 == 0 && N > 0 && N % 4 == 0 && ldx % 8 == 0);
   const sb::W4StreamArgs a = {(const __nv_bfloat16*)x, (const uint32_t*)wk8, (const __nv_bfloat16*)scales,
-                              (const __nv_bfloat16*)residual, (__nv_bfloat16*)y, M, N, K, ldx, gamma, eps, {}};
+                              (const __nv_bfloat16*)residual, (__nv_bfloat16*)y, M, N, K, ldx, gamma, eps, static_w, {}};
   return sb::launch_w4_stream(a, sb::W4S_PLAIN, st);
 }
 
 // y[M, I] = silu(g) * v with [g | v] = (rmsnorm(x) or x) @ dequant(W[K, 2I]): the gated in-projection of a
 // decode step, activation included. M <= 4, K % 128 == 0, I % 4 == 0.
 extern "C" int sb_w4_gemv_cluster_swiglu(const void* x, const void* wk8, const void* scales, void* y, int M, int N,
-                                         int K, long ldx, const float* gamma, float eps, cudaStream_t st) {
+                                         int K, long ldx, const float* gamma, float eps, int static_w, cudaStream_t st) {
   SB_CHECK_ARG(M >= 1 && M <= 4 && K > 0 && K % 128 == 0 && N > 0 && N % 8 == 0 && ldx % 8 == 0);
   const sb::W4StreamArgs a = {(const __nv_bfloat16*)x, (const uint32_t*)wk8, (const __nv_bfloat16*)scales, nullptr,
-                              (__nv_bfloat16*)y, M, N, K, ldx, gamma, eps, {}};
+                              (__nv_bfloat16*)y, M, N, K, ldx, gamma, eps, static_w, {}};
   return sb::launch_w4_stream(a, sb::W4S_GATED, st);
 }
 
@@ -691,7 +692,7 @@ extern "C" int sb_w4_gemv_cluster_swiglu(const void* x, const void* wk8, const v
 extern "C" int sb_w4_gemv_cluster_rope(const void* x, const void* wk8, const void* scales, void* y, int M, int N, int K,
                                        long ldx, const float* gamma, float eps, const float* cos_t, const float* sin_t,
                                        void* k_cache, void* v_cache, const int* pos_ptr, int Hq, int Hkv, int D,
-                                       const long* cache_strides, int cap, cudaStream_t st) {
+                                       const long* cache_strides, int cap, int static_w, cudaStream_t st) {
   SB_CHECK_ARG(M >= 1 && M <= 4 && K > 0 && K % 128 == 0 && N == (Hq + 2 * Hkv) * D && D % 2 == 0 && ldx % 8 == 0);
   SB_CHECK_ARG(cos_t && sin_t && k_cache && v_cache && pos_ptr && cap > 0);
   sb::RopeAppend r;
@@ -699,7 +700,7 @@ extern "C" int sb_w4_gemv_cluster_rope(const void* x, const void* wk8, const voi
   r.Hq = Hq; r.Hkv = Hkv; r.D = D; r.cap = cap;
   r.c_sb = cache_strides[0]; r.c_ss = cache_strides[1]; r.c_sh = cache_strides[2];
   const sb::W4StreamArgs a = {(const __nv_bfloat16*)x, (const uint32_t*)wk8, (const __nv_bfloat16*)scales, nullptr,
-                              (__nv_bfloat16*)y, M, N, K, ldx, gamma, eps, r};
+                              (__nv_bfloat16*)y, M, N, K, ldx, gamma, eps, static_w, r};
   return sb::launch_w4_stream(a, sb::W4S_ROPE, st);
 }
 
@@ -764,10 +765,10 @@ w4_gemv_mma_kernel(const __nv_bfloat16* __restrict__ x, const uint32_t* __restri
     for (int j = 0; j < 4; ++j)
       w[j] = live ? __ldcs(reinterpret_cast<const uint4*>(wk8 + (long)(16 * g + 4 * j + tq) * N + cb)) : make_uint4(0u, 0u, 0u, 0u);
   };
+  asm volatile("griddepcontrol.wait;" ::: "memory");       // (the weights may come from the preceding kernel too)
   asm volatile("griddepcontrol.launch_dependents;");
   int g = g_lo + warp;
   if (g < g_hi) load_group(wc, g);
-  asm volatile("griddepcontrol.wait;" ::: "memory");
   // ---- stage the M rows of x, optional fused RMSNorm, per-group sums
   for (int i = threadIdx.x; i < M * k8n; i += WM_WARPS * 32) {
     const int m = i / k8n, c = i - m * k8n;
@@ -1001,10 +1002,10 @@ w4_gemv_stream_kernel(const __nv_bfloat16* __restrict__ x, const uint32_t* __res
     }
     cp_async_commit();
   };
+  asm volatile("griddepcontrol.wait;" ::: "memory");       // (the weights may come from the preceding kernel too)
   asm volatile("griddepcontrol.launch_dependents;");
 #pragma unroll
   for (int q = 0; q < WP_STAGES - 1; ++q) issue();
-  asm volatile("griddepcontrol.wait;" ::: "memory");
   // ---- stage x once per CTA, optional fused RMSNorm, per-group sums
   const int k8n = K >> 3;
   for (int i = threadIdx.x; i < MR * k8n; i += WP_WARPS * 32) {

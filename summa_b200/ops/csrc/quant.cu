@@ -757,12 +757,10 @@ extern "C" int sb_w4a16_gemm(const void* x, const void* packed_k8, const void* s
   SB_CHECK_ARG(M >= 1 && K % 128 == 0 && N % 4 == 0 && N > 0 && ldx % 8 == 0);
   SB_CHECK_ARG((reinterpret_cast<uintptr_t>(x) & 15) == 0 && (reinterpret_cast<uintptr_t>(packed_k8) & 15) == 0);
   (void)acc;
-  // Up to 8 rows the streaming kernel is ahead as long as x fits its shared memory in one pass (M 8, K 4096: N 28672
-  // 28.6 us against 48.4, N 6144 10.8 against 17.6; M 4, K 14336, N 4096: 18.2 us against 20.3). From 9 rows on it would need
-  // a second set of mma columns.
-  if (M <= 4 || (M <= W4S_MAX_ROWS && w4_stream_one_pass(M, K))) {
+  // (not static_w: the caller says nothing about where the weights come from)
+  if (w4_stream_preferred(M, K)) {
     const W4StreamArgs a = {(const __nv_bfloat16*)x, (const uint32_t*)packed_k8, (const __nv_bfloat16*)scales,
-                            (const __nv_bfloat16*)residual, (__nv_bfloat16*)y, M, N, K, ldx, nullptr, 0.f, {}};
+                            (const __nv_bfloat16*)residual, (__nv_bfloat16*)y, M, N, K, ldx, nullptr, 0.f, 0, {}};
     return launch_w4_stream(a, W4S_PLAIN, st);
   }
   if (M <= 64) return launch_w4a16<64, W4A16_GROUPS>(x, packed_k8, scales, residual, y, M, N, K, ldx, st);

@@ -18,7 +18,7 @@
 //   * per tile every warp leaves its partial sums in one of four shared-memory buffers and streams on; the warp whose
 //     turn it is adds them and runs the epilogue two tiles later (mbarriers both ways). With one block barrier and an
 //     immediate epilogue per tile its latency was paid per tile. No cluster, no atomics.
-//   * the weights depend on nothing, so the first groups are requested before `griddepcontrol.wait`.
+//   * weights that nothing in flight writes (`static_w`) are requested before `griddepcontrol.wait`.
 // Measured against the CUDA-core cluster kernel it replaces (weights from HBM, graph of launches, one row): K 4096 N 6144
 // 12.0 -> 7.4 us, N 4096 7.4 -> 5.8, N 28672 29.0 -> 18.9 (gated with norm 32.9 -> 21.3), N 32000 30.2 -> 21.2, K 14336 N 4096
 // 19.8 -> 13.0; four rows: 20.0 -> 9.2, 14.6 -> 7.4, 60.6 -> 26.2, 66.4 -> 29.0, 41.9 -> 18.2. Error of the sums against 64 bits
@@ -91,6 +91,9 @@ w4_stream_kernel(const W4StreamArgs p, const int tile_base, const int tiles, con
   extern __shared__ __align__(128) unsigned char w4s_smem[];
   __shared__ uint64_t full[W4S_NB], empty[W4S_NB];
   __shared__ int abort_flag;
+  // Weights that the preceding kernel may have written are only visible behind the wait; and a following launch, which may
+  // take them for settled, only starts once every CTA here has passed it.
+  if (!p.static_w) asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;");
   const int M = p.M, N = p.N, K = p.K, RP = DIGITS ? 8 : (p.M + 1) & ~1;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gq = lane >> 2, tq = lane & 3;
@@ -511,7 +514,7 @@ static int w4s_launch(const W4StreamArgs& a, const W4SPlan& plan, int tiles, cud
     cfg.stream = st;
     cudaLaunchAttribute attr[1];
     // programmatic dependent launch: this grid may start while its predecessor in the stream still runs; before
-    // `griddepcontrol.wait` it only reads weights, and it writes nothing
+    // `griddepcontrol.wait` it reads weights at most (static_w), and it writes nothing
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
@@ -521,9 +524,9 @@ static int w4s_launch(const W4StreamArgs& a, const W4SPlan& plan, int tiles, cud
   return SB_OK;
 }
 
-bool w4_stream_one_pass(int M, int K) {
+bool w4_stream_preferred(int M, int K) {
   W4SPlan plan;
-  return w4s_plan(M, K, 1, 1, false, plan) && plan.pass_groups == K / 128;
+  return M <= 4 || (M <= W4S_MAX_ROWS && w4s_plan(M, K, 1, 1, false, plan) && plan.pass_groups == K / 128);
 }
 
 template <int MODE>
@@ -547,6 +550,8 @@ int launch_w4_stream(const W4StreamArgs& a, W4StreamMode mode, cudaStream_t st) 
 }
 
 }  // namespace sb
+
+extern "C" int sb_w4_stream_preferred(int M, int K) { return sb::w4_stream_preferred(M, K) ? 1 : 0; }
 
 // Host check of the cut of a call on a GPU of `sms` SMs: dynamic shared memory of its largest launch in bytes, -1 when the call
 // would be refused. passes (may be null) receives the number of K passes.

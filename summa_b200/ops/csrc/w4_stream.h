@@ -30,12 +30,15 @@ struct W4StreamArgs {
   long ldx;
   const float* gamma;              // fp32 [K]: y = rmsnorm(x; gamma, eps) @ W; null = no norm
   float eps;
+  int static_w;                    // nothing in flight on the stream writes codes or scales: they may be requested early
   RopeAppend rope;                 // W4S_ROPE only
 };
 
 constexpr int W4S_MAX_ROWS = 8;
-// Whether the rows of x fit shared memory at once (otherwise K is walked in passes, each with its own staging).
-bool w4_stream_one_pass(int M, int K);
+// Whether this kernel is ahead of the tcgen05 one (sb_w4a16_gemm). Up to 8 rows as long as x fits its shared memory in one pass
+// (M 8, K 4096: N 28672 28.6 us against 48.4, N 6144 10.8 against 17.6; M 4, K 14336, N 4096: 18.2 us against 20.3; otherwise K
+// is walked in passes, each with its own staging). From 9 rows on it would need a second set of mma columns.
+bool w4_stream_preferred(int M, int K);
 int launch_w4_stream(const W4StreamArgs& a, W4StreamMode mode, cudaStream_t st);
 
 }  // namespace sb

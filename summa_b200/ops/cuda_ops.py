@@ -1206,25 +1206,28 @@ N.register("sb_argmax_rows", [N.P, N.P, N.I, N.I, N.L, N.I, N.P])
 
 N.register("sb_w4a16_gemm", [N.P] * 6 + [N.I, N.I, N.I, N.L, N.P])
 N.register("sb_w4_gemv_small", [N.P] * 5 + [N.I, N.I, N.I, N.L, N.P])
-N.register("sb_w4_gemv_cluster", [N.P] * 5 + [N.I, N.I, N.I, N.L, N.P, N.F, N.P])
+N.register("sb_w4_stream_preferred", [N.I, N.I])
+N.register("sb_w4_gemv_cluster", [N.P] * 5 + [N.I, N.I, N.I, N.L, N.P, N.F, N.I, N.P])
 N.register("sb_w4_gemv_mma", [N.P] * 5 + [N.I, N.I, N.I, N.L, N.P, N.F, N.P])
 N.register("sb_w4_gemv_stream", [N.P] * 5 + [N.I, N.I, N.I, N.L, N.P, N.F, N.I, N.P])
 # "cluster" (default; the name of the form it replaced): the streaming kernel (w4_stream.cu); "mma" / "stream": older forms
 # (slower at every decode shape; kept as independent implementations for the tests).
 W4_GEMV_KERNEL = os.environ.get("SUMMA_W4_GEMV", "cluster")
-N.register("sb_w4_gemv_cluster_swiglu", [N.P] * 4 + [N.I, N.I, N.I, N.L, N.P, N.F, N.P])
+N.register("sb_w4_gemv_cluster_swiglu", [N.P] * 4 + [N.I, N.I, N.I, N.L, N.P, N.F, N.I, N.P])
 
 
-N.register("sb_w4_gemv_cluster_rope", [N.P] * 4 + [N.I, N.I, N.I, N.L, N.P, N.F] + [N.P] * 5 + [N.I, N.I, N.I, N.P, N.I, N.P])
+N.register("sb_w4_gemv_cluster_rope", [N.P] * 4 + [N.I, N.I, N.I, N.L, N.P, N.F] + [N.P] * 5 + [N.I, N.I, N.I, N.P, N.I, N.I, N.P])
 
 
-def _w4_operands(packed_k8: torch.Tensor, scales: torch.Tensor):
-    """The streaming kernel copies codes in 16-byte and scales in 8-byte pieces; a view that starts elsewhere is copied."""
-    return (packed_k8 if packed_k8.data_ptr() % 16 == 0 else packed_k8.clone(),
-            scales if scales.data_ptr() % 8 == 0 else scales.clone())
+def _w4_operands(packed_k8: torch.Tensor, scales: torch.Tensor, static_w: bool):
+    """The streaming kernel copies codes in 16-byte and scales in 8-byte pieces; a view that starts elsewhere is copied, and then
+    is not `static_w` any more: the copy is still in flight."""
+    if packed_k8.data_ptr() % 16 or scales.data_ptr() % 8:
+        return packed_k8.clone(), scales.clone(), 0
+    return packed_k8, scales, int(static_w)
 
 
-def int4_gemv_rope_append(x, packed_k8, scales, norm, cos, sin, k_cache, v_cache, pos, Hq, Hkv, D, cap):
+def int4_gemv_rope_append(x, packed_k8, scales, norm, cos, sin, k_cache, v_cache, pos, Hq, Hkv, D, cap, static_w=False):
     """The qkv projection of a decode step (x `[M <= 4, K]`, optional fused RMSNorm) with interleaved RoPE at the
     device-side position `pos` (int32 tensor) and the append of k / v to the caches in its epilogue. Returns
     `[M, (Hq + 2 Hkv) D]` whose q part is rotated (its k / v parts are not written)."""
@@ -1236,15 +1239,15 @@ def int4_gemv_rope_append(x, packed_k8, scales, norm, cos, sin, k_cache, v_cache
         x2 = rmsnorm(x2, norm[0], norm[1])
         ldx = x2.stride(0)
     y = torch.empty(M, Nn, device=x.device, dtype=BF16)
-    packed_k8, scales = _w4_operands(packed_k8, scales)
+    packed_k8, scales, static_w = _w4_operands(packed_k8, scales, static_w)
     cs = (ctypes.c_long * 3)(k_cache.stride(0), k_cache.stride(1), k_cache.stride(2))
     N.call("sb_w4_gemv_cluster_rope", x2.data_ptr(), packed_k8.data_ptr(), scales.data_ptr(), y.data_ptr(), M, Nn, K,
            ldx, norm[0].data_ptr() if fuse else None, float(norm[1]) if fuse else 0.0, cos.data_ptr(), sin.data_ptr(),
-           k_cache.data_ptr(), v_cache.data_ptr(), pos.data_ptr(), Hq, Hkv, D, cs, cap, N.stream())
+           k_cache.data_ptr(), v_cache.data_ptr(), pos.data_ptr(), Hq, Hkv, D, cs, cap, static_w, N.stream())
     return y
 
 
-def int4_gemv_swiglu(x, packed_k8, scales, norm=None):
+def int4_gemv_swiglu(x, packed_k8, scales, norm=None, static_w=False):
     """silu(g) * v with [g | v] = (rmsnorm(x) or x) @ dequant(W `[K, 2I]`), x `[M <= 4, K]` -> `[M, I]`:
     the gated in-projection of a decode step in one launch."""
     M, K = x.shape
@@ -1254,25 +1257,26 @@ def int4_gemv_swiglu(x, packed_k8, scales, norm=None):
     if norm is not None and not fuse:
         x2 = rmsnorm(x2, norm[0], norm[1])
         ldx = x2.stride(0)
-    packed_k8, scales = _w4_operands(packed_k8, scales)
+    packed_k8, scales, static_w = _w4_operands(packed_k8, scales, static_w)
     y = torch.empty(M, Nn // 2, device=x.device, dtype=BF16)
     N.call("sb_w4_gemv_cluster_swiglu", x2.data_ptr(), packed_k8.data_ptr(), scales.data_ptr(), y.data_ptr(), M, Nn, K,
-           ldx, norm[0].data_ptr() if fuse else None, float(norm[1]) if fuse else 0.0, N.stream())
+           ldx, norm[0].data_ptr() if fuse else None, float(norm[1]) if fuse else 0.0, static_w, N.stream())
     return y
 
 
-def int4_gemv(x, packed, scales, residual=None, packed_k8=None, norm=None):
+def int4_gemv(x, packed, scales, residual=None, packed_k8=None, norm=None, static_w=False):
     """x `[M <= 64, K]` @ dequant(W) (+ residual). With the repacked weight (`reference.repack_int4_k8`)
     the product runs on the streaming kernel (few rows) or the tcgen05 W4A16 kernel;
     otherwise on the CUDA-core weight-streaming kernel. `norm=(gamma fp32 [K], eps)` applies RMSNorm
-    to x first (fused into the GEMV for M <= 4)."""
+    to x first (fused into the GEMV for M <= 4). `static_w`: nothing in flight on the stream writes the
+    repacked weight or the scales, so that they may be requested before the preceding kernel is done."""
     M, K = x.shape
     Nn = packed.shape[1]
     x2, ldx = _rows(x)
     y = torch.empty(M, Nn, device=x.device, dtype=BF16)
     res = residual.contiguous() if residual is not None else None
     if packed_k8 is not None and M <= 8:
-        packed_k8, scales = _w4_operands(packed_k8, scales)
+        packed_k8, scales, static_w = _w4_operands(packed_k8, scales, static_w)
     use_mma = W4_GEMV_KERNEL == "mma"
     if (W4_GEMV_KERNEL == "stream" and packed_k8 is not None and M <= 4 and ldx % 8 == 0 and x2.data_ptr() % 16 == 0
             and K % 128 == 0 and Nn % 4 == 0 and K <= 16384):
@@ -1290,12 +1294,22 @@ def int4_gemv(x, packed, scales, residual=None, packed_k8=None, norm=None):
         if norm is not None and not fuse:
             x2 = rmsnorm(x2, norm[0], norm[1])
             ldx = x2.stride(0)
-        N.call("sb_w4_gemv_mma" if use_mma else "sb_w4_gemv_cluster", x2.data_ptr(), packed_k8.data_ptr(), scales.data_ptr(), N.ptr(res), y.data_ptr(),
-               M, Nn, K, ldx, norm[0].data_ptr() if fuse else None, float(norm[1]) if fuse else 0.0, N.stream())
+        args = (x2.data_ptr(), packed_k8.data_ptr(), scales.data_ptr(), N.ptr(res), y.data_ptr(), M, Nn, K, ldx,
+                norm[0].data_ptr() if fuse else None, float(norm[1]) if fuse else 0.0)
+        if use_mma:
+            N.call("sb_w4_gemv_mma", *args, N.stream())
+        else:
+            N.call("sb_w4_gemv_cluster", *args, static_w, N.stream())
         return y
     if norm is not None:
         x2 = rmsnorm(x2, norm[0], norm[1])
         ldx = x2.stride(0)
+    if (static_w and not use_mma and W4_GEMV_KERNEL != "stream" and packed_k8 is not None and ldx % 8 == 0 and x2.data_ptr() % 16 == 0
+            and K % 128 == 0 and Nn % 4 == 0 and N.call_value("sb_w4_stream_preferred", M, K)):
+        # the same kernel that sb_w4a16_gemm would pick, told that it may request the weights early
+        N.call("sb_w4_gemv_cluster", x2.data_ptr(), packed_k8.data_ptr(), scales.data_ptr(), N.ptr(res), y.data_ptr(), M, Nn, K, ldx,
+               None, 0.0, 1, N.stream())
+        return y
     acc = torch.empty(max(M, 64), Nn, device=x.device, dtype=torch.float32)
     if packed_k8 is not None and ldx % 8 == 0 and x2.data_ptr() % 16 == 0:
         N.call("sb_w4a16_gemm", x2.data_ptr(), packed_k8.data_ptr(), scales.data_ptr(), acc.data_ptr(), N.ptr(res),

@@ -105,6 +105,29 @@ def test_w4_projection_takes_unaligned_operand_views():
 
 
 @gpu
+@pytest.mark.parametrize("M", [2, 7])
+def test_w4_layer_marks_its_weights_settled_only_once_they_are(M, monkeypatch):
+    """The first call of a layer repacks (and aligns) right in front of the kernel, which must not read the weights early then;
+    later calls may. A raw call never may unless its caller says so, and a copy made for the call never is."""
+    from summa_b200 import ops
+    from summa_b200.models.quantized import QuantLinear
+    from summa_b200.ops import cuda_ops
+    packed, scales, k8, wq = _w4(512, 32, 7)
+    off = torch.empty(scales.numel() + 1, device="cuda", dtype=scales.dtype)[1:].view_as(scales).copy_(scales)
+    x = torch.randn(M, 512, device="cuda").to(torch.bfloat16)
+    flags, call = [], cuda_ops.N.call
+    monkeypatch.setattr(cuda_ops.N, "call", lambda name, *a: (flags.append(a[-2]) if name == "sb_w4_gemv_cluster" else None, call(name, *a))[1])
+    layer, unaligned = QuantLinear(packed, scales), QuantLinear(packed, off)
+    assert unaligned.scales.data_ptr() % 8
+    want = [ops.int4_gemv(x, packed, scales, None, k8), ops.int4_gemv(x, packed, off, None, k8, static_w=True),
+            ops.int4_gemv(x, packed, scales, None, k8, static_w=True)]
+    got = [m(x) for m in (layer, layer, unaligned, unaligned)]
+    # five to eight rows of unsettled weights go through the entry that has no such flag
+    assert flags == ([0, 0, 1, 0, 1, 0, 1] if M <= 4 else [1, 1, 1])
+    assert all(torch.equal(t, want[0]) for t in want + got)
+
+
+@gpu
 @pytest.mark.parametrize("M,K,I", [(1, 128, 4), (3, 9088, 20), (2, 14464, 12)])
 def test_w4_gated_projection_edges(M, K, I):
     from summa_b200.ops import cuda_ops
