@@ -329,7 +329,8 @@ mamba_conv_step_kernel(const __nv_bfloat16* __restrict__ x, long ldx, __nv_bfloa
   xc[(long)b * C + c] = __float2bfloat16(silu_f(a));
 }
 
-// h = exp(dt A) h + dt u B, y = <h, C> + D u, out = y silu(z), with dt = softplus(delta) and A = -exp(a_log). A lane owns
+// h = exp(dt A) h + dt u B, y = <h, C> + D u, out = y silu(z), with dt = softplus(delta) and A = -exp(a_log), formed in 64 bits
+// and rounded once as in the prefill form, so that both walk the same recurrence bit for bit. A lane owns
 // SPL states (4, or 8 for N = 256, or 2 for N = 8) of one channel; N / SPL lanes share a channel.
 template <int N, int SPL>
 __global__ void __launch_bounds__(256)
@@ -358,7 +359,8 @@ mamba_scan_step_kernel(const __nv_bfloat16* __restrict__ u, const __nv_bfloat16*
 #pragma unroll
     for (int i = 0; i < SPL; ++i) {
       const float bv = __bfloat162float(Bm[b * ld_bc + n0 + i]), cv = __bfloat162float(Cm[b * ld_bc + n0 + i]);
-      hv[i] = fmaf(__expf(-dt * __expf(al[i])), hv[i], du * bv);
+      const float A2 = -static_cast<float>(exp(static_cast<double>(al[i]))) * 1.4426950408889634f;
+      hv[i] = fmaf(fast_exp2(dt * A2), hv[i], du * bv);
       acc = fmaf(hv[i], cv, acc);
     }
 #pragma unroll

@@ -252,6 +252,24 @@ def test_mamba_decode_step_matches_the_general_path(B, state_dim, taps):
 
 
 @gpu
+@pytest.mark.parametrize("B,C,N", [(1, 8, 8), (3, 72, 16), (2, 40, 64), (1, 3072, 128), (2, 24, 256)])
+def test_mamba_scan_step_walks_the_prefill_recurrence(B, C, N):
+    """One token through the decode step and through the prefill scan from the same state, fast-decaying states included
+    (A = -exp(a_log) down to -3000): the new states are the same bits."""
+    from summa_b200.ops import cuda_ops, native
+    torch.manual_seed(C + N)
+    u, delta, z, Bm, Cm = [torch.randn(B, 1, n, device="cuda").to(torch.bfloat16) for n in (C, C, C, N, N)]
+    delta = (delta - 4).to(torch.bfloat16)
+    a_log, D, h0 = torch.rand(C, N, device="cuda") * 9 - 1, torch.randn(C, device="cuda"), torch.randn(B, C, N, device="cuda")
+    with torch.no_grad():
+        _, want = cuda_ops.selective_scan_log(u, delta, a_log, Bm, Cm, D, h0, True)
+    h, out = h0.clone(), torch.empty(B, C, device="cuda", dtype=torch.bfloat16)
+    native.call("sb_mamba_scan_step", u.data_ptr(), delta.data_ptr(), a_log.data_ptr(), Bm.data_ptr(), Cm.data_ptr(), N, D.data_ptr(),
+                z.data_ptr(), C, h.data_ptr(), out.data_ptr(), B, C, N, native.stream())
+    assert torch.equal(h, want)
+
+
+@gpu
 @pytest.mark.parametrize("B", [1, 5, 9])
 def test_hybrid_graph_decode_against_eager(B):
     """The captured step of a model with recurrent blocks: states after one token, repeated and continued requests."""
