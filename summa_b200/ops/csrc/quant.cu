@@ -117,6 +117,12 @@ template <int MPMAX, int G> struct WqCfg {
   static constexpr int THREADS = 128 * DQ + 64;
   static constexpr int NA = 4;                              // expanded weight buffers in tensor memory (32 columns each)
   static_assert(NS > NA, "the stage's barrier must still be in the phase of block i - NA when block i is expanded");
+  // A group waits for the loads of its own blocks only, so it does not see every phase of a stage's `full` barrier. The phase
+  // it waits for is unambiguous all the same: the stage is not loaded again before the block is consumed, and the load of block
+  // i - NS is long complete, because the group has waited for it itself (NS % DQ == 0) or, at its own block i - DQ, for the
+  // products of block i - DQ - NA, which come after those of every earlier block. (Waiting for the other groups' blocks in
+  // order as well would not close that but open a gap: nothing keeps their stages from being loaded twice meanwhile.)
+  static_assert(NS % DQ == 0 || NS >= DQ + NA, "a group could take an older load's phase for the one it needs");
 };
 
 struct W4Params {
@@ -218,12 +224,9 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
       return n < p.N && i < nkb ? p.scales[(long)((kb0 + i) >> 1) * p.N + n] : __float2bfloat16(0.f);
     };
     __nv_bfloat16 sc_next = scale_of(h);
-    for (int i = 0; i < nkb && ok; ++i) {
+    for (int i = h; i < nkb && ok; i += DQ) {
       const int s = i % WQ_NS, b = i % NA;
-      // every group waits for every block's load in order (a group that skipped phases of `full` could otherwise
-      // take an older phase of the same parity for the one it needs)
       if (!mbar_wait(&full[s], (i / WQ_NS) & 1, abort_flag, p.err)) { ok = false; break; }
-      if (DQ > 1 && i % DQ != h) continue;
       const __nv_bfloat162 s2 = __halves2bfloat162(sc_next, sc_next);
       sc_next = scale_of(i + DQ);
       const uint32_t* wt = reinterpret_cast<const uint32_t*>(smem + s * WQ_STAGE) + t;
