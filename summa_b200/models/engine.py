@@ -94,7 +94,11 @@ class InferenceEngine:
     @torch.no_grad()
     def decode(self, first: torch.Tensor, steps: int) -> torch.Tensor:
         """Greedy-decodes `steps` tokens after `first` `[B, 1]`; returns `[B, steps]` (the
-        tokens produced, not including `first`)."""
+        tokens produced, not including `first`). No steps: an empty tensor, and the state stays as it is."""
+        if steps < 0:
+            raise ValueError(f"cannot decode {steps} tokens")
+        if steps == 0:
+            return torch.empty(first.shape[0], 0, dtype=torch.long, device=first.device)
         if self.use_graph and self.device.type == "cuda":
             if self._graph is None:
                 self._graph = _GraphDecoder.try_build(self.model, self.state, steps)

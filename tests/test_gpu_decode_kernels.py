@@ -373,3 +373,33 @@ def test_decode_attention_many_sequences(B, Hq, Hkv, Sk):
     want = (p @ v).transpose(1, 2)
     assert bool(((o.double() - want).abs() <= 2.0 ** -7 * (p @ v.abs()).transpose(1, 2) + 2.0 ** -8 * want.abs()).all())
     assert native.read_error_flag() == 0
+
+
+@pytest.mark.parametrize("device", ["cpu", pytest.param("cuda", marks=gpu)])
+@pytest.mark.parametrize("before", [0, 1, 3])
+def test_decoding_no_tokens_leaves_the_state_alone(device, before):
+    """`decode(first, 0)` on a fresh engine, after one step (no graph kept yet) and after several: nothing moves, and what
+    follows is what follows without it. A negative count is an error."""
+    from summa_b200.models import Transformer
+    from summa_b200.models.engine import InferenceEngine
+    torch.manual_seed(before)
+    cfg = _hybrid(8, 2)
+    with torch.device(device):
+        model = Transformer(cfg, init_std=0.1)
+    if device == "cuda":
+        model.prepare_inference(torch.bfloat16)
+    eng = InferenceEngine(model)
+    eng.reset(2, 24)
+    tok = eng.prefill(torch.randint(0, 512, (2, 5), device=device))
+    if before:
+        tok = eng.decode(tok, before)[:, -1:]
+    held = [{k: v.clone() if torch.is_tensor(v) else v for k, v in vars(s).items()} for s in eng.state.layers]
+    pos = eng.state.pos
+    none = eng.decode(tok, 0)
+    assert none.shape == (2, 0) and none.dtype == torch.long and eng.state.pos == pos
+    for s, old in zip(eng.state.layers, held):
+        for k, v in old.items():
+            assert torch.equal(getattr(s, k), v) if torch.is_tensor(v) else getattr(s, k) == v
+    with pytest.raises(ValueError):
+        eng.decode(tok, -1)
+    assert eng.decode(tok, 2).shape == (2, 2)
