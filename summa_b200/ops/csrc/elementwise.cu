@@ -1212,7 +1212,7 @@ extern "C" int sb_colsum(const void* x, float* part, float* out, long rows, int 
 
 // out = a x + b y over n bf16 elements (n % 8 == 0, 16-byte aligned); out may be x or y
 extern "C" int sb_axpby(const void* x, const void* y, void* out, long n, float a, float b, cudaStream_t st) {
-  SB_CHECK_ARG(n > 0 && n % 8 == 0);
+  SB_CHECK_ARG(n > 0 && n % 8 == 0 && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(out)) & 15) == 0);
   axpby_kernel<<<grid_for(n / 8, 256), 256, 0, st>>>((const uint4*)x, (const uint4*)y, (uint4*)out, n / 8, a, b);
   SB_CHECK_CUDA(cudaGetLastError());
   return SB_OK;
@@ -1221,6 +1221,7 @@ extern "C" int sb_axpby(const void* x, const void* y, void* out, long n, float a
 // out[b, :] = x[b, :] / div[b] over `batch` matrices of `per` bf16 elements (per % 8 == 0, 16-byte aligned)
 extern "C" int sb_matrix_div(const void* x, const void* div, void* out, int batch, long per, cudaStream_t st) {
   SB_CHECK_ARG(batch > 0 && batch <= 65535 && per > 0 && per % 8 == 0);
+  SB_CHECK_ARG(((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(out)) & 15) == 0);
   long bx = (per / 8 + 255) / 256, cap = (16L * num_sms() + batch - 1) / batch;
   if (bx > cap) bx = cap;
   matrix_div_kernel<<<dim3((int)bx, batch), 256, 0, st>>>((const uint4*)x, (const __nv_bfloat16*)div, (uint4*)out, per / 8);

@@ -44,7 +44,8 @@ def newton_schulz(G: torch.Tensor, steps: int = NS_STEPS) -> torch.Tensor:
     device = X.is_cuda and X.shape[1] % 8 == 0 and X.shape[2] % 8 == 0       # then the products keep whole 16-byte rows too
     if device:
         from ..ops import cuda_ops
-        X, mix = cuda_ops.matrix_div(X.contiguous(), div), cuda_ops.axpby
+        X, mix = X.contiguous(), cuda_ops.axpby
+        X = cuda_ops.matrix_div(X, div) if X.data_ptr() % 16 == 0 else X / div     # (a view may start anywhere; what follows is ours)
     else:
         X = X / div
 

@@ -75,6 +75,25 @@ def test_newton_schulz_elementwise_steps(shape):
 
 
 @gpu
+@pytest.mark.parametrize("shape,off", [((2, 24, 40), 1), ((1, 64, 32), 4), ((3, 16, 16), 8)])
+def test_newton_schulz_of_a_view_that_starts_anywhere(shape, off):
+    """A contiguous bf16 batch whose first element is off a 16-byte boundary gives the same bits as its aligned copy, and the raw
+    entry points refuse it on the host."""
+    from summa_b200.ops import cuda_ops, native
+    from summa_b200.train.muon import newton_schulz
+    torch.manual_seed(off)
+    n = shape[0] * shape[1] * shape[2]
+    g = torch.randn(n + off, device="cuda").to(torch.bfloat16)[off:].view(shape)
+    assert g.is_contiguous() and (g.data_ptr() % 16 != 0) == (off % 8 != 0)
+    assert torch.equal(newton_schulz(g), newton_schulz(g.clone()))
+    if off % 8:
+        with pytest.raises(native.NativeError):
+            cuda_ops.axpby(1.0, g, 1.0, g)
+        with pytest.raises(native.NativeError):
+            cuda_ops.matrix_div(g, torch.ones(shape[0], 1, 1, device="cuda", dtype=torch.bfloat16))
+
+
+@gpu
 @pytest.mark.parametrize("T,Hq,Hkv,D", [(1, 1, 1, 64), (9, 3, 1, 128), (12000, 8, 4, 64)])
 def test_qk_norm_rope_backward_gains(T, Hq, Hkv, D):
     """Input and gain gradients with fewer and more (token, head) items than one round of the grid, against fp64 autograd
