@@ -172,7 +172,8 @@ def selective_scan(u, delta, A, Bm, Cm, D, h0=None, need_final_state=False):
 
 def selective_scan_log(u, delta, a_log, Bm, Cm, D, h0=None, need_final_state=False):
     """`selective_scan` with A = -exp(a_log)."""
-    if native_enabled(u) and not torch.is_grad_enabled():
+    # (forward-mode derivatives keep to the autograd function, which refuses them: this form would drop a tangent of a_log)
+    if native_enabled(u) and not torch.is_grad_enabled() and torch.autograd.forward_ad._current_level < 0:
         return _cu().selective_scan_log(u, delta, a_log, Bm, Cm, D, h0, need_final_state)
     return selective_scan(u, delta, -torch.exp(a_log.float()), Bm, Cm, D, h0, need_final_state)
 

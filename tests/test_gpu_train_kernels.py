@@ -199,3 +199,20 @@ def test_scan_backward_tiles(B, T, C, Ns):
     torch.stack(ys, 1).backward(dy.double())
     for a, b in zip(lo, hi):
         assert float((a.grad.double() - b.grad).norm() / b.grad.norm()) <= 2.0 ** -8
+
+
+@gpu
+def test_scan_without_gradients_does_not_drop_a_forward_mode_tangent():
+    from summa_b200 import ops
+    import torch.autograd.forward_ad as fwd
+    torch.manual_seed(0)
+    u, delta, Bm, Cm = [torch.randn(1, 9, n, device="cuda").to(torch.bfloat16) for n in (16, 16, 8, 8)]
+    a_log, D = torch.rand(16, 8, device="cuda"), torch.ones(16, device="cuda")
+    with torch.no_grad():
+        y, _ = ops.selective_scan_log(u, delta, a_log, Bm, Cm, D)
+        with fwd.dual_level():
+            with pytest.raises((RuntimeError, NotImplementedError)):
+                ops.selective_scan_log(u, delta, fwd.make_dual(a_log, torch.ones_like(a_log)), Bm, Cm, D)
+            again, _ = ops.selective_scan_log(u, delta, a_log, Bm, Cm, D)
+    # without a tangent the autograd function runs: A from the library's exponential, one unit in the last place of fp32 away
+    torch.testing.assert_close(again.float(), y.float(), rtol=2 ** -7, atol=2 ** -10)
