@@ -99,7 +99,7 @@ class InferenceEngine:
             raise ValueError(f"cannot decode {steps} tokens")
         if steps == 0:
             return torch.empty(first.shape[0], 0, dtype=torch.long, device=first.device)
-        if self.use_graph and self.device.type == "cuda":
+        if self.use_graph and self.device.type == "cuda" and not _has_hooks(self.model):
             if self._graph is None:
                 self._graph = _GraphDecoder.try_build(self.model, self.state, steps)
             if self._graph is not None and self._graph.max_steps >= steps:
@@ -111,6 +111,13 @@ class InferenceEngine:
             tok = ops.argmax(logits).view(-1, 1)
             out.append(tok)
         return torch.cat(out, dim=1)
+
+
+def _has_hooks(model) -> bool:
+    """Whether something watches or changes module calls: the captured step goes past the modules, so such a model decodes eagerly."""
+    from torch.nn.modules import module as M
+    return bool(M._global_forward_hooks or M._global_forward_pre_hooks
+                or any(m._forward_hooks or m._forward_pre_hooks for m in model.modules()))
 
 
 class _GraphDecoder:

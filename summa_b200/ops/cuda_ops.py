@@ -849,14 +849,17 @@ N.register("sb_mamba_scan_step", [N.P] * 5 + [N.L, N.P, N.P, N.L, N.P, N.P] + [N
 
 
 def mamba_decode_usable(mixer) -> bool:
-    """Whether `mamba_decode_step` takes this mixer: bf16 projections, fp32 scan parameters, supported state and taps."""
+    """Whether `mamba_decode_step` takes this mixer: the package's own modules (a subclass may compute something else), bf16
+    projections, fp32 scan parameters, supported state and taps."""
+    from ..models.layers import Linear, MambaMixer
+    if type(mixer) is not MambaMixer or any(type(p) is not Linear for p in (mixer.in_proj, mixer.x_proj, mixer.dt_proj, mixer.out_proj)):
+        return False
     w = mixer.conv1d.weight
     small = (mixer.a_log, mixer.d, mixer.conv1d.bias)
     return (mixer.d_state in _SCAN_STATES and 2 <= mixer.d_conv <= 4 and w.is_cuda and w.is_contiguous()
             and w.dtype in (BF16, torch.float32) and all(t.dtype == torch.float32 and t.is_contiguous() for t in small)
             and mixer.a_log.data_ptr() % 8 == 0
-            and all(getattr(p, "weight", None) is not None and p.weight.dtype == BF16
-                    for p in (mixer.in_proj, mixer.x_proj, mixer.dt_proj, mixer.out_proj)))
+            and all(p.weight.dtype == BF16 for p in (mixer.in_proj, mixer.x_proj, mixer.dt_proj, mixer.out_proj)))
 
 
 def mamba_decode_step(mixer, xz, conv, h):

@@ -403,3 +403,44 @@ def test_decoding_no_tokens_leaves_the_state_alone(device, before):
     with pytest.raises(ValueError):
         eng.decode(tok, -1)
     assert eng.decode(tok, 2).shape == (2, 2)
+
+
+@gpu
+def test_hybrid_decode_runs_hooks_and_subclasses():
+    """A forward hook on a mixer or a projection sees every token, before and after a graph was kept, and may change the output; a
+    subclass of the mixer or of a projection computes what its own forward says."""
+    from summa_b200.models import Transformer
+    from summa_b200.models.engine import InferenceEngine
+    from summa_b200.models.layers import Linear, MambaMixer
+    from summa_b200.ops import cuda_ops
+    torch.manual_seed(5)
+    with torch.device("cuda"):
+        model = Transformer(_hybrid(16, 4), init_std=0.1)
+    model.prepare_inference(torch.bfloat16)
+    prompt, eng = torch.randint(0, 512, (2, 7), device="cuda"), InferenceEngine(model)
+
+    def tokens(use_graph=True):
+        eng.use_graph = use_graph
+        eng.reset(2, 24)
+        return eng.decode(eng.prefill(prompt), 4)
+    plain, seen = tokens(), []
+    assert eng._graph is not None
+    for mod in (model.layers[0].ssm, model.layers[2].ssm.in_proj, model.final_norm):
+        hook, n = mod.register_forward_hook(lambda *a: seen.append(1)), len(seen)
+        assert torch.equal(tokens(), tokens(False)) and len(seen) - n == 2 * 5        # the prompt and four tokens, twice
+        hook.remove()
+    assert torch.equal(tokens(), plain)
+
+    class Off(MambaMixer):
+        def forward(self, x, state=None):
+            return torch.zeros_like(x)
+
+    class Double(Linear):
+        def forward(self, x):
+            return 2 * super().forward(x)
+    assert cuda_ops.mamba_decode_usable(model.layers[0].ssm)
+    model.layers[0].ssm.__class__ = Off
+    assert not cuda_ops.mamba_decode_usable(model.layers[0].ssm)
+    model.layers[0].ssm.__class__ = MambaMixer
+    model.layers[0].ssm.out_proj.__class__ = Double
+    assert not cuda_ops.mamba_decode_usable(model.layers[0].ssm)
