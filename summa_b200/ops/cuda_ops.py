@@ -148,6 +148,8 @@ N.register("sb_matrix_div", [N.P, N.P, N.P, N.I, N.L, N.P])
 def column_sum(x: torch.Tensor) -> torch.Tensor:
     """fp32 sums over the rows of a 2-D tensor (bias gradients)."""
     rows, Nn = x.shape
+    if torch.is_grad_enabled() and x.requires_grad:      # (backward under create_graph: the sum stays differentiable)
+        return x.float().sum(dim=0)
     if x.dtype != BF16 or rows == 0 or Nn % 8 or x.stride(1) != 1 or x.stride(0) % 8 or x.data_ptr() % 16:
         return x.float().sum(dim=0)
     part = torch.empty(N.call_value("sb_colsum_chunks", rows, Nn), Nn, device=x.device, dtype=torch.float32)

@@ -216,3 +216,17 @@ def test_scan_without_gradients_does_not_drop_a_forward_mode_tangent():
             again, _ = ops.selective_scan_log(u, delta, a_log, Bm, Cm, D)
     # without a tangent the autograd function runs: A from the library's exponential, one unit in the last place of fp32 away
     torch.testing.assert_close(again.float(), y.float(), rtol=2 ** -7, atol=2 ** -10)
+
+
+@gpu
+def test_bias_gradient_stays_differentiable():
+    """The gradient of a bias under `create_graph`, differentiated once more with respect to what came from above."""
+    from summa_b200 import ops
+    torch.manual_seed(2)
+    x, w = torch.randn(40, 32, device="cuda").to(torch.bfloat16), torch.randn(32, 16, device="cuda").to(torch.bfloat16)
+    b = torch.zeros(16, device="cuda", requires_grad=True)
+    up = torch.randn(40, 16, device="cuda").to(torch.bfloat16).requires_grad_(True)
+    db, = torch.autograd.grad(ops.linear(x, w, b), b, up, create_graph=True)
+    again, = torch.autograd.grad(db.pow(2).sum(), up)
+    want = (2 * up.detach().double().sum(0)).expand(40, 16)
+    torch.testing.assert_close(again.double(), want, rtol=2 ** -8, atol=1e-6)
