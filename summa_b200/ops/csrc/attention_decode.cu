@@ -28,9 +28,8 @@ constexpr int DEC_N = 8;                           // padded query heads per kv 
 constexpr int DEC_THREADS = 192;
 constexpr int DEC_TILE = 128 * DEC_D * 2;          // 32 KB
 constexpr int DEC_OFF_K = 0;
-// K/V ring stages: 3 for few (batch, kv head) pairs, where one CTA per SM has to keep HBM busy by itself; 1 when there are
-// more pairs than SMs, where three CTAs per SM hide each other's loads and softmax steps instead (64 sequences x 8 kv heads,
-// 150 cached tokens: 22.8 us and a merge of 3.4 with 3 stages and 3.5 rounds of CTAs, 17.4 with 1).
+// K/V ring stages: with 3 one CTA per SM keeps HBM busy by itself; with 1 three CTAs per SM hide each other's loads and softmax
+// steps instead. `one_stage` below says which.
 template <int NS> struct DecLayout {
   static constexpr int OFF_V = NS * DEC_TILE;
   static constexpr int OFF_Q = 2 * NS * DEC_TILE;    // 8 rows x 256 B (two swizzle atoms)
@@ -315,6 +314,21 @@ extern "C" int sb_attention_decode_splits(int B, int Hkv, int Sk) {
   return want;
 }
 
+// Whether the one-stage form is ahead, for `ctas` CTAs of `blocks` blocks of 128 keys. 8 kv heads, us with three stages / with one:
+//   no more CTAs than SMs: level (8 sequences x 150 keys 8.25 / 8.30), and three stages have the shorter chain;
+//   up to six blocks per CTA its rounds are mostly start and end, and three at a time hide those (64 x 150: 24.5 / 17.2, 8 x 600:
+//   17.6 / 11.5, 16 x 2100: 37.1 / 30.9, 64 x 600: 40.6 / 37.6);
+//   longer ones run at memory speed either way, a round of three per SM taking two and a half rounds of one, so what counts is
+//   how the CTAs fill their last round (512 CTAs, i.e. 4 rounds or 2: 64 x 1100 60.4 / 62.5, 64 x 2100 98.5 / 114, 64 x 4200
+//   177 / 217; 296, 2 or 1: 37 x 4200 98.5 / 109; 384, 3 or 1: 24 x 4200 77.0 / 70.3; 768, 6 or 2: 96 x 2100 146 / 130).
+// Over 123 shapes (1..128 sequences, 1..8 kv heads, 150..8200 keys) the choice is 0.1 % behind the better form on average and 6 %
+// at most; "more than two rounds of CTAs", the rule before, 3.9 % and 35 %; three stages always 15 % and 66 %.
+static bool one_stage(long ctas, int blocks, int sms) {
+  const long rounds3 = (ctas + sms - 1) / sms, rounds1 = (ctas + 3L * sms - 1) / (3L * sms);
+  return ctas > sms && (blocks <= 6 || 2 * rounds3 >= 5 * rounds1);
+}
+extern "C" int sb_attention_decode_one_stage(long ctas, int blocks, int sms) { return one_stage(ctas, blocks, sms) ? 1 : 0; }
+
 static int decode_launch(const void* q, const void* k, const void* v, void* o, float* work, int B, int Hq, int Hkv,
                          int Sk, const int* sk_ptr, int sk_add, int cap, int D, const long* q_strides,
                          const long* k_strides, const long* v_strides, const long* o_strides, float scale, int splits,
@@ -347,7 +361,7 @@ static int decode_launch(const void* q, const void* k, const void* v, void* o, f
   if (!p.err) return SB_ERR_CUDA;
   p.o = splits == 1 ? (__nv_bfloat16*)o : nullptr;
   p.o_sb = o_strides[0]; p.o_sh = o_strides[1];
-  const bool many = (long)splits * Hkv * B > 2L * num_sms();
+  const bool many = one_stage((long)splits * Hkv * B, p.blocks_per_split, num_sms());
   auto kern = many ? attention_decode_kernel<1> : attention_decode_kernel<3>;
   const int smem = many ? DecLayout<1>::SMEM : DecLayout<3>::SMEM;
   static bool attr_set[2][64] = {{false}};

@@ -357,11 +357,24 @@ def test_argmax_rows_vector_and_scalar(dtype, rows, vocab, ld, off):
     assert int(ops.argmax(x)[0]) == 0
 
 
+@pytest.mark.parametrize("ctas,blocks,one", [
+    (148, 1, 0), (149, 1, 1), (512, 2, 1), (512, 6, 1), (512, 7, 0), (512, 33, 0), (296, 9, 0), (296, 6, 1), (304, 4, 1), (320, 33, 1),
+    (384, 17, 1), (444, 33, 1), (445, 33, 0), (768, 17, 1), (1024, 17, 0), (1024, 5, 1)])
+def test_decode_attention_form(ctas, blocks, one):
+    """The rule on a GPU of 148 SMs, at shapes where the two forms were timed against each other."""
+    from summa_b200.ops import native
+    import ctypes
+    f = native.lib().sb_attention_decode_one_stage
+    f.argtypes = [ctypes.c_long, ctypes.c_int, ctypes.c_int]
+    assert f(ctas, blocks, 148) == one
+
+
 @gpu
-@pytest.mark.parametrize("B,Hq,Hkv,Sk", [(38, 16, 8, 1), (40, 32, 8, 127), (64, 8, 8, 129), (75, 12, 4, 300), (37, 64, 8, 513), (5, 8, 8, 140)])
+@pytest.mark.parametrize("B,Hq,Hkv,Sk", [(38, 16, 8, 1), (40, 32, 8, 127), (64, 8, 8, 129), (75, 12, 4, 300), (37, 64, 8, 513), (5, 8, 8, 140),
+                                         (2, 16, 8, 2100), (16, 16, 8, 2100), (64, 8, 8, 1100), (37, 8, 8, 1100)])
 def test_decode_attention_many_sequences(B, Hq, Hkv, Sk):
-    """More (sequence, kv head) pairs than two rounds of SMs: the one-stage kernel, which writes the output itself when the keys
-    are not split; the last case stays on the split form. bf16 probabilities and values: 2^-8 of the weighted sum's terms."""
+    """Both forms of the kernel (one stage and three), each with split keys and with whole ones, where it writes the output
+    itself; (5, 8, 8, 140) has fewer CTAs than SMs. bf16 probabilities and values: 2^-8 of the weighted sum's terms."""
     from summa_b200.ops import cuda_ops, native
     torch.manual_seed(B + Sk)
     q = torch.randn(B, 1, Hq, 128, device="cuda").to(torch.bfloat16)
