@@ -439,15 +439,22 @@ static int scan_fwd(int a_is_log, const void* u, const void* delta, const float*
           (((uintptr_t)u | (uintptr_t)delta | (uintptr_t)Bm | (uintptr_t)Cm) & 15) == 0;
   // States per thread and channels per block. The sequence is serial, so the warps in flight are B C N / (32 states per
   // thread) however long it is: few states per thread until there are about 20 warps per SM. N 16, 4 states instead of 16:
-  // B 27 T 1024 C 1024 396 -> 254 us, B 24 T 301 119 -> 78; N 128, 8 instead of 16: B 1 T 4096 C 3072 1136 -> 999 us (32
-  // channels, one block per SM at most), B 2 T 8192 2889 -> 2881 (16 channels; 3493 with 32, whose last round is short).
+  // B 27 T 1024 C 1024 396 -> 254 us, B 24 T 301 119 -> 78. N 8, 4 instead of 8: B 1 T 77 C 3072 30 -> 24, B 2 T 8192 2153 ->
+  // 1517, B 27 T 1024 C 1024 312 -> 233. N 32, 8 instead of 16: B 2 T 8192 C 3072 2421 -> 1729, B 27 411 -> 362, B 64 T 512
+  // 435 -> 384; N 64 the same: 2334 -> 1505, 679 -> 594, 693 -> 657. N 128, 8 instead of 16: B 1 T 4096 C 3072 1136 -> 999 us
+  // (32 channels, one block per SM at most), B 2 T 8192 2596 -> 2441 (16 channels; 32 leave a short last round), B 3 T 1024 411 ->
+  // 399; where 16 states give 20 warps per SM already they stay: B 4 574 against 582 (with checkpoints 653 against 680), B 27 C
+  // 1024 1083 against 1108 (1250, 1304).
   const bool one_round = (long)B * ((C + 31) / 32) <= num_sms();
+  const bool wide128 = (long)B * C * 128 / (16 * 32) >= 20L * num_sms();
   switch (N) {
     case 8: return launch_scan_fwd<8, 4, 32>(p, st);
     case 16: return launch_scan_fwd<16, 4, 32>(p, st);
     case 32: return launch_scan_fwd<32, 8, 32>(p, st);
     case 64: return launch_scan_fwd<64, 8, 16>(p, st);
-    case 128: return one_round ? launch_scan_fwd<128, 8, 32>(p, st) : launch_scan_fwd<128, 8, 16>(p, st);
+    case 128:
+      if (one_round) return launch_scan_fwd<128, 8, 32>(p, st);
+      return wide128 ? launch_scan_fwd<128, 16, 16>(p, st) : launch_scan_fwd<128, 8, 16>(p, st);
     case 256: return launch_scan_fwd<256, 16, 16>(p, st);
     default:
       fprintf(stderr, "summa_b200: selective scan supports d_state in {8,16,32,64,128,256}, got %d\n", N);

@@ -230,3 +230,26 @@ def test_bias_gradient_stays_differentiable():
     again, = torch.autograd.grad(db.pow(2).sum(), up)
     want = (2 * up.detach().double().sum(0)).expand(40, 16)
     torch.testing.assert_close(again.double(), want, rtol=2 ** -8, atol=1e-6)
+
+
+@gpu
+@pytest.mark.parametrize("B,T,C,N", [(1, 19, 40, 8), (2, 33, 72, 16), (3, 17, 40, 32), (2, 16, 24, 64), (2, 17, 2368, 128), (2, 17, 2370, 128),
+                                     (11, 9, 1076, 128), (12, 9, 1024, 128), (1, 17, 24, 256)])
+def test_scan_forward_tilings_against_fp64(B, T, C, N):
+    """Every number of states per thread and channels per block, with N 128 on both sides of its two lines (148 blocks of 32
+    channels, 11840 channels in all). The states are fp32 sums with decays of a few 2^-22 each; y is rounded to bf16."""
+    from summa_b200.ops import cuda_ops
+    torch.manual_seed(B + C + N)
+    u, delta, Bm, Cm = [torch.randn(B, T, n, device="cuda").to(torch.bfloat16) for n in (C, C, N, N)]
+    a_log, D, h0 = torch.rand(C, N, device="cuda") * 2 - 1, torch.randn(C, device="cuda"), torch.randn(B, C, N, device="cuda")
+    with torch.no_grad():
+        y, h = cuda_ops.selective_scan_log(u, delta, a_log, Bm, Cm, D, h0, True)
+    hs, mag, A = h0.double(), h0.double().abs(), -torch.exp(a_log.double())
+    for t in range(T):
+        dt, x = torch.nn.functional.softplus(delta[:, t].double()), u[:, t].double()
+        decay, inp = torch.exp(dt[..., None] * A), (dt * x)[..., None] * Bm[:, t].double()[:, None]
+        hs, mag = decay * hs + inp, decay * mag + inp.abs()
+        want = (hs * Cm[:, t].double()[:, None]).sum(-1) + D.double() * x
+        tol = 2.0 ** -15 * ((mag * Cm[:, t].double().abs()[:, None]).sum(-1) + (D.double() * x).abs()) + 2.0 ** -8 * want.abs()
+        assert bool(((y[:, t].double() - want).abs() <= tol).all())
+    assert bool(((h.double() - hs).abs() <= 2.0 ** -15 * mag).all())
