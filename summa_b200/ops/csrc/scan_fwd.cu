@@ -444,7 +444,8 @@ static int scan_fwd(int a_is_log, const void* u, const void* delta, const float*
   // 435 -> 384; N 64 the same: 2334 -> 1505, 679 -> 594, 693 -> 657. N 128, 8 instead of 16: B 1 T 4096 C 3072 1136 -> 999 us
   // (32 channels, one block per SM at most), B 2 T 8192 2596 -> 2441 (16 channels; 32 leave a short last round), B 3 T 1024 411 ->
   // 399; where 16 states give 20 warps per SM already they stay: B 4 574 against 582 (with checkpoints 653 against 680), B 27 C
-  // 1024 1083 against 1108 (1250, 1304).
+  // 1024 1083 against 1108 (1250, 1304). (Of twelve shapes around the line one loses, by how its blocks fill the last round: B 16
+  // C 1024 667 with 8, 689 with 16.)
   const bool one_round = (long)B * ((C + 31) / 32) <= num_sms();
   const bool wide128 = (long)B * C * 128 / (16 * 32) >= 20L * num_sms();
   switch (N) {
