@@ -237,7 +237,10 @@ bf16_stream_kernel(const Bf16StreamArgs p, const int static_w, const int tile_ba
       // ---- tile done: hand this warp's sums over
       ci = 0;
       const int hb = handed % NB;
-      if (handed >= NB && !mbar_wait(&empty[hb], ((handed / NB) - 1) & 1, &abort_flag, err)) return;
+      if (handed >= NB && !mbar_wait(&empty[hb], ((handed / NB) - 1) & 1, &abort_flag, err)) {
+        cp_async_wait_all();                  // (no copy may land in shared memory that is someone else's by then)
+        return;
+      }
 #pragma unroll
       for (int h = 0; h < CH; ++h) {
         float* r = red + ((hb * BFS_WARPS + warp) * ROWS + 2 * tq) * TC + 16 * h + gq;
