@@ -506,11 +506,6 @@ extern "C" int sb_moe_plan_gates(const float* logits, int* idx, int* counts, int
   return SB_OK;
 }
 
-extern "C" int sb_moe_plan(const float* logits, int* idx, int* counts, int* meta, int* tile_expert, int* dest,
-                           int* row_route, int T, int E, int k, int max_rows, cudaStream_t st) {
-  return sb_moe_plan_gates(logits, idx, counts, meta, tile_expert, dest, row_route, nullptr, nullptr, T, E, k, max_rows, st);
-}
-
 // dlogits `[T, E]` fp32 from the gradient of the gates of sb_moe_plan_gates
 extern "C" int sb_moe_gates_bwd(const int* idx, const float* gates, const float* dgates, float* dlogits, int T, int E, int k,
                                 cudaStream_t st) {

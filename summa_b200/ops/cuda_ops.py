@@ -884,7 +884,6 @@ def mamba_decode_step(mixer, xz, conv, h):
 # ------------------------------------------------------------------ mixture of experts
 
 N.register("sb_router_logits", [N.P, N.P, N.P, N.I, N.I, N.I, N.L, N.P])
-N.register("sb_moe_plan", [N.P] * 7 + [N.I] * 4 + [N.P])
 N.register("sb_moe_plan_gates", [N.P] * 9 + [N.I] * 4 + [N.P])
 N.register("sb_moe_gates_bwd", [N.P] * 4 + [N.I] * 3 + [N.P])
 N.register("sb_moe_gather", [N.P, N.P, N.P, N.P, N.I, N.I, N.I, N.L, N.I, N.P])
