@@ -20,8 +20,8 @@
 //     immediate epilogue per tile its latency was paid per tile. No cluster, no atomics.
 //   * weights that nothing in flight writes (`static_w`) are requested before `griddepcontrol.wait`.
 // Measured against the CUDA-core cluster kernel it replaces (weights from HBM, graph of launches, one row): K 4096 N 6144
-// 12.0 -> 7.4 us, N 4096 7.4 -> 5.8, N 28672 29.0 -> 18.9 (gated with norm 32.9 -> 21.3), N 32000 30.2 -> 21.2, K 14336 N 4096
-// 19.8 -> 13.0; four rows: 20.0 -> 9.2, 14.6 -> 7.4, 60.6 -> 26.2, 66.4 -> 29.0, 41.9 -> 18.2. Error of the sums against 64 bits
+// 12.0 -> 7.3 us, N 4096 7.4 -> 5.6, N 28672 28.9 -> 18.7 (gated with norm 32.9 -> 20.9), N 32000 30.3 -> 20.9, K 14336 N 4096
+// 20.0 -> 12.3; four rows: 20.0 -> 9.6, 14.6 -> 7.8, 61.0 -> 26.0, 66.9 -> 28.6, 41.8 -> 19.0. Error of the sums against 64 bits
 // 2.5e-6 of the result (2.7e-6), and no more with outliers of 4096 whose weights are zero (3.6e-3: that kernel multiplied
 // 128 + q and took 136 times the sum of x away). The first form of the digits (three, elements below 2^-21 of the largest lost)
 // took 7.3, 5.7, 20.1, 22.4 and 12.4 us; bf16 products for one row 26.0 us at N 28672. Issue slots matter: with a division and
@@ -230,7 +230,6 @@ w4_stream_kernel(const W4StreamArgs p, const int tile_base, const int tiles, con
     const int g0 = pass * pass_groups, g1 = min(groups, g0 + pass_groups), ng = g1 - g0;
     const int gpw = (ng + W4S_WARPS - 1) / W4S_WARPS;
     const int mine = (ng - warp + W4S_WARPS - 1) / W4S_WARPS;
-    const int total = ntiles * gpw;
     lt = t_lo; li = 0; lmine = mine; lgpw = gpw;
     lw = p.wk8 + (long)(16 * (g0 + warp) + cr) * N + (long)lt * TILE_COLS + ccol;
     ls = p.scales + (long)(g0 + warp) * N + (long)lt * TILE_COLS + ccol;
@@ -241,6 +240,32 @@ w4_stream_kernel(const W4StreamArgs p, const int tile_base, const int tiles, con
     // ---- the rows of x of this pass, normed on the way, as they are or as digits; half a warp takes one (row, group)
     const int l16 = threadIdx.x & 15;
     uint4 v[4];
+    // `f` on the items i, i + 32, .. of this half-warp that v holds. Bf16 rows: one after another. Digits: alone, or two at a
+    // time in a loop, so that the shuffles of two overlap; all four unrolled took longer in a decode step, where every launch
+    // finds its instructions cold (33.6 ms for 64 tokens of eight 7B blocks against 35.2).
+    auto items = [&](int i, int count, auto f) {
+      const int first = i - (lane >> 4);
+      if constexpr (!DIGITS) {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          if (first + 32 * q >= count) break;
+          f(std::integral_constant<int, 1>{}, i + 32 * q, v + q);
+        }
+      } else if (first + 32 >= count) {
+        f(std::integral_constant<int, 1>{}, i, v);
+      } else {
+        const bool swap = first + 64 < count;
+#pragma unroll 1
+        for (int r = 0; r < (swap ? 2 : 1); ++r) {
+          f(std::integral_constant<int, 2>{}, i + 64 * r, v);
+          if (swap) {
+            const uint4 t0 = v[0], t1 = v[1];
+            v[0] = v[2]; v[1] = v[3];
+            v[2] = t0; v[3] = t1;
+          }
+        }
+      }
+    };
     bool kept = false;                        // v holds this half-warp's items already
     int any_lost = 0;
     if (pass == 0) {
@@ -254,18 +279,26 @@ w4_stream_kernel(const W4StreamArgs p, const int tile_base, const int tiles, con
           kept = passes == 1 && M * groups <= 128;
 #pragma unroll
           for (int q = 0; q < 4; ++q) {
-            const int i = i0 + 32 * q, m = i / groups, g = i - m * groups;
+            const int i = i0 + 32 * q, m = M == 1 ? 0 : i / groups, g = i - m * groups;
             v[q] = i < M * groups ? __ldcg(reinterpret_cast<const uint4*>(p.x + (long)m * p.ldx + g * 128) + l16) : make_uint4(0u, 0u, 0u, 0u);
           }
+          items(i0, M * groups, [&](auto n, int i, const uint4* at) {
+            constexpr int NQ = decltype(n)::value;
+            float s[NQ];
 #pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            const float a0 = bf16_lo(v[q].x), a1 = bf16_hi(v[q].x), a2 = bf16_lo(v[q].y), a3 = bf16_hi(v[q].y);
-            const float a4 = bf16_lo(v[q].z), a5 = bf16_hi(v[q].z), a6 = bf16_lo(v[q].w), a7 = bf16_hi(v[q].w);
-            float s = a0 * a0 + a1 * a1 + a2 * a2 + a3 * a3 + a4 * a4 + a5 * a5 + a6 * a6 + a7 * a7;
+            for (int q = 0; q < NQ; ++q) {
+              const float a0 = bf16_lo(at[q].x), a1 = bf16_hi(at[q].x), a2 = bf16_lo(at[q].y), a3 = bf16_hi(at[q].y);
+              const float a4 = bf16_lo(at[q].z), a5 = bf16_hi(at[q].z), a6 = bf16_lo(at[q].w), a7 = bf16_hi(at[q].w);
+              s[q] = a0 * a0 + a1 * a1 + a2 * a2 + a3 * a3 + a4 * a4 + a5 * a5 + a6 * a6 + a7 * a7;
+            }
 #pragma unroll
-            for (int o = 8; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-            if (l16 == 0 && i0 + 32 * q < M * groups) gsq[i0 + 32 * q] = s;
-          }
+            for (int o = 8; o > 0; o >>= 1)
+#pragma unroll
+              for (int q = 0; q < NQ; ++q) s[q] += __shfl_xor_sync(0xffffffffu, s[q], o);
+#pragma unroll
+            for (int q = 0; q < NQ; ++q)
+              if (l16 == 0 && i + 32 * q < M * groups) gsq[i + 32 * q] = s[q];
+          });
         }
         __syncthreads();
         for (int m = warp; m < M; m += W4S_WARPS) {
@@ -281,74 +314,93 @@ w4_stream_kernel(const W4StreamArgs p, const int tile_base, const int tiles, con
       const int i0 = i1 + (lane >> 4);
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
-        const int i = i0 + 32 * q, m = i / ng, gl = i - m * ng;
+        const int i = i0 + 32 * q, m = M == 1 ? 0 : i / ng, gl = i - m * ng;
         if (!kept) v[q] = i < M * ng ? __ldcg(reinterpret_cast<const uint4*>(p.x + (long)m * p.ldx + (g0 + gl) * 128) + l16) : make_uint4(0u, 0u, 0u, 0u);
       }
+      items(i0, M * ng, [&](auto n, int ifirst, const uint4* from) {
+        constexpr int NQ = decltype(n)::value;
+        int row[NQ], grp[NQ];
+        bool there[NQ];
+        uint4 u[NQ];
 #pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        if (i1 + 32 * q >= M * ng) break;
-        const int i = min(i0 + 32 * q, M * ng - 1), m = i / ng, gl = i - m * ng;
-        const bool mine_too = i0 + 32 * q < M * ng;                              // (the warp's second half may be past the end)
-        uint4 u = v[q];
-        if (p.gamma != nullptr) {
-          const float r = rstd[m];
-          const float2* gp = reinterpret_cast<const float2*>(p.gamma + (g0 + gl) * 128 + 8 * l16);
-          const float2 a = __ldg(gp), b = __ldg(gp + 1), c = __ldg(gp + 2), d = __ldg(gp + 3);
-          u.x = pack_bf16(bf16_lo(u.x) * r * a.x, bf16_hi(u.x) * r * a.y);
-          u.y = pack_bf16(bf16_lo(u.y) * r * b.x, bf16_hi(u.y) * r * b.y);
-          u.z = pack_bf16(bf16_lo(u.z) * r * c.x, bf16_hi(u.z) * r * c.y);
-          u.w = pack_bf16(bf16_lo(u.w) * r * d.x, bf16_hi(u.w) * r * d.y);
+        for (int q = 0; q < NQ; ++q) {
+          const int i = ifirst + 32 * q;
+          there[q] = i < M * ng;
+          row[q] = M == 1 || !there[q] ? 0 : i / ng;
+          grp[q] = there[q] ? i - row[q] * ng : 0;
+          u[q] = from[q];
+          if (p.gamma != nullptr) {
+            const float r = rstd[row[q]];
+            const float2* gp = reinterpret_cast<const float2*>(p.gamma + (g0 + grp[q]) * 128 + 8 * l16);
+            const float2 a = __ldg(gp), b = __ldg(gp + 1), c = __ldg(gp + 2), d = __ldg(gp + 3);
+            u[q].x = pack_bf16(bf16_lo(u[q].x) * r * a.x, bf16_hi(u[q].x) * r * a.y);
+            u[q].y = pack_bf16(bf16_lo(u[q].y) * r * b.x, bf16_hi(u[q].y) * r * b.y);
+            u[q].z = pack_bf16(bf16_lo(u[q].z) * r * c.x, bf16_hi(u[q].z) * r * c.y);
+            u[q].w = pack_bf16(bf16_lo(u[q].w) * r * d.x, bf16_hi(u[q].w) * r * d.y);
+          }
         }
         if constexpr (!DIGITS) {
-          if (mine_too) *reinterpret_cast<uint4*>(w4s_smem + m * L.pitch + gl * 256 + 16 * l16) = u;
+#pragma unroll
+          for (int q = 0; q < NQ; ++q)
+            if (there[q]) *reinterpret_cast<uint4*>(w4s_smem + row[q] * L.pitch + grp[q] * 256 + 16 * l16) = u[q];
         } else {
           // largest magnitude of the group and smallest one that is not zero, as bf16 bits (NaN > Inf > finite as unsigned
-          // numbers; zero - 1 wraps above them all): max in the upper half, ~(min - 1) in the lower
-          uint32_t mx = 0u, mn = 0xFFFFFFFFu;
-          const uint32_t uw[4] = {u.x, u.y, u.z, u.w};
+          // numbers): max in the upper half, ~(min - 1) in the lower (zeros count as 0 in either)
+          uint32_t both[NQ];
 #pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            const uint32_t mag = uw[e] & 0x7FFF7FFFu;
-            mx = __vmaxu2(mx, mag);
-            mn = __vminu2(mn, __vsub2(mag, 0x00010001u));
-          }
-          uint32_t both = __vmaxu2(__byte_perm(mx, ~mn, 0x7632), __byte_perm(mx, ~mn, 0x5410));      // (max | ~min) of either half
-          both = __byte_perm(both, 0u, 0x1032);
+          for (int q = 0; q < NQ; ++q) {
+            uint32_t mx = 0u, mn = 0u;
+            const uint32_t uw[4] = {u[q].x, u[q].y, u[q].z, u[q].w};
 #pragma unroll
-          for (int o = 8; o > 0; o >>= 1) both = __vmaxu2(both, __shfl_xor_sync(0xffffffffu, both, o));
-          const int top = max((int)(both >> 23), 27), low = (int)(((~both & 0xFFFFu) + 1u) >> 7);     // exponents (all zero: low 512)
-          // whole numbers below 2^29 in steps of 2^(top - 127 - 28): exact down to exponent top - 21
-          const bool lost = top > 254 || low < top - 21 || (top < 33 && low < 512);                   // (the last: steps below 2^-126)
-          const float inv = __uint_as_float((274u - (uint32_t)min(top, 254)) << 23);                  // |x inv| < 2^21
-          uint32_t y[8];
-#pragma unroll
-          for (int e = 0; e < 8; ++e) {
-            const float a = e & 1 ? bf16_hi(uw[e >> 1]) : bf16_lo(uw[e >> 1]);
-            const float whole = fmaf(a, inv, W4S_MAGICF), rest = fmaf(fmaf(a, inv, -(whole - W4S_MAGICF)), 256.f, W4S_MAGICF);
-            // 256 whole + rest, in four signed digits of base 256
-            y[e] = (__float_as_uint(whole) * 256u + __float_as_uint(rest) + (0x80808080u - 257u * (uint32_t)W4S_MAGIC)) ^ 0x80808080u;
-          }
-          any_lost |= lost && mine_too;
-          if (mine_too) {
-            unsigned char* at = w4s_smem + 4 * m * L.pitch + gl * 128 + 8 * l16;
-            if (lost) {                                                          // elements 0..3 in the first row, 4..7 in the second
-              *reinterpret_cast<uint2*>(at) = make_uint2(u.x, u.y);
-              *reinterpret_cast<uint2*>(at + L.pitch) = make_uint2(u.z, u.w);
-            } else {
-#pragma unroll
-              for (int d = 0; d < 4; ++d) {
-                const uint32_t sel = d | ((4 + d) << 4);
-                const uint32_t b0 = __byte_perm(__byte_perm(y[0], y[4], sel), __byte_perm(y[1], y[5], sel), 0x5410);
-                const uint32_t b1 = __byte_perm(__byte_perm(y[2], y[6], sel), __byte_perm(y[3], y[7], sel), 0x5410);
-                *reinterpret_cast<uint2*>(at + d * L.pitch) = make_uint2(b0, b1);
-              }
+            for (int e = 0; e < 4; ++e) {
+              mx = __vmaxu2(mx, uw[e] & 0x7FFF7FFFu);
+              mn = __vmaxu2(mn, ((uw[e] | 0x80008000u) - 0x00010001u) ^ 0x7FFF7FFFu);
             }
-            // 2^(top - 127 - 28) / 16 for the lowest digit
-            if (l16 < 4) sx[gl * 8 + 4 * m + l16] = lost ? 0.f : __uint_as_float((uint32_t)max(top - 32 + 8 * l16, 0) << 23);
-            if (l16 < 2 && (l16 == 0 || M == 1)) w4s_smem[L.flags + 2 * gl + m + l16] = l16 == 0 && lost ? 1 : 0;
+            both[q] = __vmaxu2(__byte_perm(mn, mx, 0x7632), __byte_perm(mn, mx, 0x5410));           // (max | ~min) of either half
+          }
+#pragma unroll
+          for (int o = 8; o > 0; o >>= 1)
+#pragma unroll
+            for (int q = 0; q < NQ; ++q) both[q] = __vmaxu2(both[q], __shfl_xor_sync(0xffffffffu, both[q], o));
+#pragma unroll
+          for (int q = 0; q < NQ; ++q) {
+            const uint32_t uw[4] = {u[q].x, u[q].y, u[q].z, u[q].w};
+            const int top = max((int)(both[q] >> 23), 27), low = (int)(((~both[q] & 0xFFFFu) + 1u) >> 7);     // exponents (all zero: low 512)
+            // whole numbers below 2^29 in steps of 2^(top - 127 - 28): exact down to exponent top - 21
+            const bool lost = top > 254 || low < top - 21 || (top < 33 && low < 512);                   // (the last: steps below 2^-126)
+            const float inv = __uint_as_float((274u - (uint32_t)min(top, 254)) << 23);                  // |x inv| < 2^21
+            uint32_t y[8];
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+              const float a = e & 1 ? bf16_hi(uw[e >> 1]) : bf16_lo(uw[e >> 1]);
+              const float whole = fmaf(a, inv, W4S_MAGICF), rest = fmaf(fmaf(a, inv, -(whole - W4S_MAGICF)), 256.f, W4S_MAGICF);
+              // 256 whole + rest, in four signed digits of base 256
+              y[e] = (__float_as_uint(whole) * 256u + __float_as_uint(rest) + (0x80808080u - 257u * (uint32_t)W4S_MAGIC)) ^ 0x80808080u;
+            }
+            // bytes of elements 0,4,1,5 / 2,6,3,7, digit by digit
+            uint32_t lo[4], hi[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+              lo[e] = __byte_perm(y[e], y[e + 4], 0x5140);                     // digits 0 0 1 1
+              hi[e] = __byte_perm(y[e], y[e + 4], 0x7362);                     // digits 2 2 3 3
+            }
+            // a group that the digits cannot hold: its bf16 elements 0..3 in the first row, 4..7 in the second
+            const uint2 d0 = lost ? make_uint2(uw[0], uw[1]) : make_uint2(__byte_perm(lo[0], lo[1], 0x5410), __byte_perm(lo[2], lo[3], 0x5410));
+            const uint2 d1 = lost ? make_uint2(uw[2], uw[3]) : make_uint2(__byte_perm(lo[0], lo[1], 0x7632), __byte_perm(lo[2], lo[3], 0x7632));
+            any_lost |= lost;
+            if (there[q]) {
+              unsigned char* at = w4s_smem + 4 * row[q] * L.pitch + grp[q] * 128 + 8 * l16;
+              *reinterpret_cast<uint2*>(at) = d0;
+              *reinterpret_cast<uint2*>(at + L.pitch) = d1;
+              *reinterpret_cast<uint2*>(at + 2 * L.pitch) = make_uint2(__byte_perm(hi[0], hi[1], 0x5410), __byte_perm(hi[2], hi[3], 0x5410));
+              *reinterpret_cast<uint2*>(at + 3 * L.pitch) = make_uint2(__byte_perm(hi[0], hi[1], 0x7632), __byte_perm(hi[2], hi[3], 0x7632));
+              // 2^(top - 127 - 28) / 16 for the lowest digit
+              if (l16 < 4) sx[grp[q] * 8 + 4 * row[q] + l16] = lost ? 0.f : __uint_as_float((uint32_t)max(top - 32 + 8 * l16, 0) << 23);
+              if (l16 < 2 && (l16 == 0 || M == 1)) w4s_smem[L.flags + 2 * grp[q] + row[q] + l16] = l16 == 0 && lost ? 1 : 0;
+            }
           }
         }
-      }
+      });
     }
     any_lost = __syncthreads_or(any_lost);
 
@@ -361,94 +413,99 @@ w4_stream_kernel(const W4StreamArgs p, const int tile_base, const int tiles, con
       float acc[4] = {0.f, 0.f, 0.f, 0.f};      // first column, x rows (digits: digit columns) 2 t, 2 t + 1; second column
       int ci = 0, xg = xg0;                     // consume cursor: unit of the tile
       uint32_t off = 0;                         // and its slot, which the next load refills
-      for (int it = 0; it < total; ++it) {
-        cp_async_wait_group<D - 1>();
-        __syncwarp();
-        if (ci < mine) {
-          const unsigned char* sl = w4s_smem + L.ring + warp * (D * W4S_SLOT) + off;
-          auto words = [&](int j, uint32_t& w0, uint32_t& w1) {
-            if (MODE == W4S_GATED) {
-              w0 = *reinterpret_cast<const uint32_t*>(sl + rsrc + 256 * j);
-              w1 = *reinterpret_cast<const uint32_t*>(sl + (rsrc ^ 32u) + 256 * j);
-            } else {
-              const uint2 w = *reinterpret_cast<const uint2*>(sl + rsrc + 256 * j);
-              w0 = w.x;
-              w1 = w.y;
-            }
-          };
-          float s0, s1;
-          if (MODE == W4S_GATED) {
-            s0 = bf16_lo(*reinterpret_cast<const unsigned short*>(sl + 1024 + 2 * gq));
-            s1 = bf16_lo(*reinterpret_cast<const unsigned short*>(sl + 1040 + 2 * gq));
-          } else {
-            const uint32_t w = *reinterpret_cast<const uint32_t*>(sl + 1024 + 4 * gq);
-            s0 = bf16_lo(w);
-            s1 = bf16_hi(w);
-          }
-          uint32_t lost = 0u;                   // rows of this group that keep bf16 values
-          if (!EXACT) lost = *reinterpret_cast<const unsigned short*>(w4s_smem + L.flags + (xg >> 6));
-          if (DIGITS && (EXACT || lost != (M == 1 ? 1u : 0x101u))) {
-            int dd[4] = {W4S_MAGIC, W4S_MAGIC, W4S_MAGIC, W4S_MAGIC};
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              uint32_t w0, w1;
-              words(j, w0, w1);
-              const uint2 xb = gq < 4 * M ? *reinterpret_cast<const uint2*>(xr + xg + 32 * j) : make_uint2(0u, 0u);
-              w4s_mma_s8(dd, w4s_lo(w0), w4s_lo(w1), w4s_hi(w0), w4s_hi(w1), xb.x, xb.y);
-            }
-            const float2 st = *reinterpret_cast<const float2*>(w4s_smem + L.sx + (xg >> 2) + 8 * tq);
-            acc[0] = fmaf(__int_as_float(dd[0]) - W4S_MAGICF, s0 * st.x, acc[0]);
-            acc[1] = fmaf(__int_as_float(dd[1]) - W4S_MAGICF, s0 * st.y, acc[1]);
-            acc[2] = fmaf(__int_as_float(dd[2]) - W4S_MAGICF, s1 * st.x, acc[2]);
-            acc[3] = fmaf(__int_as_float(dd[3]) - W4S_MAGICF, s1 * st.y, acc[3]);
-          }
-          if (!DIGITS || (!EXACT && lost != 0u)) {
-            float d[4] = {0.f, 0.f, 0.f, 0.f};
-            // (digits: row gq / 4 in its first digit's column)
-            const bool xrow = DIGITS ? (gq & 3) == 0 && gq < 4 * M && (lost >> (2 * gq) & 1u) != 0 : gq < M;
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              uint32_t w0, w1;
-              words(j, w0, w1);
-              uint4 xv = make_uint4(0u, 0u, 0u, 0u);
-              if (xrow) {
-                if (DIGITS) {
-                  const uint2 lo = *reinterpret_cast<const uint2*>(xr + xg + 32 * j), hi = *reinterpret_cast<const uint2*>(xr + L.pitch + xg + 32 * j);
-                  xv = make_uint4(lo.x, lo.y, hi.x, hi.y);
+      // One turn per tile, and at the end one per epilogue that is left (a second copy of it would be cold).
+      for (int tile = 0;; ++tile) {
+        if (tile < ntiles) {
+          for (ci = 0; ci < gpw; ++ci) {
+            cp_async_wait_group<D - 1>();
+            __syncwarp();
+            if (ci < mine) {
+              const unsigned char* sl = w4s_smem + L.ring + warp * (D * W4S_SLOT) + off;
+              auto words = [&](int j, uint32_t& w0, uint32_t& w1) {
+                if (MODE == W4S_GATED) {
+                  w0 = *reinterpret_cast<const uint32_t*>(sl + rsrc + 256 * j);
+                  w1 = *reinterpret_cast<const uint32_t*>(sl + (rsrc ^ 32u) + 256 * j);
                 } else {
-                  xv = *reinterpret_cast<const uint4*>(xr + xg + 64 * j);
+                  const uint2 w = *reinterpret_cast<const uint2*>(sl + rsrc + 256 * j);
+                  w0 = w.x;
+                  w1 = w.y;
                 }
+              };
+              float s0, s1;
+              if (MODE == W4S_GATED) {
+                s0 = bf16_lo(*reinterpret_cast<const unsigned short*>(sl + 1024 + 2 * gq));
+                s1 = bf16_lo(*reinterpret_cast<const unsigned short*>(sl + 1040 + 2 * gq));
+              } else {
+                const uint32_t w = *reinterpret_cast<const uint32_t*>(sl + 1024 + 4 * gq);
+                s0 = bf16_lo(w);
+                s1 = bf16_hi(w);
               }
-              w4s_mma(d, w4s_pair(w0, 0), w4s_pair(w1, 0), w4s_pair(w0, 1), w4s_pair(w1, 1), xv.x, xv.y);
-              w4s_mma(d, w4s_pair(w0, 2), w4s_pair(w1, 2), w4s_pair(w0, 3), w4s_pair(w1, 3), xv.z, xv.w);
+              uint32_t lost = 0u;                   // rows of this group that keep bf16 values
+              if (!EXACT) lost = *reinterpret_cast<const unsigned short*>(w4s_smem + L.flags + (xg >> 6));
+              if (DIGITS && (EXACT || lost != (M == 1 ? 1u : 0x101u))) {
+                int dd[4] = {W4S_MAGIC, W4S_MAGIC, W4S_MAGIC, W4S_MAGIC};
+    #pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                  uint32_t w0, w1;
+                  words(j, w0, w1);
+                  const uint2 xb = gq < 4 * M ? *reinterpret_cast<const uint2*>(xr + xg + 32 * j) : make_uint2(0u, 0u);
+                  w4s_mma_s8(dd, w4s_lo(w0), w4s_lo(w1), w4s_hi(w0), w4s_hi(w1), xb.x, xb.y);
+                }
+                const float2 st = *reinterpret_cast<const float2*>(w4s_smem + L.sx + (xg >> 2) + 8 * tq);
+                acc[0] = fmaf(__int_as_float(dd[0]) - W4S_MAGICF, s0 * st.x, acc[0]);
+                acc[1] = fmaf(__int_as_float(dd[1]) - W4S_MAGICF, s0 * st.y, acc[1]);
+                acc[2] = fmaf(__int_as_float(dd[2]) - W4S_MAGICF, s1 * st.x, acc[2]);
+                acc[3] = fmaf(__int_as_float(dd[3]) - W4S_MAGICF, s1 * st.y, acc[3]);
+              }
+              if (!DIGITS || (!EXACT && lost != 0u)) {
+                float d[4] = {0.f, 0.f, 0.f, 0.f};
+                // (digits: row gq / 4 in its first digit's column)
+                const bool xrow = DIGITS ? (gq & 3) == 0 && gq < 4 * M && (lost >> (2 * gq) & 1u) != 0 : gq < M;
+    #pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                  uint32_t w0, w1;
+                  words(j, w0, w1);
+                  uint4 xv = make_uint4(0u, 0u, 0u, 0u);
+                  if (xrow) {
+                    if (DIGITS) {
+                      const uint2 lo = *reinterpret_cast<const uint2*>(xr + xg + 32 * j), hi = *reinterpret_cast<const uint2*>(xr + L.pitch + xg + 32 * j);
+                      xv = make_uint4(lo.x, lo.y, hi.x, hi.y);
+                    } else {
+                      xv = *reinterpret_cast<const uint4*>(xr + xg + 64 * j);
+                    }
+                  }
+                  w4s_mma(d, w4s_pair(w0, 0), w4s_pair(w1, 0), w4s_pair(w0, 1), w4s_pair(w1, 1), xv.x, xv.y);
+                  w4s_mma(d, w4s_pair(w0, 2), w4s_pair(w1, 2), w4s_pair(w0, 3), w4s_pair(w1, 3), xv.z, xv.w);
+                }
+                acc[0] = fmaf(d[0], s0, acc[0]);
+                acc[1] = fmaf(d[1], s0, acc[1]);
+                acc[2] = fmaf(d[2], s1, acc[2]);
+                acc[3] = fmaf(d[3], s1, acc[3]);
+              }
             }
-            acc[0] = fmaf(d[0], s0, acc[0]);
-            acc[1] = fmaf(d[1], s0, acc[1]);
-            acc[2] = fmaf(d[2], s1, acc[2]);
-            acc[3] = fmaf(d[3], s1, acc[3]);
+            __syncwarp();                         // everyone has read the slot
+            load(off);
+            off = off == (D - 1) * W4S_SLOT ? 0u : off + W4S_SLOT;
+            xg += XG;
           }
+          // ---- tile done: hand this warp's sums over
+          xg = xg0;
+          const int hb = handed & (W4S_NB - 1);
+          if (handed >= W4S_NB && !mbar_wait(&empty[hb], ((handed / W4S_NB) - 1) & 1, &abort_flag, err)) return false;
+          if (DIGITS || 2 * tq < M) {
+            float* r = red + ((hb * W4S_WARPS + warp) * RP + 2 * tq) * W4S_TILE + 2 * gq;
+            *reinterpret_cast<float2*>(r) = make_float2(acc[0], acc[2]);
+            *reinterpret_cast<float2*>(r + W4S_TILE) = make_float2(acc[1], acc[3]);
+          }
+          acc[0] = acc[1] = acc[2] = acc[3] = 0.f;
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&full[hb]);
+          if (++handed - ep_q <= 2) continue;
+        } else if (pass + 1 < passes || ep_q == handed) {
+          return true;
         }
-        __syncwarp();                         // everyone has read the slot
-        load(off);
-        off = off == (D - 1) * W4S_SLOT ? 0u : off + W4S_SLOT;
-        xg += XG;
-        if (++ci < gpw) continue;
-        // ---- tile done: hand this warp's sums over
-        ci = 0;
-        xg = xg0;
-        const int hb = handed & (W4S_NB - 1);
-        if (handed >= W4S_NB && !mbar_wait(&empty[hb], ((handed / W4S_NB) - 1) & 1, &abort_flag, err)) return false;
-        if (DIGITS || 2 * tq < M) {
-          float* r = red + ((hb * W4S_WARPS + warp) * RP + 2 * tq) * W4S_TILE + 2 * gq;
-          *reinterpret_cast<float2*>(r) = make_float2(acc[0], acc[2]);
-          *reinterpret_cast<float2*>(r + W4S_TILE) = make_float2(acc[1], acc[3]);
-        }
-        acc[0] = acc[1] = acc[2] = acc[3] = 0.f;
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&full[hb]);
-        if (++handed > 2) epilogue();
+        epilogue();
       }
-      return true;
     };
     bool ok;
     if constexpr (DIGITS) ok = any_lost ? stream(std::false_type{}) : stream(std::true_type{});
@@ -457,7 +514,6 @@ w4_stream_kernel(const W4StreamArgs p, const int tile_base, const int tiles, con
     if (!ok) return;
     if (pass + 1 < passes) __syncthreads();   // every warp is done with x
   }
-  while (ep_q < handed) epilogue();
 }
 
 // How a call is cut: digits or bf16 products, ring depth, scale groups per K pass, column tiles per launch. The rows of x of a
