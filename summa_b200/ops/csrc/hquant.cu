@@ -443,7 +443,7 @@ struct ArFuse {
   unsigned int* epoch_word;          // call number (device, owned by the kernel)
   unsigned int* counter;             // CTA arrival counter for the epoch bump
   unsigned int* err;
-  int rank, world;                   // world == 0: plain epilogue
+  int rank, world;                   // world >= 2
   long n_pad;
 };
 
@@ -939,10 +939,8 @@ extern "C" int sb_w4_gemv_mma(const void* x, const void* wk8, const void* scales
 // groups round robin and use the 16-byte-vector fragment mapping of w4_gemv_mma_kernel, the weights arriving
 // through a per-warp ring of asynchronous copies three groups ahead. Per block the warps' tiles meet in shared
 // memory and the epilogue adds the residual or applies SwiGLU (a gated block is 16 gate columns + the matching
-// 16 value columns). Measured on a B200 (N 28672, K 4096, one row: 31 us against 33 us for the cluster kernel,
-// DRAM 24 % of peak, the integer pipe at 45 % still the busiest unit) it is level with the cluster kernel launch
-// by launch and slower inside the decode step's graph, where a resident grid leaves the next kernel's prologue
-// nothing to overlap with; the decode path therefore stays on the cluster kernel and this one is an explicit
+// 16 value columns). Measured on a B200: N 28672, K 4096, one row 31 us (DRAM 24 % of peak, the
+// integer pipe at 45 % the busiest unit). The decode path runs on w4_stream.cu (18.7 us there); this one is an explicit
 // alternative (sb_w4_gemv_stream).
 namespace sb {
 
@@ -1216,8 +1214,8 @@ static int launch_w4_stream(const void* x, const void* wk8, const void* scales, 
 
 // y[M,N] = (rmsnorm(x) or x)[M,K] @ dequant(W) (+ residual), or with gated != 0 y[M,N/2] = silu(g) * v for
 // W = [gate | value], on the persistent streaming kernel. M <= 4, K % 128 == 0, N % 4 == 0 (gated: N % 8 == 0).
-// An alternative to sb_w4_gemv_cluster / sb_w4_gemv_cluster_swiglu: level with them launch by launch, behind them
-// inside a decode step's graph (a resident grid gives the next kernel's prologue nothing to overlap with).
+// An independent form of sb_w4_gemv_cluster / sb_w4_gemv_cluster_swiglu, for tests and comparison (one row, N 28672, K 4096: 31 us
+// against 18.7 for those).
 extern "C" int sb_w4_gemv_stream(const void* x, const void* wk8, const void* scales, const void* residual, void* y,
                                  int M, int N, int K, long ldx, const float* gamma, float eps, int gated,
                                  cudaStream_t st) {

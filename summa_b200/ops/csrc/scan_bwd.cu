@@ -32,7 +32,7 @@ struct ScanBwdParams {
   const __nv_bfloat16 *u, *delta, *Bm, *Cm, *dy;
   const float *A, *ckpt, *dh_out;          // dh_out: grad wrt final state [B,C,N] or null
   float *ddt_part, *du_part;               // [NS][B][T][C] partial sums over this block's states
-  float *dB_part, *dC_part;                // [C/32 tiles][B][T][N]
+  float *dB_part, *dC_part;                // [C / sb_scan_bwd_tile_channels tiles][B][T][N]
   float *dA, *dD;                          // [C,N], [C] (atomic accumulate over batch)
   float* dh0;                              // [B,C,N] or null
   int B, T, C;
