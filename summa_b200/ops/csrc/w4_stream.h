@@ -36,8 +36,8 @@ struct W4StreamArgs {
 
 constexpr int W4S_MAX_ROWS = 8;
 // Whether this kernel is ahead of the tcgen05 one (sb_w4a16_gemm). Up to 8 rows as long as x fits its shared memory in one pass
-// (M 8, K 4096: N 28672 28.6 us against 48.4, N 6144 10.8 against 17.6; M 4, K 14336, N 4096: 18.2 us against 20.3; otherwise K
-// is walked in passes, each with its own staging). From 9 rows on it would need a second set of mma columns.
+// (M 8, K 4096, N 28672: 28.7 us, there 39.9 for 12 rows; M 4, K 14336, N 4096: 19.0 us, there 19.6 for 6 rows; otherwise K is
+// walked in passes, each with its own staging). From 9 rows on it would need a second set of mma columns.
 bool w4_stream_preferred(int M, int K);
 int launch_w4_stream(const W4StreamArgs& a, W4StreamMode mode, cudaStream_t st);
 
