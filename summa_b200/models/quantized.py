@@ -41,23 +41,38 @@ class QuantLinear(nn.Module):
         self.register_buffer("bias", bias)
         self._k8 = None           # repacked copy for the tensor-core decode kernel (built on first use)
         self._scales8 = None      # aligned copy of scales that start off an 8-byte boundary (built on first use)
+        self._stamps = {}         # what the copies were made from: address and version of the buffer
+
+    def _prepared(self, name: str, source: torch.Tensor, make) -> bool:
+        """Brings the copy `name` up to date with `source` (a write to the buffer, `load_state_dict`, another device); whether it
+        was up to date already. A copy of the same form is rewritten in place: a captured step may hold its address."""
+        stamp = (source.data_ptr(), -1 if source.is_inference() else source._version)
+        old, seen = getattr(self, name), self._stamps.get(name)
+        if old is not None and old.device == source.device and seen == stamp:
+            return True
+        new = make(source)
+        if old is not None and old.device == new.device and old.shape == new.shape:
+            old.copy_(new)
+        else:
+            setattr(self, name, new)
+        self._stamps[name] = stamp
+        return False
 
     def packed_k8(self) -> torch.Tensor:
-        if self._k8 is None or self._k8.device != self.packed.device:
-            self._k8 = reference.repack_int4_k8(self.packed)
+        self._prepared("_k8", self.packed, reference.repack_int4_k8)
         return self._k8
 
     def decode_operands(self):
         """(codes, scales, settled) for the decode kernels: the repacked codes, the scales on the 8-byte boundary that those need
-        (a view that starts elsewhere is copied once, here), and whether both were there before this call, i.e. nothing in
-        flight writes them."""
-        settled = self._k8 is not None and self._k8.device == self.packed.device
-        k8, scales = self.packed_k8(), self.scales
-        if scales.is_cuda and scales.data_ptr() % 8:
-            if self._scales8 is None or self._scales8.device != scales.device:
-                self._scales8, settled = scales.clone(), False
-            scales = self._scales8
-        return k8, scales, settled
+        (a view that starts elsewhere is copied, here), and whether all of it was there before this call, i.e. nothing in flight
+        writes it."""
+        settled = self._prepared("_k8", self.packed, reference.repack_int4_k8)
+        stamp = (self.scales.data_ptr(), -1 if self.scales.is_inference() else self.scales._version)
+        settled, self._stamps["scales"] = settled and self._stamps.get("scales") == stamp, stamp
+        if self.scales.is_cuda and self.scales.data_ptr() % 8:
+            settled = self._prepared("_scales8", self.scales, torch.clone) and settled
+            return self._k8, self._scales8, settled
+        return self._k8, self.scales, settled
 
     @staticmethod
     def from_linear(lin: Linear) -> "QuantLinear":

@@ -457,3 +457,27 @@ def test_hybrid_decode_runs_hooks_and_subclasses():
     model.layers[0].ssm.__class__ = MambaMixer
     model.layers[0].ssm.out_proj.__class__ = Double
     assert not cuda_ops.mamba_decode_usable(model.layers[0].ssm)
+
+
+@pytest.mark.parametrize("device", ["cpu", pytest.param("cuda", marks=gpu)])
+def test_w4_layer_follows_its_buffers(device):
+    """New codes and scales in a layer's buffers are what it computes with: the repacked codes and the aligned scales are made again
+    (in place, so that an address held by a captured step stays good), and the call that does it is not a settled one."""
+    from summa_b200.models.quantized import QuantLinear
+    from summa_b200.ops import reference
+    torch.manual_seed(11)
+    a, b = [[t.to(device) for t in reference.quantize_int4_g128(torch.randn(256, 24) * 0.05)] for _ in range(2)]
+    off = torch.empty(a[1].numel() + 1, device=device, dtype=a[1].dtype)[1:].view_as(a[1]).copy_(a[1])
+    x = torch.randn(2, 256, device=device).to(torch.bfloat16)
+    for scales in (a[1], off):
+        layer, other = QuantLinear(a[0].clone(), scales), QuantLinear(*b)
+        layer(x)
+        k8 = layer.decode_operands()[0]
+        assert torch.equal(k8, reference.repack_int4_k8(a[0])) and layer.decode_operands()[2]
+        layer.load_state_dict(other.state_dict())
+        again, s, settled = layer.decode_operands()
+        assert not settled and again.data_ptr() == k8.data_ptr()
+        assert torch.equal(again, reference.repack_int4_k8(b[0])) and torch.equal(s, b[1])
+        assert torch.equal(layer(x), other(x)) and layer.decode_operands()[2]
+        layer.scales.mul_(2)
+        assert not layer.decode_operands()[2] and torch.equal(layer(x), 2 * other(x))
